@@ -12,6 +12,8 @@ enum GemmEpi {
     GE_MUL,          // acc * aux[m][n] (operand type), operand type
     GE_GROUP_GATE,   // acc * sigmoid(gate[m][group]) (FP32), operand type
     GE_GEGLU,        // columns in tiles of 8 gates and the 8 values they gate: gelu_tanh(gate) * value, operand type, half as many columns
+    GE_F32_ROW,      // acc * row_scale[m], FP32
+    GE_SILU_ROW,     // columns as GE_GEGLU, silu(gate * row_scale[m]) * value * row_scale[m], FP32, half as many columns
 };
 
 // `groups` > 1: a block-diagonal product (one block per attention head): group z multiplies columns a_step*z.. of `a` with rows
@@ -30,8 +32,10 @@ struct GemmArgs {
     int ldaux = 0;
     int groups = 1, a_step = 0, w_step = 0, o_step = 0;
     int w_rows = 0;  // rows of `w` in memory (0: N, or w_step * groups)
+    bool half = false;                // operands are FP16 instead of BF16 (GE_F32_ROW and GE_SILU_ROW only)
+    const float *row_scale = nullptr;
 };
-int launch_gemm_rows_tc(juno_ctx *c, const GemmArgs &a, unsigned *err, cudaStream_t st);  // BF16, tcgen05
+int launch_gemm_rows_tc(juno_ctx *c, const GemmArgs &a, unsigned *err, cudaStream_t st);  // 16-bit operands, tcgen05
 int launch_gemm_rows(juno_ctx *c, int dt, const GemmArgs &a, unsigned *err, cudaStream_t st);
 
 }  // namespace juno

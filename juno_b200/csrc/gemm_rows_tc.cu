@@ -1,4 +1,4 @@
-// BF16 matrix products of many rows on the 5th-generation tensor cores.
+// 16-bit matrix products of many rows on the 5th-generation tensor cores.
 //
 // A persistent CTA walks 128 x BN output tiles.  One warp streams both operands with TMA (64 K values = 128-byte rows, 128-byte
 // swizzle) through a ring of shared-memory stages; one thread issues tcgen05.mma into one of two TMEM accumulators and commits
@@ -13,6 +13,7 @@
 #include <mutex>
 
 #include "gemm_rows.cuh"
+#include "tile_math.cuh"
 
 namespace juno {
 
@@ -108,6 +109,31 @@ __device__ __forceinline__ void store_row(const GemmArgs &g, int z, int m, int n
 #pragma unroll
             for (int j = 0; j < 32; j++)
                 if (j < nv) out[j] = __uint_as_float(r[j]);
+        }
+        return;
+    }
+    if (EPI == GE_F32_ROW) {  // N and ldo are multiples of 16
+        const float s = g.row_scale[m];
+        float *out = static_cast<float *>(g.out) + o;
+#pragma unroll
+        for (int j = 0; j < 32; j += 4) {
+            if (j >= nv) break;
+            *reinterpret_cast<float4 *>(out + j) = make_float4(__uint_as_float(r[j]) * s, __uint_as_float(r[j + 1]) * s, __uint_as_float(r[j + 2]) * s,
+                                                               __uint_as_float(r[j + 3]) * s);
+        }
+        return;
+    }
+    if (EPI == GE_SILU_ROW) {
+        const float s = g.row_scale[m];
+        float *out = static_cast<float *>(g.out) + (size_t)m * g.ldo + (n >> 1);
+#pragma unroll
+        for (int j = 0; j < 32; j += 16) {
+            if (j >= nv) break;
+            float v[8];
+#pragma unroll
+            for (int e = 0; e < 8; e++) v[e] = __fmul_rn(silu_ref(__uint_as_float(r[j + e]) * s), __uint_as_float(r[j + 8 + e]) * s);
+            *reinterpret_cast<float4 *>(out + j / 2) = make_float4(v[0], v[1], v[2], v[3]);
+            *reinterpret_cast<float4 *>(out + j / 2 + 4) = make_float4(v[4], v[5], v[6], v[7]);
         }
         return;
     }
@@ -209,8 +235,8 @@ __global__ void __launch_bounds__(kTileThreads, 1) gemm_rows_tc_kernel(const __g
         }
     } else if (warp == 1) {
         if (lane == 0) {
-            // D FP32, A and B BF16, both K-major
-            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
+            // D FP32, A and B BF16 or both FP16, both K-major
+            const uint32_t idesc = (1u << 4) | (g.half ? 0u : (1u << 7) | (1u << 10)) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
             unsigned it = 0, tile = 0;
             bool ok = true;
             for (int work = blockIdx.x; ok && work < p.n_work; work += gridDim.x, tile++) {
@@ -283,7 +309,7 @@ static EncodeTiled encode_tiled() {
     return fn;
 }
 
-// Row-major BF16 matrix [rows][cols] with pitch ld, boxes of box_rows x 64 columns.
+// Row-major matrix of 16-bit elements [rows][cols] with pitch ld, boxes of box_rows x 64 columns.
 int tensor_map_bf16(CUtensorMap *map, const void *base, int64_t rows, int64_t cols, int64_t ld, int box_rows) {
     EncodeTiled enc = encode_tiled();
     JUNO_REQUIRE(enc, "the driver has no cuTensorMapEncodeTiled");
@@ -320,6 +346,8 @@ static int gemm_tc_epi(juno_ctx *c, const GemmTcParams &p, cudaStream_t st) {
     case GE_RELU2: return gemm_tc_inst<BN, GE_RELU2>(c, p, st);
     case GE_MUL: return gemm_tc_inst<BN, GE_MUL>(c, p, st);
     case GE_GEGLU: return gemm_tc_inst<BN, GE_GEGLU>(c, p, st);
+    case GE_F32_ROW: return gemm_tc_inst<BN, GE_F32_ROW>(c, p, st);
+    case GE_SILU_ROW: return gemm_tc_inst<BN, GE_SILU_ROW>(c, p, st);
     default: return gemm_tc_inst<BN, GE_GROUP_GATE>(c, p, st);
     }
 }

@@ -18,7 +18,9 @@
 #include "common.cuh"
 #include "dequant.cuh"
 #include "gemv.cuh"
+#include "gemm_rows.cuh"
 #include "model.cuh"
+#include "prompt.cuh"
 #include "qgemv.cuh"
 #include "stack.cuh"
 
@@ -347,6 +349,8 @@ static void model_release(juno_model *m) {
     for (void *b : bufs)
         if (b) cudaFree(b);
     if (m->h_step) cudaFreeHost(m->h_step);
+    if (m->prompt.dev) cudaFree(m->prompt.dev);
+    if (m->prompt.h_step) cudaFreeHost(m->prompt.h_step);
     stack_free(m->stack);
     m->stack = nullptr;
     m->magic = kMagicDead;
@@ -909,6 +913,218 @@ static int enqueue_layers_batched(juno_model *m, int n, const int32_t *d_slot, c
     return product(lm, lo, 1, EPI_STORE, m->vocab_loc, m->img_h, sc_h);
 }
 
+// ───────────────────────────── prompt passes of many positions ────────────────────────────
+constexpr int kPromptRows = 2048;  // most positions per pass
+
+static int step_sync(juno_model *m);
+
+// Does a portion of n positions take the many-row path?  Its cost hardly depends on n below a few hundred (every weight is read,
+// turned into FP16 and read again), so it pays as soon as the batched kernels would need a second pass: Llama-3-8B, 65 positions
+// through them 14 ms.  A model opened for few sequences has small passes that cost less each, hence the third pass there.
+static bool prompt_takes(const juno_model *m, int n) {
+    if (m->stack || m->world > 1) return false;
+    const int chunk = std::min(m->cfg.max_batch, kGemmMaxBatch);
+    return n > (chunk >= 8 ? chunk : 2 * chunk);
+}
+
+// Room for n rows; JUNO_ERR_OOM leaves the model without the workspace (the caller then uses the smaller passes).
+static int prompt_reserve(juno_model *m, int n) {
+    JunoPrompt &P = m->prompt;
+    const int rows = (std::min(n, kPromptRows) + 127) / 128 * 128;
+    if (rows <= P.rows) return JUNO_OK;
+    const size_t H = m->cfg.hidden, R = rows, I = m->inter_loc;
+    size_t w16 = 0;  // elements of the largest group of matrices that one product takes
+    for (const JunoLayer &L : m->layers) {
+        auto elems = [&](int k) { return (size_t)L.w[k]->row_tiles * 16 * (size_t)L.w[k]->cols; };
+        w16 = std::max({w16, elems(JUNO_T_ATTN_Q) + elems(JUNO_T_ATTN_K) + elems(JUNO_T_ATTN_V), elems(JUNO_T_ATTN_OUT), elems(JUNO_T_FFN_GATE), elems(JUNO_T_FFN_DOWN)});
+    }
+    const size_t sizes[] = {R * H * 4, R * H * 4, R * m->qkv_ld * 4, R * H * 4, R * H * 4, R * I * 4, R * 4, R * std::max(H, I) * 2, w16 * 2,
+                            R * (m->hd / 2) * sizeof(float2), 4 * R * 4};
+    size_t total = 0;
+    for (size_t s : sizes) total += (s + 1023) & ~(size_t)1023;
+    JUNO_TRY(step_sync(m));
+    if (P.dev) cudaFree(P.dev);
+    if (P.h_step) cudaFreeHost(P.h_step);
+    P = JunoPrompt();
+    JUNO_TRY(dev_alloc((void **)&P.dev, total));
+    if (cudaMallocHost((void **)&P.h_step, 4 * R * 4) != cudaSuccess) {
+        cudaGetLastError();
+        cudaFree(P.dev);
+        P = JunoPrompt();
+        set_error("cudaMallocHost of %zu bytes failed", 4 * R * 4);
+        return JUNO_ERR_OOM;
+    }
+    uint8_t *at = P.dev;
+    int k = 0;
+    auto take = [&]() {
+        uint8_t *p = at;
+        at += (sizes[k++] + 1023) & ~(size_t)1023;
+        return p;
+    };
+    P.x[0] = (float *)take();
+    P.x[1] = (float *)take();
+    P.qkv = (float *)take();
+    P.att = (float *)take();
+    P.proj = (float *)take();
+    P.hdn = (float *)take();
+    P.scale = (float *)take();
+    P.img = take();
+    P.w16 = take();
+    P.cs = (float2 *)take();
+    P.step = (int32_t *)take();
+    P.rows = rows;
+    return JUNO_OK;
+}
+
+// Layers of one pass of n consecutive positions of one sequence.  On return the residual stream is x[cur] + proj.
+static int enqueue_layers_prompt(juno_model *m, int n, int pos0, int &cur, cudaStream_t st) {
+    juno_ctx *c = m->ctx;
+    const juno_model_cfg &f = m->cfg;
+    JunoPrompt &P = m->prompt;
+    const int H = f.hidden, hd = m->hd, Hl = m->heads_loc * hd, KVl = m->kv_loc * hd, I = m->inter_loc, R = P.rows;
+    const int32_t *d_pos = P.step + R, *d_slot = P.step + 2 * R, *d_len = P.step + 3 * R;
+    auto stage = [&](const float *x, const float *add, const float *normw, float *x_out, int K) {
+        StageRowsArgs a;
+        a.x = x;
+        a.add = add;
+        a.normw = normw;
+        a.x_out = x_out;
+        a.eps = f.rms_eps;
+        a.n = n;
+        a.K = K;
+        a.out = P.img;
+        a.scale = P.scale;
+        return launch_stage_rows(c, a, st);
+    };
+    auto product = [&](juno_qmat *const *mats, int count, int epi, float *out, int ldo) -> int {
+        DequantSeg seg[3];
+        GemmArgs a;
+        a.K = (int)mats[0]->cols;
+        for (int i = 0; i < count; i++) {
+            seg[i].w = mats[i]->dev;
+            seg[i].type = mats[i]->type;
+            seg[i].row_tiles = (int)mats[i]->row_tiles;
+            a.N += (int)mats[i]->rows;
+        }
+        JUNO_TRY(launch_dequant_rows(c, seg, count, a.K, P.w16, st));
+        a.a = P.img;
+        a.lda = a.K;
+        a.w = P.w16;
+        a.ldw = a.K;
+        a.M = n;
+        a.out = out;
+        a.ldo = ldo;
+        a.epi = epi;
+        a.half = true;
+        a.row_scale = P.scale;
+        return launch_gemm_rows(c, DT_BF16, a, c->gemv_scratch.qerr, st);
+    };
+    cur = 0;
+    for (int l = 0; l < f.n_layers; l++) {
+        JunoLayer &L = m->layers[l];
+        JUNO_TRY(stage(P.x[cur], l ? P.proj : nullptr, L.attn_norm, l ? P.x[cur ^ 1] : nullptr, H));
+        if (l) cur ^= 1;
+        juno_qmat *qkv_m[3] = {L.w[JUNO_T_ATTN_Q], L.w[JUNO_T_ATTN_K], L.w[JUNO_T_ATTN_V]};
+        JUNO_TRY(product(qkv_m, 3, GE_F32_ROW, P.qkv, m->qkv_ld));
+        if (L.bqkv) {
+            const int width = Hl + 2 * KVl;
+            qkv_bias_kernel<<<dim3((width + 255) / 256, n), 256, 0, st>>>(P.qkv, L.bqkv, n, width, m->qkv_ld);
+            JUNO_CUDA_TRY(cudaGetLastError());
+            c->kernel_launches++;
+        }
+        if (m->pool->dtype == 0) {
+            PromptAttnArgs at;
+            at.pool = m->pool;
+            at.layer = l;
+            at.n = n;
+            at.pos0 = pos0;
+            at.n_heads = m->heads_loc;
+            at.qkv = P.qkv;
+            at.ld = m->qkv_ld;
+            at.cs = P.cs;
+            at.slot = d_slot;
+            at.out = P.att;
+            at.algo_bytes = (double)(pos0 + n) * KVl * 2 * m->pool->elem_bytes;
+            JUNO_TRY(launch_prompt_append(c, at, st));
+            JUNO_TRY(launch_prompt_attn(c, at, st));
+        } else {  // FP32 pages: the decode attention, a row at a time, as many rows per launch as its scratch is made for
+            JUNO_TRY(launch_rope_append(c, m->pool, l, n, m->heads_loc, P.qkv, m->qkv_ld, P.qkv + Hl, P.qkv + Hl + KVl, m->qkv_ld, d_slot, d_pos, P.cs, st));
+            const int step = std::min(f.max_batch, kGemmMaxBatch);
+            for (int r = 0; r < n; r += step) {
+                AttnArgs at;
+                at.pool = m->pool;
+                at.layer = l;
+                at.n = std::min(step, n - r);
+                at.n_heads = m->heads_loc;
+                at.q = P.qkv + (size_t)r * m->qkv_ld;
+                at.ldq = m->qkv_ld;
+                at.out = P.att + (size_t)r * Hl;
+                at.slots = d_slot + r;
+                at.seq_lens = d_len + r;
+                at.n_splits = attn_pick_splits(c, at.n, m->kv_loc, pos0 + r + at.n);
+                at.part_o = m->attn_scratch;
+                at.part_ml = m->attn_scratch + (size_t)at.n * m->heads_loc * at.n_splits * hd;
+                at.algo_bytes = (double)at.n * (pos0 + r) * KVl * 2 * m->pool->elem_bytes;
+                JUNO_TRY(launch_attn(c, at, st));
+            }
+        }
+        JUNO_TRY(stage(P.att, nullptr, nullptr, nullptr, Hl));
+        JUNO_TRY(product(&L.w[JUNO_T_ATTN_OUT], 1, GE_F32_ROW, P.proj, H));
+        JUNO_TRY(stage(P.x[cur], P.proj, L.ffn_norm, P.x[cur ^ 1], H));
+        cur ^= 1;
+        JUNO_TRY(product(&L.w[JUNO_T_FFN_GATE], 1, GE_SILU_ROW, P.hdn, I));
+        JUNO_TRY(stage(P.hdn, nullptr, nullptr, nullptr, I));
+        JUNO_TRY(product(&L.w[JUNO_T_FFN_DOWN], 1, GE_F32_ROW, P.proj, H));
+    }
+    return JUNO_OK;
+}
+
+static int q_group(juno_model *m, juno_qmat *const *mats, float *const *outs, int count, const QGemvArgs &proto, cudaStream_t st);
+
+// Logits of `count` rows of the pass that enqueue_layers_prompt left behind, into the first rows of logits_loc: on the exact
+// product for up to eight of them, on the batched one above.
+static int prompt_logits(juno_model *m, const std::pair<int, int> *rows, int count, int cur, cudaStream_t st) {
+    juno_ctx *c = m->ctx;
+    const int H = m->cfg.hidden;
+    JunoPrompt &P = m->prompt;
+    std::vector<int32_t> idx(count);
+    for (int i = 0; i < count; i++) idx[i] = rows[i].first;
+    // the tokens of the pass have been read: their place takes the row numbers
+    JUNO_CUDA_TRY(cudaMemcpyAsync(P.step, idx.data(), (size_t)count * 4, cudaMemcpyHostToDevice, st));
+    JUNO_TRY(launch_gather_rows(c, P.x[cur], P.proj, P.step, 0, count, H, m->x[0], st));
+    juno_qmat *lm[1] = {m->output};
+    float *lo[1] = {m->logits_loc};
+    if (count <= 8) {
+        QGemvArgs a;
+        a.batch = count;
+        a.x = m->x[0];
+        a.ldx = H;
+        a.normw = m->output_norm;
+        a.eps = m->cfg.rms_eps;
+        a.ld_out = m->vocab_loc;
+        return q_group(m, lm, lo, 1, a, st);
+    }
+    StageArgs s;
+    s.mode = STAGE_RMSNORM;
+    s.x = m->x[0];
+    s.ldx = H;
+    s.normw = m->output_norm;
+    s.eps = m->cfg.rms_eps;
+    s.K = H;
+    s.batch = count;
+    s.img = m->img_h;
+    JUNO_TRY(launch_stage_f16(c, s, m->xsc, st, m->img_h_tc));
+    GemvArgs a;
+    a.batch = count;
+    a.ximg = m->img_h;
+    a.xscale = m->xsc;
+    a.ximg_tc = m->img_h_tc;
+    a.tc_err = m->tc_err;
+    a.ld_out = m->vocab_loc;
+    m->tc_used = true;
+    return gemv_group(m, lm, lo, 1, a, st);
+}
+
 // ───────────────────────────── decode step on the integer-MMA GEMV (1..8 sequences) ───────
 // Matrices that share an input share a launch: one block format, or Q4_K mixed with Q6_K.
 static int q_group(juno_model *m, juno_qmat *const *mats, float *const *outs, int count, const QGemvArgs &proto, cudaStream_t st) {
@@ -1368,21 +1584,26 @@ static int prefill_run(juno_model *m, juno_seq *seq, const int32_t *token_ids, i
     JUNO_REQUIRE(n_want == 0 || !m->vocab_sharded, "prefill logits are not implemented for a sharded vocabulary");
     cudaStream_t st = c->stream;
     for (int done = 0; done < n_tokens;) {
-        const int n = std::min(chunk_max, n_tokens - done), pos0 = start_pos + done;
+        // without memory for the workspace of the many-row path the portion goes through the smaller passes
+        const bool many = prompt_takes(m, n_tokens - done) && prompt_reserve(m, n_tokens - done) == JUNO_OK;
+        const int n = std::min(many ? std::min(m->prompt.rows, kPromptRows) : chunk_max, n_tokens - done), pos0 = start_pos + done;
         JUNO_TRY(step_sync(m));  // the pinned step buffer is reused
         JUNO_TRY(seq_reserve(seq, pos0, pos0 + n, st));
+        int32_t *h = many ? m->prompt.h_step : m->h_step, *d = many ? m->prompt.step : m->d_step;
+        const int ld = many ? m->prompt.rows : B;
         for (int i = 0; i < n; i++) {
-            m->h_step[i] = token_ids[done + i];
-            m->h_step[B + i] = pos0 + i;
-            m->h_step[2 * B + i] = seq->slot;
-            m->h_step[3 * B + i] = pos0 + i + 1;
+            h[i] = token_ids[done + i];
+            h[ld + i] = pos0 + i;
+            h[2 * ld + i] = seq->slot;
+            h[3 * ld + i] = pos0 + i + 1;
         }
-        JUNO_CUDA_TRY(cudaMemcpyAsync(m->d_step, m->h_step, (size_t)4 * B * 4, cudaMemcpyHostToDevice, st));
+        JUNO_CUDA_TRY(cudaMemcpyAsync(d, h, (size_t)4 * ld * 4, cudaMemcpyHostToDevice, st));
         c->h2d_bytes += 4 * n * 4;
+        int px = 0;                             // x[px] of the many-row path
         std::vector<std::pair<int, int>> rows;  // (row of this pass, index into want)
         for (int k = 0; k < n_want; k++)
             if (want[k] >= done && want[k] < done + n) rows.emplace_back(want[k] - done, k);
-        const int32_t *d_tok = m->d_step, *d_pos = m->d_step + B, *d_slot = m->d_step + 2 * B, *d_len = m->d_step + 3 * B;
+        const int32_t *d_tok = d, *d_pos = d + ld, *d_slot = d + 2 * ld, *d_len = d + 3 * ld;
         if (m->stack) {
             RowSet rs;
             rs.n = n;
@@ -1399,19 +1620,26 @@ static int prefill_run(juno_model *m, juno_seq *seq, const int32_t *token_ids, i
             juno_qmat *e = m->tok_embd;
             dim3 grid((f.hidden + 255) / 256, n);
             int64_t rb = e->tiled ? 0 : e->cols / raw_block_elems(e->type) * raw_block_bytes(e->type);
-            embed_kernel<<<grid, 256, 0, st>>>(e->type, e->tiled, e->dev, e->nb, rb, f.hidden, V, d_tok, m->x[0]);
+            embed_kernel<<<grid, 256, 0, st>>>(e->type, e->tiled, e->dev, e->nb, rb, f.hidden, V, d_tok, many ? m->prompt.x[0] : m->x[0]);
             JUNO_CUDA_TRY(cudaGetLastError());
             c->kernel_launches++;
-            JUNO_TRY(launch_rope_table(c, d_pos, n, m->hd, f.rope_theta, m->rope_cs, st));
+            JUNO_TRY(launch_rope_table(c, d_pos, n, m->hd, f.rope_theta, many ? m->prompt.cs : m->rope_cs, st));
             int cur = 0;
-            JUNO_TRY(enqueue_layers_batched(m, n, d_slot, d_len, n_splits, cur, st, d_pos, !rows.empty()));
+            if (many)
+                JUNO_TRY(enqueue_layers_prompt(m, n, pos0, cur, st));
+            else
+                JUNO_TRY(enqueue_layers_batched(m, n, d_slot, d_len, n_splits, cur, st, d_pos, !rows.empty()));
             m->last_x = cur;
+            px = cur;
         }
         m->last_n = n;
         c->forward_calls++;
         for (size_t i0 = 0; i0 < rows.size();) {
-            // a stack computes the wanted rows only, as many as the buffer holds at a time; the quantised layers have computed all
-            size_t i1 = m->stack ? std::min(rows.size(), i0 + (size_t)m->logit_cap) : rows.size();
+            // a stack and the many-row path compute the wanted rows only, as many as the buffer holds at a time; the smaller passes
+            // of the quantised layers have computed all
+            const bool some = m->stack || many;
+            size_t i1 = some ? std::min(rows.size(), i0 + (size_t)(many ? std::min(f.max_batch, kGemmMaxBatch) : m->logit_cap)) : rows.size();
+            if (many) JUNO_TRY(prompt_logits(m, &rows[i0], (int)(i1 - i0), px, st));
             if (m->stack) {
                 std::vector<int32_t> idx;
                 for (size_t i = i0; i < i1; i++) idx.push_back(rows[i].first);
@@ -1419,9 +1647,9 @@ static int prefill_run(juno_model *m, juno_seq *seq, const int32_t *token_ids, i
                 JUNO_TRY(stack_enqueue_logits(c, m->stack, m->stack->row_idx, (int)idx.size(), m->logits_loc, st));
             }
             for (size_t i = i0; i < i1;) {
-                const int src = m->stack ? (int)(i - i0) : rows[i].first;
+                const int src = some ? (int)(i - i0) : rows[i].first;
                 size_t run = 1;  // rows that lie side by side at both ends travel as one copy
-                while (i + run < i1 && rows[i + run].second == rows[i].second + (int)run && (m->stack || rows[i + run].first == src + (int)run)) run++;
+                while (i + run < i1 && rows[i + run].second == rows[i].second + (int)run && (some || rows[i + run].first == src + (int)run)) run++;
                 if (logits_host) {
                     JUNO_CUDA_TRY(cudaMemcpyAsync(logits_host + (size_t)rows[i].second * V, m->logits_loc + (size_t)src * m->vocab_loc, run * V * 4, cudaMemcpyDeviceToHost, st));
                     c->d2h_bytes += (int64_t)run * V * 4;
@@ -1432,7 +1660,7 @@ static int prefill_run(juno_model *m, juno_seq *seq, const int32_t *token_ids, i
                 LogitsView lv;
                 lv.n = 1;
                 lv.vocab = V;
-                lv.base = m->logits_loc + (size_t)(m->stack ? i1 - 1 - i0 : rows[i1 - 1].first) * m->vocab_loc;
+                lv.base = m->logits_loc + (size_t)(some ? i1 - 1 - i0 : rows[i1 - 1].first) * m->vocab_loc;
                 lv.vloc = V;
                 argmax_partial_kernel<<<dim3(kArgmaxBlocks, 1), 256, 0, st>>>(lv, m->d_pval, m->d_pidx);
                 argmax_final_kernel<<<1, 64, 0, st>>>(m->d_pval, m->d_pidx, 1, m->d_argmax);
@@ -1442,6 +1670,11 @@ static int prefill_run(juno_model *m, juno_seq *seq, const int32_t *token_ids, i
                 c->d2h_bytes += 4;
             }
             i0 = i1;
+        }
+        if (many && done + n == n_tokens) {  // the residual rows that juno_model_last_hidden can be asked for
+            m->last_n = (n - 1) % chunk_max + 1;
+            m->last_x = 0;
+            JUNO_TRY(launch_gather_rows(c, m->prompt.x[px], m->prompt.proj, nullptr, n - m->last_n, m->last_n, f.hidden, m->x[0], st));
         }
         done += n;
     }

@@ -29,6 +29,18 @@ struct JunoGraph {
     int seen = 0;
 };
 
+// Workspace of a prompt pass of the quantised layers (prompt.cuh): rows of one pass, and one matrix in FP16.  Made by the first
+// prompt that needs it, grown by longer ones, kept until the model is freed.
+struct JunoPrompt {
+    int rows = 0;
+    uint8_t *dev = nullptr;  // one allocation, carved up below
+    float *x[2], *qkv, *att, *proj, *hdn, *scale;
+    void *img, *w16;
+    float2 *cs;
+    int32_t *step;           // tokens | positions | lengths | slots, `rows` each
+    int32_t *h_step = nullptr;  // pinned mirror
+};
+
 struct juno_model {
     uint32_t magic;
     juno_ctx *ctx;
@@ -60,6 +72,7 @@ struct juno_model {
     float *d_pval = nullptr;
     int out_ids_cap = 0;
     int32_t *h_step = nullptr;  // pinned mirror of d_step
+    JunoPrompt prompt;
     int last_n = 0, last_x = 0;
     double step_kv_bytes = 0;  // K+V bytes one layer's attention reads in the current step
     std::map<uint64_t, JunoGraph> graphs;

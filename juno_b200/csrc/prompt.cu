@@ -1,0 +1,504 @@
+// Prompts of the quantised LLaMA layers: FP16 operands of the row products, and flash attention over FP16 pages.
+//
+// A pass takes up to some thousand positions, so a product is bound by the tensor cores and a weight is met by every row of the
+// pass: the quantised tiles are turned into FP16 rows once per pass and matrix (one read of the blocks, one write of 2 bytes a
+// weight) and the product itself is the one of the dense layers (gemm_rows_tc.cu).  Measured on whole prompts against passes of
+// 64 positions through the batched kernels (gemm.cu, gemm_tc.cu, decode attention), which read every block 32 times: Llama-3-8B
+// Q4_K_M, 2048 positions 368.9 -> 41.9 ms; TinyLlama Q8_0, 333 positions 22.8 -> 3.51 ms.
+#include <cuda_fp16.h>
+
+#include <algorithm>
+#include <cstring>
+
+#include "dequant.cuh"
+#include "mma_bf16.cuh"
+#include "prompt.cuh"
+#include "tile_math.cuh"
+
+namespace juno {
+
+// ───────────────────────────── weights ────────────────────────────────────────────────────
+// Integers below 256 as exact floats without a conversion instruction: byte k of w in the low bits of 2^23.
+__device__ __forceinline__ float byte_f32(uint32_t w, int k) {
+    return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440 + k)) - 8388608.f;
+}
+__device__ __forceinline__ uint32_t pack_f16(float a, float b) {
+    const __half2 h = __floats2half2_rn(a, b);
+    return *reinterpret_cast<const uint32_t *>(&h);
+}
+// The eight values of one row and 32-column block: columns 4c..4c+3 and 16+4c..16+4c+3 (the order of prompt_col).
+__device__ __forceinline__ void put8(__half *dst, const float (&v)[8]) {
+    *reinterpret_cast<uint4 *>(dst) = make_uint4(pack_f16(v[0], v[1]), pack_f16(v[2], v[3]), pack_f16(v[4], v[5]), pack_f16(v[6], v[7]));
+}
+
+__device__ __forceinline__ void dequant_tile(const TileRegs<12> &R, __half *row_r, __half *row_q, int lane) {
+    const int c = lane & 3;
+#pragma unroll
+    for (int half = 0; half < 2; half++) {
+        const uint32_t dm = half ? R.dm1 : R.dm0, sm = half ? R.sm1 : R.sm0;
+        const float d = f16bits_to_f32(dm), dmin = f16bits_to_f32(dm >> 16);
+        // this lane's two sub-blocks 2c, 2c+1; the others' come from the quad
+        const float s0 = d * byte_f32(sm, 0), s1 = d * byte_f32(sm, 1), m0 = dmin * byte_f32(sm, 2), m1 = dmin * byte_f32(sm, 3);
+        __half *row = half ? row_q : row_r;
+#pragma unroll
+        for (int g = 0; g < 4; g++) {
+            const int src = (lane & ~3) | g;
+            const float a = __shfl_sync(0xffffffffu, s0, src), b = __shfl_sync(0xffffffffu, s1, src);
+            const float am = __shfl_sync(0xffffffffu, m0, src), bm = __shfl_sync(0xffffffffu, m1, src);
+            const uint32_t w0 = half ? R.q[g].z : R.q[g].x, w1 = half ? R.q[g].w : R.q[g].y;
+            float v[8];
+#pragma unroll
+            for (int t = 0; t < 4; t++) {
+                v[t] = fmaf(a, byte_f32(w0 & 0x0F0F0F0Fu, t), -am);
+                v[4 + t] = fmaf(a, byte_f32(w1 & 0x0F0F0F0Fu, t), -am);
+            }
+            put8(row + g * 64 + c * 8, v);
+#pragma unroll
+            for (int t = 0; t < 4; t++) {
+                v[t] = fmaf(b, byte_f32((w0 >> 4) & 0x0F0F0F0Fu, t), -bm);
+                v[4 + t] = fmaf(b, byte_f32((w1 >> 4) & 0x0F0F0F0Fu, t), -bm);
+            }
+            put8(row + g * 64 + 32 + c * 8, v);
+        }
+    }
+}
+__device__ __forceinline__ void dequant_tile(const TileRegs<14> &R, __half *row_r, __half *row_q, int lane) {
+    const int c = lane & 3;
+#pragma unroll
+    for (int half = 0; half < 2; half++) {
+        const float d = f16bits_to_f32(half ? R.d01 >> 16 : R.d01);
+        const uint32_t sc = half ? R.sc1 : R.sc0;  // scales of the sub-blocks 4c..4c+3
+        __half *row = half ? row_q : row_r;
+        float s[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) s[k] = d * i8_to_f32(sc, k);
+#pragma unroll
+        for (int m = 0; m < 4; m++) {
+            const uint32_t WA = half ? R.ql[m].z : R.ql[m].x, WB = half ? R.ql[m].w : R.ql[m].y;
+            const uint4 hq = R.qh[m >> 1];
+            const uint32_t H = half ? ((m & 1) ? hq.w : hq.z) : ((m & 1) ? hq.y : hq.x);
+            const uint32_t V[4] = {(WA & 0x0F0F0F0Fu) | (H & 0x30303030u), ((WA >> 4) & 0x0F0F0F0Fu) | ((H >> 2) & 0x30303030u),
+                                   (WB & 0x0F0F0F0Fu) | ((H << 2) & 0x30303030u), ((WB >> 4) & 0x0F0F0F0Fu) | ((H << 4) & 0x30303030u)};
+            const int src = (lane & ~3) | m;
+#pragma unroll
+            for (int k = 0; k < 4; k += 2) {  // two 16-column sub-blocks make a group of 32; bytes hold columns 4c + 0, 2, 1, 3
+                const float sa = __shfl_sync(0xffffffffu, s[k], src), sb = __shfl_sync(0xffffffffu, s[k + 1], src);
+                float v[8];
+#pragma unroll
+                for (int t = 0; t < 4; t++) {
+                    const int byte = feed_pos(t);
+                    v[t] = sa * (byte_f32(V[k], byte) - 32.f);
+                    v[4 + t] = sb * (byte_f32(V[k + 1], byte) - 32.f);
+                }
+                put8(row + m * 64 + (k >> 1) * 32 + c * 8, v);
+            }
+        }
+    }
+}
+__device__ __forceinline__ void dequant_tile(const TileRegs<8> &R, __half *row_r, __half *row_q, int lane) {
+    const int c = lane & 3;
+#pragma unroll
+    for (int half = 0; half < 2; half++) {
+        const uint4 dd = half ? R.d1 : R.d0;
+        const uint32_t dw[4] = {dd.x, dd.y, dd.z, dd.w};
+        __half *row = half ? row_q : row_r;
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            const float d = f16bits_to_f32((j & 1) ? dw[j >> 1] >> 16 : dw[j >> 1]);
+            const uint32_t w0 = (half ? R.q[j].z : R.q[j].x) ^ 0x80808080u, w1 = (half ? R.q[j].w : R.q[j].y) ^ 0x80808080u;
+            float v[8];
+#pragma unroll
+            for (int t = 0; t < 4; t++) {
+                v[t] = d * (byte_f32(w0, t) - 128.f);
+                v[4 + t] = d * (byte_f32(w1, t) - 128.f);
+            }
+            put8(row + j * 32 + c * 8, v);
+        }
+    }
+}
+
+struct DequantParams {
+    DequantSeg seg[3];
+    int tiles[3];  // tiles before the end of each segment
+    int nseg, nb, K;
+    __half *out;
+};
+// Bound by the writes of 2 bytes a weight: Q4_K takes about 5 instructions a weight, less than half of what an SM issues while it
+// writes them.  One warp per 16 x 256 tile; neighbouring warps take neighbouring tiles of a row tile, so a CTA writes whole 4 KB pieces of rows.
+__global__ void __launch_bounds__(256) dequant_rows_kernel(const DequantParams p) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int tile = blockIdx.x * 8 + warp;
+    int s = 0;
+    while (s < p.nseg && tile >= p.tiles[s]) s++;
+    pdl_launch_dependents();
+    if (s >= p.nseg) return;
+    const int t = tile - (s ? p.tiles[s - 1] : 0), rt = t / p.nb, sb = t - rt * p.nb;
+    const size_t row0 = (size_t)((s ? p.tiles[s - 1] / p.nb : 0) + rt) * 16 + (lane >> 2);
+    __half *row_r = p.out + row0 * p.K + sb * 256, *row_q = row_r + (size_t)8 * p.K;
+    const int type = p.seg[s].type;
+    const uint8_t *src = p.seg[s].w + (size_t)t * tile_bytes(type);
+    if (type == 12) {
+        TileRegs<12> R;
+        load_tile<12>(R, src, lane);
+        pdl_wait();  // the product before this one may still read the rows that are written here
+        dequant_tile(R, row_r, row_q, lane);
+    } else if (type == 14) {
+        TileRegs<14> R;
+        load_tile<14>(R, src, lane);
+        pdl_wait();
+        dequant_tile(R, row_r, row_q, lane);
+    } else {
+        TileRegs<8> R;
+        load_tile<8>(R, src, lane);
+        pdl_wait();
+        dequant_tile(R, row_r, row_q, lane);
+    }
+}
+
+int launch_dequant_rows(juno_ctx *c, const DequantSeg *seg, int nseg, int K, void *out, cudaStream_t st) {
+    JUNO_REQUIRE(nseg >= 1 && nseg <= 3 && K > 0 && K % 256 == 0 && out, "dequantise: bad arguments (K=%d)", K);
+    DequantParams p;
+    memset((void *)&p, 0, sizeof(p));
+    p.nseg = nseg;
+    p.nb = K / 256;
+    p.K = K;
+    p.out = static_cast<__half *>(out);
+    int tiles = 0;
+    double bytes = 0;
+    for (int s = 0; s < nseg; s++) {
+        JUNO_REQUIRE(seg[s].w && (seg[s].type == 12 || seg[s].type == 14 || seg[s].type == 8), "dequantise: type %d has no tiles", seg[s].type);
+        p.seg[s] = seg[s];
+        tiles += seg[s].row_tiles * p.nb;
+        p.tiles[s] = tiles;
+        bytes += (double)seg[s].row_tiles * p.nb * (tile_bytes(seg[s].type) + 8192);
+    }
+    ProfScope prof(c, st, PROF_OTHER, bytes);
+    JUNO_CUDA_TRY(launch_pdl(dequant_rows_kernel, dim3((unsigned)((tiles + 7) / 8)), dim3(256), 0, st, p));
+    c->kernel_launches++;
+    return JUNO_OK;
+}
+
+// ───────────────────────────── activations ────────────────────────────────────────────────
+constexpr int kStageThreads = 256;
+__global__ void __launch_bounds__(kStageThreads) stage_rows_kernel(const StageRowsArgs a) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, K = a.K;
+    const size_t row = blockIdx.x;
+    __shared__ float red[8], redm[8];
+    pdl_wait();
+    pdl_launch_dependents();
+    const float *x = a.x + row * K, *add = a.add ? a.add + row * K : nullptr;
+    float *xo = a.x_out ? a.x_out + row * K : nullptr;
+    float ss = 0.f, vmax = 0.f;
+    for (int i = tid * 4; i < K; i += kStageThreads * 4) {
+        float4 v = *reinterpret_cast<const float4 *>(x + i);
+        if (add) {
+            const float4 b = *reinterpret_cast<const float4 *>(add + i);
+            v = make_float4(__fadd_rn(v.x, b.x), __fadd_rn(v.y, b.y), __fadd_rn(v.z, b.z), __fadd_rn(v.w, b.w));
+        }
+        if (xo) *reinterpret_cast<float4 *>(xo + i) = v;
+        if (a.normw) {
+            ss = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, ss))));
+            const float4 w = *reinterpret_cast<const float4 *>(a.normw + i);
+            v = make_float4(w.x * v.x, w.y * v.y, w.z * v.z, w.w * v.w);
+        }
+        vmax = fmaxf(fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))), vmax);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        vmax = fmaxf(vmax, __shfl_xor_sync(0xffffffffu, vmax, o));
+    }
+    if (lane == 0) {
+        red[warp] = ss;
+        redm[warp] = vmax;
+    }
+    __syncthreads();
+    ss = 0.f;
+#pragma unroll
+    for (int w = 0; w < kStageThreads / 32; w++) {
+        ss += red[w];
+        vmax = fmaxf(vmax, redm[w]);
+    }
+    const float inv = a.normw ? __fdiv_rn(1.f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, (float)K), a.eps))) : 1.f;
+    vmax *= inv;
+    // power of two that brings vmax into [256, 512) (1 for an all-zero or non-finite row)
+    float down = 1.f, up = 1.f;
+    if (vmax > 0.f && vmax < 3.0e38f) {
+        int e;
+        frexpf(vmax, &e);
+        down = ldexpf(1.f, 9 - e);
+        up = ldexpf(1.f, e - 9);
+    }
+    if (tid == 0) a.scale[row] = up;
+    __half *out = static_cast<__half *>(a.out) + row * K;
+    const float *src = xo ? xo : x;  // this thread's own stores
+    for (int i = tid * 4; i < K; i += kStageThreads * 4) {
+        float4 v = *reinterpret_cast<const float4 *>(src + i);
+        if (add && !xo) {
+            const float4 b = *reinterpret_cast<const float4 *>(add + i);
+            v = make_float4(__fadd_rn(v.x, b.x), __fadd_rn(v.y, b.y), __fadd_rn(v.z, b.z), __fadd_rn(v.w, b.w));
+        }
+        if (a.normw) {
+            const float4 w = *reinterpret_cast<const float4 *>(a.normw + i);
+            v = make_float4(__fmul_rn(__fmul_rn(w.x, v.x), inv), __fmul_rn(__fmul_rn(w.y, v.y), inv), __fmul_rn(__fmul_rn(w.z, v.z), inv),
+                            __fmul_rn(__fmul_rn(w.w, v.w), inv));
+        }
+        *reinterpret_cast<uint2 *>(out + prompt_col(i)) = make_uint2(pack_f16(v.x * down, v.y * down), pack_f16(v.z * down, v.w * down));
+    }
+}
+
+int launch_stage_rows(juno_ctx *c, const StageRowsArgs &a, cudaStream_t st) {
+    JUNO_REQUIRE(a.n > 0 && a.K > 0 && a.K % 32 == 0 && a.x && a.out && a.scale, "stage rows: bad arguments (K=%d, n=%d)", a.K, a.n);
+    ProfScope prof(c, st, PROF_OTHER, (double)a.n * a.K * 6);
+    JUNO_CUDA_TRY(launch_pdl(stage_rows_kernel, dim3((unsigned)a.n), dim3(kStageThreads), 0, st, a));
+    c->kernel_launches++;
+    return JUNO_OK;
+}
+
+__global__ void gather_rows_kernel(const float *x, const float *add, const int32_t *rows, int row0, int K, float *out) {
+    const int i = blockIdx.y, col = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
+    if (col >= K) return;
+    const size_t src = (size_t)(rows ? rows[i] : row0 + i) * K + col;
+    const float4 v = *reinterpret_cast<const float4 *>(x + src), b = *reinterpret_cast<const float4 *>(add + src);
+    *reinterpret_cast<float4 *>(out + (size_t)i * K + col) = make_float4(__fadd_rn(v.x, b.x), __fadd_rn(v.y, b.y), __fadd_rn(v.z, b.z), __fadd_rn(v.w, b.w));
+}
+int launch_gather_rows(juno_ctx *c, const float *x, const float *add, const int32_t *rows, int row0, int n, int K, float *out, cudaStream_t st) {
+    gather_rows_kernel<<<dim3((unsigned)((K / 4 + 127) / 128), (unsigned)n), 128, 0, st>>>(x, add, rows, row0, K, out);
+    JUNO_CUDA_TRY(cudaGetLastError());
+    c->kernel_launches++;
+    return JUNO_OK;
+}
+
+// ───────────────────────────── attention ──────────────────────────────────────────────────
+struct PromptAttnParams {
+    PromptAttnArgs a;
+    __half *k, *v;  // this layer's planes
+    const int32_t *table;
+    int max_pages, kv_heads, hd;
+    float scale_log2;
+};
+
+// One CTA per position: k of every key/value head rotated (rope :1657-1671), k and v rounded and stored.
+__global__ void __launch_bounds__(256) prompt_append_kernel(const PromptAttnParams p) {
+    const int r = blockIdx.x, pos = p.a.pos0 + r, half = p.hd / 2, pairs = p.kv_heads * half;
+    const int page = p.table[(size_t)*p.a.slot * p.max_pages + pos / kPageTokens];
+    const float *kx = p.a.qkv + (size_t)r * p.a.ld + p.a.n_heads * p.hd, *vx = kx + p.kv_heads * p.hd;
+    for (int i = threadIdx.x; i < pairs; i += blockDim.x) {
+        const int h = i / half, e = i - h * half;
+        const size_t dst = (((size_t)page * p.kv_heads + h) * kPageTokens + pos % kPageTokens) * p.hd + 2 * e;
+        const float2 cs = p.a.cs[(size_t)r * half + e], x = *reinterpret_cast<const float2 *>(kx + 2 * i), v = *reinterpret_cast<const float2 *>(vx + 2 * i);
+        *reinterpret_cast<__half2 *>(p.k + dst) = __floats2half2_rn(__fsub_rn(__fmul_rn(x.x, cs.x), __fmul_rn(x.y, cs.y)),
+                                                                  __fadd_rn(__fmul_rn(x.x, cs.y), __fmul_rn(x.y, cs.x)));
+        *reinterpret_cast<__half2 *>(p.v + dst) = __floats2half2_rn(v.x, v.y);
+    }
+}
+
+__device__ __forceinline__ void mma16816_f16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// (a, b) as FP16 and what the rounding left over, as FP16.
+__device__ __forceinline__ void split_f16(float a, float b, uint32_t &hi, uint32_t &lo) {
+    const __half2 h = __floats2half2_rn(a, b);
+    const float2 f = __half22float2(h);
+    hi = *reinterpret_cast<const uint32_t *>(&h);
+    lo = pack_f16(a - f.x, b - f.y);
+}
+
+// Causal flash attention: 64 rows of one query head per CTA, 16 per warp; 64 keys per step, keys and values double-buffered.
+// Queries and weights go to the tensor cores as two FP16 limbs each, as in the decode attention, so that scores and averages
+// keep FP32-level accuracy over the FP16 pages: twice the MMAs of a plain kernel, which makes their rate the bound.  The query
+// limbs live in registers for the whole row tile.
+constexpr int kPaKeys = 64, kPaThreads = 128, kPaRows = 64;
+template <int D>
+__global__ void __launch_bounds__(kPaThreads, 2) prompt_attn_kernel(const PromptAttnParams p) {
+    extern __shared__ __align__(16) uint8_t sm[];
+    constexpr int P = D + 8, KS = D / 16, CH = D / 8, RS = kPaThreads / CH;
+    __half *ks = reinterpret_cast<__half *>(sm), *vs = ks + 2 * kPaKeys * P;
+    const int h = blockIdx.x, r0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * kPaRows;  // long rows first
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    const int kvh = h / (p.a.n_heads / p.kv_heads);
+    const int32_t *table = p.table + (size_t)*p.a.slot * p.max_pages;
+    const int rows = min(kPaRows, p.a.n - r0), len = p.a.pos0 + r0 + rows;  // keys the tile's last row sees
+    const size_t page_stride = (size_t)p.kv_heads * kPageTokens * D, head_off = (size_t)kvh * kPageTokens * D;
+    const int lrow = tid / CH, lch = (tid % CH) * 8;
+    auto load_kv = [&](int j, int buf) {
+        const uint32_t kd = smem_addr(ks + (buf * kPaKeys + lrow) * P + lch), vd = smem_addr(vs + (buf * kPaKeys + lrow) * P + lch);
+#pragma unroll
+        for (int pg = 0; pg < kPaKeys / kPageTokens; pg++) {
+            const int key = j + pg * kPageTokens;
+            const size_t off = (key < len ? (size_t)table[key / kPageTokens] * page_stride : 0) + head_off + (size_t)lrow * D + lch;
+#pragma unroll
+            for (int r = 0; r < kPageTokens; r += RS) {
+                const bool ok = key + lrow + r < len;
+                const uint32_t d = (uint32_t)((pg * kPageTokens + r) * P) * 2;
+                cp16(kd + d, p.k + off + (ok ? (size_t)r * D : 0), ok);
+                cp16(vd + d, p.v + off + (ok ? (size_t)r * D : 0), ok);
+            }
+        }
+        cp_commit();
+    };
+    load_kv(0, 0);
+    // the A fragments of this warp's 16 rows: rotated, scaled into the log2 domain, split
+    const int row0 = r0 + warp * 16 + g, row1 = row0 + 8;
+    uint32_t qh[KS][4], ql[KS][4];
+    {
+        const size_t ra = (size_t)min(row0, p.a.n - 1), rb = (size_t)min(row1, p.a.n - 1);
+        const float *qa = p.a.qkv + ra * p.a.ld + h * D, *qb = p.a.qkv + rb * p.a.ld + h * D;
+        const float2 *ca = p.a.cs + ra * (D / 2), *cb = p.a.cs + rb * (D / 2);
+#pragma unroll
+        for (int k = 0; k < KS; k++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                const int col = k * 16 + (e >> 1) * 8 + 2 * t;
+                const float2 x = *reinterpret_cast<const float2 *>(((e & 1) ? qb : qa) + col), cs = ((e & 1) ? cb : ca)[col / 2];
+                const float y0 = __fsub_rn(__fmul_rn(x.x, cs.x), __fmul_rn(x.y, cs.y)), y1 = __fadd_rn(__fmul_rn(x.x, cs.y), __fmul_rn(x.y, cs.x));
+                split_f16(y0 * p.scale_log2, y1 * p.scale_log2, qh[k][e], ql[k][e]);
+            }
+    }
+    float o[2 * KS][4], mx[2] = {-INFINITY, -INFINITY}, ls[2] = {0.f, 0.f};
+#pragma unroll
+    for (int i = 0; i < 2 * KS; i++)
+#pragma unroll
+        for (int e = 0; e < 4; e++) o[i][e] = 0.f;
+    const int lr = lane & 15, lc = (lane >> 4) * 8, br = (lane & 7) + (lane >> 4) * 8, bc = ((lane >> 3) & 1) * 8;
+    const int wlast = p.a.pos0 + r0 + warp * 16 + 15;
+    int buf = 0;
+    for (int j = 0; j < len; j += kPaKeys, buf ^= 1) {
+        cp_wait<0>();
+        __syncthreads();
+        if (j + kPaKeys < len) load_kv(j + kPaKeys, buf ^ 1);
+        if (j > wlast) continue;  // every key of the tile lies behind this warp's rows
+        const __half *kt = ks + (size_t)buf * kPaKeys * P, *vt = vs + (size_t)buf * kPaKeys * P;
+        float s[kPaKeys / 8][4];
+#pragma unroll
+        for (int i = 0; i < kPaKeys / 8; i++) s[i][0] = s[i][1] = s[i][2] = s[i][3] = 0.f;
+#pragma unroll
+        for (int k = 0; k < KS; k++)
+#pragma unroll
+            for (int i = 0; i < kPaKeys / 16; i++) {
+                uint32_t b[4];
+                ldsm4(b, smem_addr(kt + (i * 16 + br) * P + k * 16 + bc));
+                mma16816_f16(s[2 * i], qh[k], b[0], b[1]);
+                mma16816_f16(s[2 * i + 1], qh[k], b[2], b[3]);
+                mma16816_f16(s[2 * i], ql[k], b[0], b[1]);
+                mma16816_f16(s[2 * i + 1], ql[k], b[2], b[3]);
+            }
+#pragma unroll
+        for (int e2 = 0; e2 < 2; e2++) {  // rows g and g + 8
+            const int pos = p.a.pos0 + r0 + warp * 16 + g + e2 * 8;
+            if (j + kPaKeys - 1 > pos) {
+#pragma unroll
+                for (int i = 0; i < kPaKeys / 8; i++)
+#pragma unroll
+                    for (int e = 0; e < 2; e++)
+                        if (j + i * 8 + 2 * t + e > pos) s[i][e2 * 2 + e] = -INFINITY;
+            }
+            float mv = mx[e2];
+#pragma unroll
+            for (int i = 0; i < kPaKeys / 8; i++) mv = fmaxf(mv, fmaxf(s[i][e2 * 2], s[i][e2 * 2 + 1]));
+            mv = fmaxf(mv, __shfl_xor_sync(0xffffffffu, mv, 1));
+            mv = fmaxf(mv, __shfl_xor_sync(0xffffffffu, mv, 2));
+            const float base = mv == -INFINITY ? 0.f : mv;  // no key seen yet in this row
+            const float f = ex2(mx[e2] - base);
+            mx[e2] = mv;
+            float sum = 0.f;
+#pragma unroll
+            for (int i = 0; i < kPaKeys / 8; i++)
+#pragma unroll
+                for (int e = 0; e < 2; e++) sum += s[i][e2 * 2 + e] = ex2(s[i][e2 * 2 + e] - base);
+            ls[e2] = fmaf(ls[e2], f, sum);
+#pragma unroll
+            for (int i = 0; i < 2 * KS; i++) {
+                o[i][e2 * 2] *= f;
+                o[i][e2 * 2 + 1] *= f;
+            }
+        }
+#pragma unroll
+        for (int kk = 0; kk < kPaKeys / 16; kk++) {
+            uint32_t ph[4], pl[4];
+            split_f16(s[2 * kk][0], s[2 * kk][1], ph[0], pl[0]);
+            split_f16(s[2 * kk][2], s[2 * kk][3], ph[1], pl[1]);
+            split_f16(s[2 * kk + 1][0], s[2 * kk + 1][1], ph[2], pl[2]);
+            split_f16(s[2 * kk + 1][2], s[2 * kk + 1][3], ph[3], pl[3]);
+#pragma unroll
+            for (int i = 0; i < KS; i++) {
+                uint32_t b[4];
+                ldsm4_trans(b, smem_addr(vt + (kk * 16 + lr) * P + i * 16 + lc));
+                mma16816_f16(o[2 * i], ph, b[0], b[1]);
+                mma16816_f16(o[2 * i + 1], ph, b[2], b[3]);
+                mma16816_f16(o[2 * i], pl, b[0], b[1]);
+                mma16816_f16(o[2 * i + 1], pl, b[2], b[3]);
+            }
+        }
+    }
+#pragma unroll
+    for (int e2 = 0; e2 < 2; e2++) {
+        float l = ls[e2];
+        l += __shfl_xor_sync(0xffffffffu, l, 1);
+        l += __shfl_xor_sync(0xffffffffu, l, 2);
+        const int row = e2 ? row1 : row0;
+        if (row >= p.a.n) continue;
+        const float f = 1.f / l;
+        float *out = p.a.out + ((size_t)row * p.a.n_heads + h) * D;
+#pragma unroll
+        for (int i = 0; i < 2 * KS; i++) *reinterpret_cast<float2 *>(out + i * 8 + 2 * t) = make_float2(o[i][e2 * 2] * f, o[i][e2 * 2 + 1] * f);
+    }
+}
+
+static int prompt_attn_params(const PromptAttnArgs &a, PromptAttnParams *p) {
+    JUNO_REQUIRE(a.pool && !a.pool->latent && a.pool->dtype == 0 && (a.pool->head_dim == 64 || a.pool->head_dim == 128) && a.n > 0 && a.pos0 >= 0 && a.qkv && a.cs &&
+                     a.slot && a.n_heads % a.pool->n_kv_heads == 0 && a.ld % 4 == 0,
+                 "prompt attention: bad arguments (n=%d)", a.n);
+    const juno_kvpool *pool = a.pool;
+    memset((void *)p, 0, sizeof(*p));
+    p->a = a;
+    p->hd = pool->head_dim;
+    p->kv_heads = pool->n_kv_heads;
+    const size_t plane = (size_t)a.layer * pool->n_pages * pool->n_kv_heads * kPageTokens * pool->head_dim;
+    p->k = static_cast<__half *>(pool->k) + plane;
+    p->v = static_cast<__half *>(pool->v) + plane;
+    p->table = pool->d_table;
+    p->max_pages = pool->max_pages_per_seq;
+    p->scale_log2 = (float)(1.0 / sqrt((double)p->hd)) * kLog2e;
+    return JUNO_OK;
+}
+
+int launch_prompt_append(juno_ctx *c, const PromptAttnArgs &a, cudaStream_t st) {
+    PromptAttnParams p;
+    JUNO_TRY(prompt_attn_params(a, &p));
+    ProfScope prof(c, st, PROF_ROPE_APPEND, 0);
+    prompt_append_kernel<<<(unsigned)a.n, 256, 0, st>>>(p);
+    JUNO_CUDA_TRY(cudaGetLastError());
+    c->kernel_launches++;
+    return JUNO_OK;
+}
+
+template <int D>
+static int prompt_attn_inst(juno_ctx *c, const PromptAttnParams &p, cudaStream_t st) {
+    constexpr size_t smem = (size_t)4 * kPaKeys * (D + 8) * 2;
+    static std::mutex mu;
+    static bool configured[16] = {false};
+    {
+        std::lock_guard<std::mutex> lk(mu);
+        if (!configured[c->device & 15]) {
+            JUNO_CUDA_TRY(cudaFuncSetAttribute(prompt_attn_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            configured[c->device & 15] = true;
+        }
+    }
+    prompt_attn_kernel<D><<<dim3((unsigned)p.a.n_heads, (unsigned)((p.a.n + kPaRows - 1) / kPaRows)), kPaThreads, smem, st>>>(p);
+    JUNO_CUDA_TRY(cudaGetLastError());
+    c->kernel_launches++;
+    return JUNO_OK;
+}
+
+int launch_prompt_attn(juno_ctx *c, const PromptAttnArgs &a, cudaStream_t st) {
+    JUNO_REQUIRE(a.out, "prompt attention: no output");
+    PromptAttnParams p;
+    JUNO_TRY(prompt_attn_params(a, &p));
+    ProfScope prof(c, st, PROF_ATTN, a.algo_bytes);
+    return p.hd == 64 ? prompt_attn_inst<64>(c, p, st) : prompt_attn_inst<128>(c, p, st);
+}
+
+}  // namespace juno

@@ -201,8 +201,7 @@ class B200TransformerHandler:
         return logits if want_logits else ids
 
     def prefill(self, request_id: str, token_ids, start_pos: int = 0, want_logits: bool = False):
-        """Chunked prompt prefill (juno_prefill): positions start_pos.. of one request in passes of up to
-        min(max_batch, 64) positions.  Returns the logits of the last position fed, or None."""
+        """Chunked prompt prefill (juno_prefill): positions start_pos.. of one request, many positions per pass.  Returns the logits of the last position fed, or None."""
         toks = np.ascontiguousarray(np.asarray(token_ids, dtype=np.int32))
         logits = np.empty(self.arch.vocab, dtype=np.float32) if want_logits else None
         check(self._L.juno_prefill(self.handle, self._seq(request_id), _ptr(toks), len(toks), int(start_pos),

@@ -74,7 +74,9 @@ int launch_gemm_rows(juno_ctx *c, int dt, const GemmArgs &a, unsigned *err, cuda
     const double es = dt_bytes(dt);
     const double algo = a.groups * ((double)a.M * a.K + (double)a.N * a.K) * es + (double)a.groups * a.M * a.N * (a.epi == GE_F32 ? 4.0 : es);
     ProfScope prof(c, st, PROF_GEMM_ROWS, algo);
-    if (dt == DT_BF16) return launch_gemm_rows_tc(c, a, err, st);
+    // Up to kFewRows rows the weights' way from memory is the bound, above them the MMAs.  A pass of Vosotar medium through the one
+    // and the other: 20 rows 0.75 and 1.34 ms, 100 rows 0.94 and 1.35, 128 rows 0.99 and 1.36; Desilorn small, 100 rows: 0.95 and 1.20.
+    if (dt == DT_BF16) return a.M <= kFewRows && !a.half ? launch_gemm_few_tc(c, a, err, st) : launch_gemm_rows_tc(c, a, err, st);
     const dim3 grid((unsigned)((a.N + kSimtTile - 1) / kSimtTile), (unsigned)((a.M + kSimtTile - 1) / kSimtTile), (unsigned)a.groups);
     gemm_simt_kernel<float><<<grid, 256, 0, st>>>(a);
     JUNO_CUDA_TRY(cudaGetLastError());

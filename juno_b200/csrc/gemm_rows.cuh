@@ -36,6 +36,8 @@ struct GemmArgs {
     const float *row_scale = nullptr;
 };
 int launch_gemm_rows_tc(juno_ctx *c, const GemmArgs &a, unsigned *err, cudaStream_t st);  // 16-bit operands, tcgen05
+constexpr int kFewRows = 128;                                                              // most rows of launch_gemm_few_tc
+int launch_gemm_few_tc(juno_ctx *c, const GemmArgs &a, unsigned *err, cudaStream_t st);  // the same for few rows, BF16
 int launch_gemm_rows(juno_ctx *c, int dt, const GemmArgs &a, unsigned *err, cudaStream_t st);
 
 }  // namespace juno

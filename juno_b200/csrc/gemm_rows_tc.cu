@@ -13,15 +13,15 @@
 #include <mutex>
 
 #include "gemm_rows.cuh"
+#include "tc5.cuh"
 #include "tile_math.cuh"
 
 namespace juno {
 
 using bf16 = __nv_bfloat16;
 
-constexpr int kBM = 128, kBK = 64, kTileThreads = 192;
+constexpr int kTileThreads = 192;
 constexpr int kMaxStages = 8;
-constexpr long long kWaitClocks = 400000000ll;  // about 0.2 s
 
 struct GemmTcParams {
     CUtensorMap ta, tw;
@@ -29,63 +29,6 @@ struct GemmTcParams {
     int m_tiles, n_tiles, n_work, k_steps, stages;
     unsigned *err;
 };
-
-__device__ __forceinline__ uint32_t s_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ bool bar_test(uint32_t bar, unsigned parity) {
-    unsigned ok;
-    asm volatile(
-        "{\n.reg .pred p;\n"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-        "selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-__device__ __forceinline__ bool bar_wait(uint32_t bar, unsigned parity, volatile unsigned *fail) {
-    if (bar_test(bar, parity)) return true;
-    const long long t0 = clock64();
-    for (;;) {
-        if (bar_test(bar, parity)) return true;
-        if (*fail) return false;
-        if (clock64() - t0 > kWaitClocks) break;
-    }
-    *fail = 1u;
-    return false;
-}
-__device__ __forceinline__ void tma_2d(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t bar) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
-                 "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar)
-                 : "memory");
-}
-// K-major operand with 128-byte swizzle: rows of 128 bytes, groups of eight rows 1024 bytes apart.
-__device__ __forceinline__ uint64_t sw128_desc(uint32_t saddr) {
-    return (uint64_t)((saddr >> 4) & 0x3FFFu) | (uint64_t)1 << 16 | (uint64_t)(1024 >> 4) << 32 | (uint64_t)1 << 46 | (uint64_t)2 << 61;
-}
-__device__ __forceinline__ void mma_bf16(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
-    asm volatile(
-        "{\n.reg .pred p;\n"
-        "setp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
-        "l"(a), "l"(b), "r"(idesc), "r"(acc)
-        : "memory");
-}
-__device__ __forceinline__ void mma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,"
-        "%29,%30,%31}, [%32];\n"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]),
-          "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]),
-          "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-        : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
-__device__ __forceinline__ float fast_sigmoid(float z) { return __fdividef(1.f, 1.f + __expf(-z)); }
-__device__ __forceinline__ float fast_geglu(float z, float v) { return z * v * fast_sigmoid(1.5957691216057308f * fmaf(0.044715f * z * z, z, z)); }
 
 // 32 columns of one output row.  nv = columns that exist (0..32).
 template <int EPI>
@@ -309,7 +252,6 @@ static EncodeTiled encode_tiled() {
     return fn;
 }
 
-// Row-major matrix of 16-bit elements [rows][cols] with pitch ld, boxes of box_rows x 64 columns.
 int tensor_map_bf16(CUtensorMap *map, const void *base, int64_t rows, int64_t cols, int64_t ld, int box_rows) {
     EncodeTiled enc = encode_tiled();
     JUNO_REQUIRE(enc, "the driver has no cuTensorMapEncodeTiled");

@@ -57,6 +57,8 @@ SIGNATURES = {
     "juno_device_total_mem": (C.c_int, [I32, C.POINTER(I64)]),
     "juno_ctx_create": (C.c_int, [I32, PP]),
     "juno_ctx_destroy": (C.c_int, [P]),
+    "juno_host_alloc": (C.c_int, [P, I64, PP]),
+    "juno_host_free": (C.c_int, [P]),
     "juno_ctx_device": (C.c_int, [P, C.POINTER(I32)]),
     "juno_ctx_synchronize": (C.c_int, [P]),
     "juno_ctx_counters": (C.c_int, [P, C.POINTER(Counters), I32]),

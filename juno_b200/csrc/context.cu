@@ -1,5 +1,7 @@
 // Context, device discovery, error text and the MatVec-operator entry points of the C ABI.
 #include <cstring>
+#include <map>
+#include <mutex>
 #include <string>
 
 #include "common.cuh"
@@ -65,11 +67,71 @@ int ensure_pinned(juno_ctx *c, size_t want) {
     return JUNO_OK;
 }
 
+// Page-locked blocks for results that a host reads.  One pool for the process, because a result may outlive the context that wrote
+// it; blocks come in powers of two, at most kHostPoolBytes of them in all, and those that nobody holds are given back when a
+// context closes or another size needs the room.
+constexpr size_t kHostPoolBytes = (size_t)96 << 20, kHostBlockMin = (size_t)256 << 10;
+struct HostPool {
+    std::mutex mu;
+    std::map<void *, size_t> held;
+    std::multimap<size_t, void *> idle;
+    size_t total = 0;
+    void release_idle() {
+        for (auto &b : idle) {
+            cudaFreeHost(b.second);
+            total -= b.first;
+        }
+        idle.clear();
+    }
+};
+static HostPool &host_pool() {
+    static HostPool *p = new HostPool();  // never destroyed: results may be dropped while the process exits
+    return *p;
+}
+
 }  // namespace juno
 
 using namespace juno;
 
 extern "C" {
+
+int juno_host_alloc(juno_ctx *c, int64_t bytes, void **out) {
+    JUNO_TRY(ctx_check(c));
+    JUNO_REQUIRE(out && bytes > 0, "bad host allocation (%lld bytes)", (long long)bytes);
+    size_t size = kHostBlockMin;
+    while (size < (size_t)bytes && size < kHostPoolBytes) size *= 2;
+    HostPool &h = host_pool();
+    std::lock_guard<std::mutex> lk(h.mu);
+    const auto it = h.idle.find(size);
+    if (it != h.idle.end() && size >= (size_t)bytes) {
+        *out = it->second;
+        h.held[it->second] = size;
+        h.idle.erase(it);
+        return JUNO_OK;
+    }
+    DeviceGuard g(c->device);
+    if (h.total + size > kHostPoolBytes) h.release_idle();
+    void *p = nullptr;
+    if (size < (size_t)bytes || h.total + size > kHostPoolBytes || cudaHostAlloc(&p, size, cudaHostAllocPortable) != cudaSuccess) {
+        cudaGetLastError();
+        set_error("no page-locked block of %lld bytes is free", (long long)bytes);
+        return JUNO_ERR_OOM;
+    }
+    h.total += size;
+    h.held[p] = size;
+    *out = p;
+    return JUNO_OK;
+}
+
+int juno_host_free(void *block) {
+    HostPool &h = host_pool();
+    std::lock_guard<std::mutex> lk(h.mu);
+    const auto it = h.held.find(block);
+    JUNO_REQUIRE(it != h.held.end(), "not a block of juno_host_alloc");
+    h.idle.emplace(it->second, block);
+    h.held.erase(it);
+    return JUNO_OK;
+}
 
 const char *juno_last_error(void) { return get_error(); }
 
@@ -155,6 +217,11 @@ int juno_ctx_destroy(juno_ctx *c) {
     if (c->stage_y) cudaFree(c->stage_y);
     if (c->pinned) cudaFreeHost(c->pinned);
     cudaStreamDestroy(c->stream);
+    {
+        HostPool &h = host_pool();
+        std::lock_guard<std::mutex> hk(h.mu);
+        h.release_idle();
+    }
     c->magic = kMagicDead;  // record kept: a second destroy reports CLOSED
     return JUNO_OK;
 }

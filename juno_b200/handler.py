@@ -192,7 +192,7 @@ class B200TransformerHandler:
         seqs = (C.c_void_p * n)(*[self._seq(r).value for r in request_ids])
         tok = np.array([t[-1] if hasattr(t, "__len__") else t for t in tokens], dtype=np.int32)
         pos = np.asarray(positions, dtype=np.int32)
-        logits = np.empty((n, self.arch.vocab), dtype=np.float32) if want_logits else None
+        logits = self.ctx.host_rows(n, self.arch.vocab) if want_logits else None
         ids = np.empty(n, dtype=np.int32) if want_argmax else None
         check(self._L.juno_forward(self.handle, n, seqs, _ptr(tok), _ptr(pos), _ptr(logits) if want_logits else None,
                                    _ptr(ids) if want_argmax else None), "juno_forward")
@@ -212,7 +212,7 @@ class B200TransformerHandler:
         """One portion of a prompt (juno_prefill_logits): logits [len(want), vocab] at the given places of the portion."""
         toks = np.ascontiguousarray(np.asarray(token_ids, dtype=np.int32))
         idx = np.ascontiguousarray(np.asarray(list(want), dtype=np.int32))
-        logits = np.empty((len(idx), self.arch.vocab), dtype=np.float32)
+        logits = self.ctx.host_rows(len(idx), self.arch.vocab)
         check(self._L.juno_prefill_logits(self.handle, self._seq(request_id), _ptr(toks), len(toks), int(start_pos), len(idx), _ptr(idx),
                                           _ptr(logits)), "juno_prefill_logits")
         return logits

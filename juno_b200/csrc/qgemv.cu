@@ -63,6 +63,7 @@ struct QParams {
     const unsigned *epoch;
     unsigned *peer_failed;
     unsigned *err;  // device word: a wait on a weight tile gave up (code | warp << 8 | block << 16)
+    int splits;     // SPLIT kernels: CTAs of a cluster that share K
 };
 
 // ───────────────────────────── shared-memory operand ──────────────────────────────────────
@@ -410,7 +411,7 @@ __device__ __forceinline__ void quantize_fetch(const QSrc &q, int b, int sb, int
 
 // nw: the RMSNorm weights of the lane's columns.
 template <int TYPE>
-__device__ __forceinline__ void quantize_slice(const QSrc &q, int b, int sb, int lane, const QIn &in, const float (&nw)[8],
+__device__ __forceinline__ void quantize_slice(const QSrc &q, bool store, int b, int sb, int lane, const QIn &in, const float (&nw)[8],
                                                uint8_t *blk, float &ss_out) {
     using B = XBlk<TYPE>;
     const int c0 = sb * 256 + lane * 8;
@@ -422,7 +423,7 @@ __device__ __forceinline__ void quantize_slice(const QSrc &q, int b, int sb, int
 #pragma unroll
         for (int i = 0; i < 8; i++) v[i] = __fadd_rn(v[i], in.s[i]);
     }
-    if (q.x_store && blockIdx.x == 0) {
+    if (q.x_store && store) {
         float *dst = q.x_store + roff;
         *reinterpret_cast<float4 *>(dst) = make_float4(v[0], v[1], v[2], v[3]);
         *reinterpret_cast<float4 *>(dst + 4) = make_float4(v[4], v[5], v[6], v[7]);
@@ -581,28 +582,48 @@ struct QCursor {
     int R, sb;    // row tile and block of tile f
 };
 
+__device__ __forceinline__ void qcluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void qcluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ float qpeer_ld(uint32_t addr, int rank) {
+    uint32_t a;
+    float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+    return v;
+}
+// Floats of the exchange of a SPLIT kernel: two buffers of a chunk's sums (all sixteen rows of its row tiles), then the sums of squares.
+__host__ __device__ constexpr int qexchange_floats(int bc) { return 2 * kQChunk * 16 * bc + 8; }
+
+// SPLIT: the CTAs of a cluster share a range of row tiles and each takes its part of K, so that the operand of three to eight
+// sequences fits beside the ring in one pass over the weights (K = 14336: 47 KB a sequence) and every CTA converts its part of the
+// input only.  The sums of a chunk meet over distributed shared memory while the next chunk is multiplied; they are added in rank
+// order, each CTA finishing its share of the outputs.
 // TAGGED: the addends are (value, step number) pairs from other GPUs (a kernel of its own, so that the polling loads
 // cost the single-GPU kernels no registers).
-template <int TYPE, int NT, int OCC, bool TAGGED>
+template <int TYPE, int NT, int OCC, bool TAGGED, bool SPLIT>
 __global__ void __launch_bounds__(kQThreads, OCC) qgemv_kernel(const QParams p) {
+    static_assert(!(TAGGED && SPLIT), "peer exchange runs without a split of K");
     using B = XBlk<TYPE>;
     constexpr int NSEQ = 2 * NT;
     extern __shared__ __align__(128) uint8_t smem[];
     pdl_launch_dependents();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int NB = p.NB;
+    const int rank = SPLIT ? (int)(blockIdx.x % (unsigned)p.splits) : 0;
+    const int sb_first = SPLIT ? p.NB * rank / p.splits : 0, NB = (SPLIT ? p.NB * (rank + 1) / p.splits : p.NB) - sb_first;  // this CTA's part of K
+    const int NBX = SPLIT ? (p.NB + p.splits - 1) / p.splits : p.NB;  // blocks the operand has room for
     // [ring: 16 warps x ring x slot_bytes][operand: bc x NB blocks][partials: kQBufs x 16 warps x 2 row tiles x 16 rows x NSEQ][ssw][rs][mbarriers]
     const size_t ring_bytes = (size_t)kQWarps * p.ring * p.slot_bytes;
     uint8_t *xop = smem + ring_bytes;
-    float *red = reinterpret_cast<float *>(xop + (size_t)p.bc * NB * B::bytes);
+    float *red = reinterpret_cast<float *>(xop + (size_t)p.bc * NBX * B::bytes);
     float *ssw = red + kQBufs * kQWarps * 2 * 16 * NSEQ;  // [16 warps][8] sums of squares of the slices a warp converted
     float *rs_s = ssw + kQWarps * 8;                  // [8] 1/rms per sequence
     const uint32_t my_ring = smem_u32(smem) + (uint32_t)(warp * p.ring * p.slot_bytes);
     int *wr_s = reinterpret_cast<int *>(rs_s + 16);   // [kQBufs][kQChunk] first | last << 8 warp of a row tile of the chunk
     const uint32_t my_bars = smem_u32(wr_s + kQBufs * kQChunk) + (uint32_t)(warp * p.ring * 8);
+    float *xch = reinterpret_cast<float *>(wr_s + kQBufs * kQChunk) + kQWarps * p.ring * 2;  // SPLIT: [2][sums of a chunk], [8] sums of squares
 
     int rt0, rtc;
-    qsplit_cta((int)blockIdx.x, (int)gridDim.x, p.total_rt, rt0, rtc);
+    qsplit_cta(SPLIT ? (int)(blockIdx.x / (unsigned)p.splits) : (int)blockIdx.x, SPLIT ? (int)(gridDim.x / (unsigned)p.splits) : (int)gridDim.x, p.total_rt, rt0, rtc);
     const int n_chunks = qsplit_chunks(rtc);
     auto chunk_lo = [&](int k) { return qsplit_chunk_lo(rt0, rtc, n_chunks, k); };
 
@@ -630,7 +651,7 @@ __global__ void __launch_bounds__(kQThreads, OCC) qgemv_kernel(const QParams p) 
         if (pc.k >= n_chunks) return;
         if (pc_fresh) {  // consecutive tiles of a row tile are contiguous; the next row tile may belong to another matrix
             int ty;
-            pc_src = qtile_addr<TYPE>(p, pc.R, pc.sb, ty);
+            pc_src = qtile_addr<TYPE>(p, pc.R, sb_first + pc.sb, ty);
             pc_bytes = (unsigned)tile_bytes(ty);
             pc_fresh = false;
         }
@@ -657,7 +678,7 @@ __global__ void __launch_bounds__(kQThreads, OCC) qgemv_kernel(const QParams p) 
     // The RMSNorm weights are model data: those of the warp's first slice are requested before the wait, so that their
     // trip to DRAM overlaps the end of the producing kernel.
     float w8[8];
-    if (p.normw && warp < p.bc * NB) ld8(p.normw + (warp % NB) * 256 + lane * 8, w8);
+    if (p.normw && warp < p.bc * NB) ld8(p.normw + (sb_first + warp % NB) * 256 + lane * 8, w8);
     pdl_wait();  // everything below reads what earlier kernels of the stream wrote
     bool failed = false;
     const unsigned step_no = (p.tagged_adds || p.n_peers) ? *reinterpret_cast<const volatile unsigned *>(p.epoch) : 0u;
@@ -689,12 +710,12 @@ __global__ void __launch_bounds__(kQThreads, OCC) qgemv_kernel(const QParams p) 
         for (int b = 0; b < 8; b++) ss[b] = 0.f;
         const int pairs = p.bc * NB;
         for (int pr = warp; pr < pairs; pr += kQWarps) {
-            const int b = pr / NB, sb = pr - b * NB;
+            const int b = pr / NB, sb = sb_first + pr - b * NB;
             QIn t;
             quantize_fetch<TAGGED>(q, b, sb, lane, t);
             if (q.normw && pr != warp) ld8(q.normw + sb * 256 + lane * 8, w8);
             float part = 0.f;
-            quantize_slice<TYPE>(q, b, sb, lane, t, w8, xop + (size_t)pr * B::bytes, part);
+            quantize_slice<TYPE>(q, SPLIT ? blockIdx.x < (unsigned)p.splits : blockIdx.x == 0, b, sb, lane, t, w8, xop + (size_t)pr * B::bytes, part);
 #pragma unroll
             for (int bb = 0; bb < 8; bb++)
                 if (bb == b) ss[bb] += part;
@@ -712,7 +733,14 @@ __global__ void __launch_bounds__(kQThreads, OCC) qgemv_kernel(const QParams p) 
         }
     }
     __syncthreads();
-    if (tid < 8) {
+    if (SPLIT) {  // the norms need the other members' sums of squares: after the first exchange
+        if (tid < 8) {
+            float s = 0.f;
+#pragma unroll
+            for (int w8 = 0; w8 < kQWarps; w8++) s += ssw[w8 * 8 + tid];
+            xch[2 * kQChunk * 16 * p.bc + tid] = s;
+        }
+    } else if (tid < 8) {
         float sc = 1.f;
         if (p.normw) {
             float s = 0.f;
@@ -749,6 +777,40 @@ __global__ void __launch_bounds__(kQThreads, OCC) qgemv_kernel(const QParams p) 
     const uint32_t xop_s = smem_u32(xop);
     int slot = 0;
     unsigned parity = 0;
+    // SPLIT: the outputs of chunk k, once every member's sums are visible.
+    auto finish = [&](int k) {
+        const uint32_t xs = smem_u32(xch);
+        if (k == 0) {
+            if (tid < 8) {
+                float sc = 1.f;
+                if (p.normw) {
+                    float s = 0.f;
+                    for (int r = 0; r < p.splits; r++) s += qpeer_ld(xs + (2 * kQChunk * 16 * p.bc + tid) * 4, r);
+                    sc = __fdiv_rn(1.f, __fsqrt_rn(__fadd_rn(__fdiv_rn(s, (float)p.K), p.eps)));
+                }
+                rs_s[tid] = sc;
+            }
+            __syncthreads();
+        }
+        const int lo = chunk_lo(k), crt = chunk_lo(k + 1) - lo;
+        const uint32_t xb = xs + (uint32_t)((k & 1) * kQChunk * 16 * p.bc) * 4;
+        const int rows_sh = (p.epi == QEPI_SILU_PAIR) ? 3 : 4, rows_out = 1 << rows_sh, per_b = crt << rows_sh, total = per_b * p.bc;
+        for (int idx = total * rank / p.splits + tid; idx < total * (rank + 1) / p.splits; idx += kQThreads) {
+            const int b = idx / per_b, rg = idx - b * per_b, l = rg >> rows_sh, row = rg & (rows_out - 1);
+            const uint32_t at = xb + (uint32_t)((b * crt + l) * 16 + row) * 4;
+            const int Rg = lo + l, s = qseg_of(p, Rg), orow = (Rg - p.rt_begin[s]) * rows_out + row;
+            float v = 0.f, v2 = 0.f;
+            for (int r = 0; r < p.splits; r++) {
+                v += qpeer_ld(at, r);
+                if (p.epi == QEPI_SILU_PAIR) v2 += qpeer_ld(at + 32, r);
+            }
+            if (orow >= p.rows[s]) continue;
+            v = __fmul_rn(v, rs_s[b]);
+            if (p.epi == QEPI_SILU_PAIR) v = __fmul_rn(silu_f(v), __fmul_rn(v2, rs_s[b]));
+            p.out[s][(size_t)b * p.ld_out + orow] = v;
+        }
+        __syncwarp();
+    };
     for (int k = 0; k < n_chunks; k++) {
         const int lo = chunk_lo(k), crt = chunk_lo(k + 1) - lo, T = crt * NB;
         int f0, f1;
@@ -795,6 +857,30 @@ __global__ void __launch_bounds__(kQThreads, OCC) qgemv_kernel(const QParams p) 
         // thread has finished reading it.
         __syncthreads();
         // K spans of a row in warp order (a fixed order: results are bitwise repeatable), then the output transform
+        if constexpr (SPLIT) {
+            __syncwarp();
+            if (k > 0) {
+                qcluster_wait();
+                finish(k - 1);
+            }
+            // its buffer was last read by the peers before they arrived at the barrier that has just been waited for
+            float *xb = xch + (size_t)(k & 1) * kQChunk * 16 * p.bc;
+            const int per_b = crt * 16;
+            for (int idx = tid; idx < per_b * p.bc; idx += kQThreads) {
+                const int b = idx / per_b, rg = idx - b * per_b, l = rg >> 4, row = rg & 15, tlo = l * NB, wr = wr_s[(k & (kQBufs - 1)) * kQChunk + l];
+                float v = 0.f;
+                for (int w = wr & 255; w <= (wr >> 8); w++) {
+                    int wf0, wf1;
+                    qsplit_warp(w, T, wf0, wf1);
+                    if (wf0 >= wf1) continue;
+                    v += cred[w * (2 * 16 * NSEQ) + (wf0 < tlo ? 16 * NSEQ : 0) + b + row * NSEQ];
+                }
+                xb[idx] = v;
+            }
+            __syncwarp();
+            qcluster_arrive();
+            continue;
+        }
         const int rows_sh = (p.epi == QEPI_SILU_PAIR) ? 3 : 4, rows_out = 1 << rows_sh;
         const int per_b = crt << rows_sh, total = per_b * p.bc;
         for (int idx = tid; idx < total; idx += kQThreads) {
@@ -825,6 +911,13 @@ __global__ void __launch_bounds__(kQThreads, OCC) qgemv_kernel(const QParams p) 
             }
         }
     }
+    if constexpr (SPLIT) {
+        __syncwarp();
+        qcluster_wait();
+        finish(n_chunks - 1);
+        qcluster_arrive();
+        qcluster_wait();  // nobody leaves while its shared memory may still be read
+    }
 }
 
 // ───────────────────────────── host: launch ───────────────────────────────────────────────
@@ -833,7 +926,7 @@ static int q_env_int(const char *name, int dflt) {
     return (v && *v) ? atoi(v) : dflt;
 }
 
-constexpr int kQMinRing = 2, kQMaxRing = 6;
+constexpr int kQMinRing = 2, kQMaxRing = 6, kQMaxSplit = 8;
 static int q_slot_bytes(int type_mix) { return type_mix == 12 ? kQ4KTileBytes : type_mix == 8 ? kQ80TileBytes : kQ6KTileBytes; }
 // Shared memory of a launch without its weight ring.
 static size_t qgemv_fixed_smem(int K, int type_mix, int bc) {
@@ -850,38 +943,83 @@ static int qgemv_ring_slots(const juno_ctx *ctx, int K, int type_mix, int bc, in
     return std::min(fit, kQMaxRing);
 }
 
+// CTAs of a cluster that share K: the fewest with which the operand of all sequences fits beside the ring, because a cluster starts
+// later and exchanges its sums.  Llama-3-8B steps of 3 / 6 / 8 sequences: 2.48 / 3.12 / 3.78 ms with the fewest, 2.64 / 3.27 / 3.78 with
+// at least two, 2.86 / 3.56 / 4.15 with at least four; without a split (several launches of as many sequences as fit, each reading all
+// weights) 6 sequences took 4.27 ms.
+static int qgemv_splits(const juno_ctx *ctx, int K, int type_mix, int bc) {
+    for (int s = 1; s <= kQMaxSplit && s <= K / 256; s *= 2) {
+        const size_t fixed = qgemv_fixed_smem((K / 256 + s - 1) / s * 256, type_mix, bc) + (s > 1 ? (size_t)qexchange_floats(bc) * 4 : 0);
+        if (fixed + (size_t)kQWarps * kQMinRing * q_slot_bytes(type_mix) <= ctx->smem_optin) return s;
+    }
+    return 1;
+}
+
 int qgemv_batch_chunk(const juno_ctx *ctx, int K, int type_mix, int batch) {
     int bc = std::min(batch, 8);
     while (bc > 1 && qgemv_ring_slots(ctx, K, type_mix, bc) < kQMinRing) bc--;
     return bc;
 }
 
-template <int TYPE, int NT, int OCC, bool TAGGED>
+template <int TYPE, int NT, int OCC, bool TAGGED, bool SPLIT>
 static int qlaunch_inst(juno_ctx *ctx, const QParams &p, int grid, size_t smem, cudaStream_t st) {
     static std::mutex mu;
     static bool configured[64] = {false};
+    static int clusters[64][kQMaxSplit + 1] = {{0}};  // clusters of that many CTAs that the device holds at a time
+    const auto kernel = qgemv_kernel<TYPE, NT, OCC, TAGGED, SPLIT>;
+    cudaLaunchConfig_t cfg = {};
+    cfg.blockDim = dim3(kQThreads);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)p.splits;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
     {
         std::lock_guard<std::mutex> g(mu);
         const int dev = ctx->device & 63;
         if (!configured[dev]) {
-            JUNO_CUDA_TRY(cudaFuncSetAttribute(qgemv_kernel<TYPE, NT, OCC, TAGGED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ctx->smem_optin));
+            JUNO_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ctx->smem_optin));
             configured[dev] = true;
         }
+        if (SPLIT) {  // as many clusters as fit at a time: one more would run alone after all the others
+            int &n = clusters[dev][p.splits];
+            if (n == 0) {
+                cfg.numAttrs = 1;
+                cfg.gridDim = dim3((unsigned)p.splits);
+                cfg.dynamicSmemBytes = ctx->smem_optin;
+                JUNO_CUDA_TRY(cudaOccupancyMaxActiveClusters(&n, kernel, &cfg));
+                JUNO_REQUIRE(n > 0, "qgemv: no cluster of %d CTAs fits", p.splits);
+            }
+            cfg.gridDim = dim3((unsigned)(std::min(n, p.total_rt) * p.splits));
+            cfg.dynamicSmemBytes = smem;
+            cfg.numAttrs = pdl_enabled() ? 2 : 1;
+        }
     }
-    JUNO_CUDA_TRY(launch_pdl(qgemv_kernel<TYPE, NT, OCC, TAGGED>, dim3(grid), dim3(kQThreads), smem, st, p));
+    if (SPLIT)
+        JUNO_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, p));
+    else
+        JUNO_CUDA_TRY(launch_pdl(kernel, dim3(grid), dim3(kQThreads), smem, st, p));
     ctx->kernel_launches++;
     return JUNO_OK;
 }
+template <int TYPE, int NT>
+static int qlaunch_nt(juno_ctx *ctx, const QParams &p, int grid, size_t smem, cudaStream_t st) {
+    if (p.splits > 1) return qlaunch_inst<TYPE, NT, 1, false, true>(ctx, p, grid, smem, st);
+    return p.tagged_adds ? qlaunch_inst<TYPE, NT, 1, true, false>(ctx, p, grid, smem, st) : qlaunch_inst<TYPE, NT, 1, false, false>(ctx, p, grid, smem, st);
+}
 template <int TYPE>
 static int qlaunch_type(juno_ctx *ctx, const QParams &p, int occ, int grid, size_t smem, cudaStream_t st) {
-    const bool tg = p.tagged_adds != 0;
     switch ((p.bc + 1) / 2) {
     case 1:
-        if (occ == 2) return tg ? qlaunch_inst<TYPE, 1, 2, true>(ctx, p, grid, smem, st) : qlaunch_inst<TYPE, 1, 2, false>(ctx, p, grid, smem, st);
-        return tg ? qlaunch_inst<TYPE, 1, 1, true>(ctx, p, grid, smem, st) : qlaunch_inst<TYPE, 1, 1, false>(ctx, p, grid, smem, st);
-    case 2: return tg ? qlaunch_inst<TYPE, 2, 1, true>(ctx, p, grid, smem, st) : qlaunch_inst<TYPE, 2, 1, false>(ctx, p, grid, smem, st);
-    case 3: return tg ? qlaunch_inst<TYPE, 3, 1, true>(ctx, p, grid, smem, st) : qlaunch_inst<TYPE, 3, 1, false>(ctx, p, grid, smem, st);
-    case 4: return tg ? qlaunch_inst<TYPE, 4, 1, true>(ctx, p, grid, smem, st) : qlaunch_inst<TYPE, 4, 1, false>(ctx, p, grid, smem, st);
+        if (occ == 2) return p.tagged_adds ? qlaunch_inst<TYPE, 1, 2, true, false>(ctx, p, grid, smem, st) : qlaunch_inst<TYPE, 1, 2, false, false>(ctx, p, grid, smem, st);
+        return qlaunch_nt<TYPE, 1>(ctx, p, grid, smem, st);
+    case 2: return qlaunch_nt<TYPE, 2>(ctx, p, grid, smem, st);
+    case 3: return qlaunch_nt<TYPE, 3>(ctx, p, grid, smem, st);
+    case 4: return qlaunch_nt<TYPE, 4>(ctx, p, grid, smem, st);
     default: break;
     }
     set_error("qgemv: unsupported batch chunk %d", p.bc);
@@ -926,10 +1064,13 @@ int launch_qgemv(juno_ctx *ctx, const QGemvArgs &a, cudaStream_t st) {
     p.total_rt = total_rt;
     p.K = a.K;
     p.NB = a.K / 256;
-    const int bc_full = qgemv_batch_chunk(ctx, a.K, type_mix, a.batch);
+    // peer exchange (tensor parallelism) keeps the whole of K in a CTA
+    const int bc_want = std::min(a.batch, 8);
+    p.splits = a.n_peers > 0 || a.tagged_adds ? 1 : qgemv_splits(ctx, a.K, type_mix, bc_want);
+    const int bc_full = p.splits > 1 ? bc_want : qgemv_batch_chunk(ctx, a.K, type_mix, a.batch);
     // two CTAs per SM (64 registers per thread, half the ring each) when the launch is a single n-tile and still gets a ring
     int occ = q_env_int("JUNO_QGEMV_OCC", 2);
-    if (occ != 2 || bc_full > 2 || qgemv_ring_slots(ctx, a.K, type_mix, bc_full, 2) < kQMinRing) occ = 1;
+    if (occ != 2 || bc_full > 2 || p.splits > 1 || qgemv_ring_slots(ctx, a.K, type_mix, bc_full, 2) < kQMinRing) occ = 1;
     // one CTA per slot of the GPU, each with its share of the row tiles (never more CTAs than row tiles)
     const int grid = std::max(1, std::min(ctx->sm_count * occ, total_rt));
     p.ld_out = a.ld_out;
@@ -964,8 +1105,9 @@ int launch_qgemv(juno_ctx *ctx, const QGemvArgs &a, cudaStream_t st) {
         // Two slots per warp, although more would fit: with 16-32 warps per SM the copies in flight already cover the
         // bandwidth-delay product, and every further slot only lengthens the queue in front of the loads of x (the
         // decode step measured 2.5-5 % slower with four to eight slots).
-        p.ring = std::max(kQMinRing, std::min(qgemv_ring_slots(ctx, a.K, type_mix, p.bc, occ), q_env_int("JUNO_QGEMV_RING", 2)));
-        const size_t smem = qgemv_fixed_smem(a.K, type_mix, p.bc) + (size_t)kQWarps * p.ring * p.slot_bytes;
+        p.ring = p.splits > 1 ? kQMinRing : std::max(kQMinRing, std::min(qgemv_ring_slots(ctx, a.K, type_mix, p.bc, occ), q_env_int("JUNO_QGEMV_RING", 2)));
+        const int k_cta = (p.NB + p.splits - 1) / p.splits * 256;
+        const size_t smem = qgemv_fixed_smem(k_cta, type_mix, p.bc) + (p.splits > 1 ? (size_t)qexchange_floats(p.bc) * 4 : 0) + (size_t)kQWarps * p.ring * p.slot_bytes;
         int rc;
         if (type_mix == 0)
             rc = qlaunch_type<0>(ctx, p, occ, grid, smem, st);

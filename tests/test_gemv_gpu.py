@@ -221,3 +221,20 @@ def test_closed_matrix_and_dimension_errors(mv):
     assert mv._L.juno_qmat_free(A.handle) == _lib.ERR_CLOSED
     with pytest.raises(ValueError):
         mv.upload_quantized(raw[:-1], synth.Q4_K, 16, 256)
+
+
+@pytest.mark.parametrize("t,rows,cols,batch", [
+    (synth.Q6_K, 100, 14336, 3), (synth.Q4_K, 4100, 14336, 8),  # K over two and over eight CTAs; fewer row tiles than clusters
+    (synth.Q6_K, 1000, 13 * 256, 8), (synth.Q8_0, 333, 33 * 256, 7),  # parts of unequal length
+    (synth.Q8_0, 21000, 8192, 8),  # more than one chunk of row tiles per cluster
+])
+def test_gemv_split_of_k_matches_oracle(mv, oracle, t, rows, cols, batch):
+    """Inputs that do not fit one CTA's shared memory: K is shared by a cluster, the result stays exact up to FP32 summation order."""
+    rng = np.random.default_rng(13)
+    raw = synth.random_blocks(rng, t, rows, cols)
+    x = rng.standard_normal((batch, cols)).astype(np.float32)
+    A = mv.upload_quantized(raw, t, rows, cols)
+    y = mv.sgemv(A, x)
+    assert rel_err(y, oracle.matvec(t, raw, x, rows, cols)) < 1e-5
+    assert np.array_equal(mv.sgemv(A, x), y)
+    A.close()

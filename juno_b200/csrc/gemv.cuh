@@ -37,7 +37,6 @@ struct StageArgs {
 enum GemvEpilogue {
     EPI_STORE = 0,       // out[b][row] = y
     EPI_SILU_PAIR = 1,   // tile rows 0-7 are gate rows, 8-15 the matching up rows: out[b][8*tile+row] = silu(gate)*up
-    EPI_RESID_NORM = 2,  // x_out = resid + y
 };
 
 struct GemvSeg {
@@ -57,10 +56,6 @@ struct GemvArgs {
     int ld_out = 0;   // stride between batch rows of every seg.out
     int epi = EPI_STORE;
     const uint8_t *ximg = nullptr;  // FP16 staged activation (launch_stage_f16) for this K and batch
-    // EPI_RESID_NORM
-    const float *resid = nullptr;
-    float *x_out = nullptr;
-    int ldx = 0;
     // batched path (launch_gemm): ximg is an FP16 image (launch_stage_f16) and xscale its per-row factors
     const float *xscale = nullptr;
     // optional: the same activation in the chunk-major layout of the tcgen05 kernel, and the device word that kernel
@@ -70,8 +65,7 @@ struct GemvArgs {
 };
 // Batched path: one pass over the weights for up to kGemmMaxBatch sequences (FP16 operands on mma.sync, gemm.cu).
 // The activation is staged as ONE FP16 column per sequence, pre-scaled per row by a power of two (xscale holds the
-// factors to multiply the products with).  Epilogues: EPI_STORE, EPI_SILU_PAIR, and EPI_RESID_NORM meaning only
-// x_out = resid + y.
+// factors to multiply the products with).
 constexpr int kGemmMaxBatch = 64;
 int gemm_min_batch();               // smallest batch routed to the batched path (JUNO_GEMM_MIN_BATCH, default 9)
 int gemm_padded_batch(int batch);   // image columns: batch rounded up to a multiple of 8

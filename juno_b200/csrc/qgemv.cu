@@ -24,6 +24,7 @@
 #include <cstdlib>
 #include <cstring>
 
+#include "bulk.cuh"
 #include "gemv.cuh"
 #include "layout.cuh"
 #include "qgemv.cuh"
@@ -132,22 +133,6 @@ __device__ __forceinline__ uint32_t pick4(const uint4 &v, int t) { return (t & 2
 __device__ __forceinline__ float silu_f(float x) { return __fdiv_rn(x, __fadd_rn(1.f, expf(-x))); }
 
 // ───────────────────────────── one weight tile against the operand ────────────────────────
-__device__ __forceinline__ uint4 lds128(uint32_t a) {
-    uint4 v;
-    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
-    return v;
-}
-__device__ __forceinline__ uint32_t lds32(uint32_t a) {
-    uint32_t v;
-    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
-    return v;
-}
-__device__ __forceinline__ uint32_t lds16(uint32_t a) {
-    uint32_t v;
-    asm volatile("{\n.reg .u16 h;\nld.shared.u16 h, [%1];\ncvt.u32.u16 %0, h;\n}\n" : "=r"(v) : "r"(a));
-    return v;
-}
-
 // Per-lane constants of the operand fetch and of the limb recombination.  Lane (g, t) FEEDS the limb column g of the
 // MMA (limb g%4 of sequence g/4 of the n-tile) and HOLDS the accumulator columns 2t, 2t+1 (limbs 0,1 or 2,- of
 // sequence t/2).
@@ -510,63 +495,6 @@ __device__ __forceinline__ const uint8_t *qtile_addr(const QParams &p, int R, in
     const int s = qseg_of(p, R);
     type = (TYPE == 0) ? p.seg_type[s] : TYPE;
     return p.w[s] + ((size_t)(R - p.rt_begin[s]) * p.NB + sb) * (size_t)tile_bytes(type);
-}
-
-// ── mbarrier / bulk-copy primitives ──────────────────────────────────────────────────────
-__device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(uint32_t bar, unsigned count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, unsigned bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-// One attempt.  ns == 0: a plain test.  Otherwise the hardware may park the warp for up to about `ns` nanoseconds when
-// the phase is not complete yet (fewer issue slots than polling, but it wakes late when the hint is long).
-__device__ __forceinline__ bool mbar_test(uint32_t bar, unsigned parity, unsigned ns) {
-    unsigned ok;
-    if (ns == 0)
-        asm volatile(
-            "{\n.reg .pred p;\n"
-            "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-            "selp.u32 %0, 1, 0, p;\n}\n"
-            : "=r"(ok)
-            : "r"(bar), "r"(parity)
-            : "memory");
-    else
-        asm volatile(
-            "{\n.reg .pred p;\n"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n"
-            "selp.u32 %0, 1, 0, p;\n}\n"
-            : "=r"(ok)
-            : "r"(bar), "r"(parity), "r"(ns)
-            : "memory");
-    return ok != 0;
-}
-// Weight tiles are read once per step: they are requested with the evict-first policy, so that the gigabytes streamed
-// through the L2 do not push out what every kernel start needs again (activations, norm weights, instructions).
-__device__ __forceinline__ uint64_t l2_evict_first_policy() {
-    uint64_t pol;
-    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
-    return pol;
-}
-__device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, unsigned bytes, uint32_t bar, uint64_t pol) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;" ::"r"(dst),
-                 "l"(src), "r"(bytes), "r"(bar), "l"(pol)
-                 : "memory");
-}
-// A wait on a weight tile gives up after this many SM cycles (about a fifth of a second); after the first give-up
-// of a warp its later waits are short, so that the kernel still drains the copies it has in flight and returns.
-constexpr long long kQWaitLimitClk = 400000000ll, kQWaitLimitAfterFail = 2000000ll;
-__device__ __forceinline__ void mbar_wait_bounded(uint32_t bar, unsigned parity, unsigned ns, unsigned *err, bool &failed) {
-    if (mbar_test(bar, parity, 0)) return;
-    const long long t0 = clock64(), limit = failed ? kQWaitLimitAfterFail : kQWaitLimitClk;
-    while (!mbar_test(bar, parity, ns)) {
-        if (clock64() - t0 > limit) {
-            if (!failed && (threadIdx.x & 31) == 0) *reinterpret_cast<volatile unsigned *>(err) = 1u | ((threadIdx.x >> 5) << 8) | (blockIdx.x << 16);
-            failed = true;
-            return;
-        }
-    }
 }
 
 constexpr int kQBufs = 2;  // buffers of partial sums (one CTA barrier per chunk)

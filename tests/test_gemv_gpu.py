@@ -238,3 +238,18 @@ def test_gemv_split_of_k_matches_oracle(mv, oracle, t, rows, cols, batch):
     assert rel_err(y, oracle.matvec(t, raw, x, rows, cols)) < 1e-5
     assert np.array_equal(mv.sgemv(A, x), y)
     A.close()
+
+
+@pytest.mark.parametrize("rows,cols,batch", [(100, 512, 9), (1000, 14336, 17), (4096, 4096, 33), (2100, 23 * 256, 47), (130, 1024, 64), (40000, 2048, 24)])
+@pytest.mark.parametrize("t", TYPES)
+def test_batched_product_shapes(mv, oracle, t, rows, cols, batch):
+    """The one-pass product at the edges of its split: units with idle warps, K over one to eight CTAs in unequal parts, every number
+    of n-tiles, more units than the GPU holds at a time."""
+    rng = np.random.default_rng(21)
+    raw = synth.random_blocks(rng, t, rows, cols)
+    x = rng.standard_normal((batch, cols)).astype(np.float32)
+    A = mv.upload_quantized(raw, t, rows, cols)
+    y = mv.sgemv(A, x)
+    pick = list(range(batch)) if rows < 10000 else [0, batch // 2, batch - 1]
+    assert rel_err(y[pick], oracle.matvec(t, raw, x[pick], rows, cols)) < TOL
+    A.close()

@@ -938,7 +938,7 @@ static int prompt_reserve(juno_model *m, int n) {
         auto elems = [&](int k) { return (size_t)L.w[k]->row_tiles * 16 * (size_t)L.w[k]->cols; };
         w16 = std::max({w16, elems(JUNO_T_ATTN_Q) + elems(JUNO_T_ATTN_K) + elems(JUNO_T_ATTN_V), elems(JUNO_T_ATTN_OUT), elems(JUNO_T_FFN_GATE), elems(JUNO_T_FFN_DOWN)});
     }
-    const size_t sizes[] = {R * H * 4, R * H * 4, R * m->qkv_ld * 4, R * H * 4, R * H * 4, R * I * 4, R * 4, R * std::max(H, I) * 2, w16 * 2,
+    const size_t sizes[] = {R * H * 4, R * H * 4, R * m->qkv_ld * 4, R * H * 4, R * H * 4, R * I * 4, R * 4, R * std::max(H, I) * 2, w16 * 2, w16 * 2,
                             R * (m->hd / 2) * sizeof(float2), 4 * R * 4};
     size_t total = 0;
     for (size_t s : sizes) total += (s + 1023) & ~(size_t)1023;
@@ -969,7 +969,8 @@ static int prompt_reserve(juno_model *m, int n) {
     P.hdn = (float *)take();
     P.scale = (float *)take();
     P.img = take();
-    P.w16 = take();
+    P.w16[0] = take();
+    P.w16[1] = take();
     P.cs = (float2 *)take();
     P.step = (int32_t *)take();
     P.rows = rows;
@@ -977,6 +978,7 @@ static int prompt_reserve(juno_model *m, int n) {
 }
 
 // Layers of one pass of n consecutive positions of one sequence.  On return the residual stream is x[cur] + proj.
+// The next product's weights are turned into FP16 rows while this product runs: two buffers take turns.
 static int enqueue_layers_prompt(juno_model *m, int n, int pos0, int &cur, cudaStream_t st) {
     juno_ctx *c = m->ctx;
     const juno_model_cfg &f = m->cfg;
@@ -996,20 +998,34 @@ static int enqueue_layers_prompt(juno_model *m, int n, int pos0, int &cur, cudaS
         a.scale = P.scale;
         return launch_stage_rows(c, a, st);
     };
-    auto product = [&](juno_qmat *const *mats, int count, int epi, float *out, int ldo) -> int {
+    // product k of the pass: q|k|v, W_o, gate|up, W_down of layer k / 4
+    auto matrices = [&](int k, juno_qmat *const **first) {
+        static const int kinds[4] = {JUNO_T_ATTN_Q, JUNO_T_ATTN_OUT, JUNO_T_FFN_GATE, JUNO_T_FFN_DOWN};
+        *first = &m->layers[(size_t)(k / 4)].w[kinds[k % 4]];
+        return k % 4 == 0 ? 3 : 1;
+    };
+    static_assert(JUNO_T_ATTN_K == JUNO_T_ATTN_Q + 1 && JUNO_T_ATTN_V == JUNO_T_ATTN_Q + 2, "q, k and v lie side by side");
+    auto rows_of = [&](int k) -> int {
+        juno_qmat *const *mats;
+        const int count = matrices(k, &mats);
         DequantSeg seg[3];
-        GemmArgs a;
-        a.K = (int)mats[0]->cols;
         for (int i = 0; i < count; i++) {
             seg[i].w = mats[i]->dev;
             seg[i].type = mats[i]->type;
             seg[i].row_tiles = (int)mats[i]->row_tiles;
-            a.N += (int)mats[i]->rows;
         }
-        JUNO_TRY(launch_dequant_rows(c, seg, count, a.K, P.w16, st));
+        return launch_dequant_rows(c, seg, count, (int)mats[0]->cols, P.w16[k & 1], st);
+    };
+    int k = 0;
+    auto product = [&](int epi, float *out, int ldo) -> int {
+        juno_qmat *const *mats;
+        const int count = matrices(k, &mats);
+        GemmArgs a;
+        a.K = (int)mats[0]->cols;
+        for (int i = 0; i < count; i++) a.N += (int)mats[i]->rows;
         a.a = P.img;
         a.lda = a.K;
-        a.w = P.w16;
+        a.w = P.w16[k & 1];
         a.ldw = a.K;
         a.M = n;
         a.out = out;
@@ -1017,15 +1033,16 @@ static int enqueue_layers_prompt(juno_model *m, int n, int pos0, int &cur, cudaS
         a.epi = epi;
         a.half = true;
         a.row_scale = P.scale;
-        return launch_gemm_rows(c, DT_BF16, a, c->gemv_scratch.qerr, st);
+        JUNO_TRY(launch_gemm_rows(c, DT_BF16, a, c->gemv_scratch.qerr, st));
+        return ++k < 4 * f.n_layers ? rows_of(k) : JUNO_OK;
     };
+    JUNO_TRY(rows_of(0));
     cur = 0;
     for (int l = 0; l < f.n_layers; l++) {
         JunoLayer &L = m->layers[l];
         JUNO_TRY(stage(P.x[cur], l ? P.proj : nullptr, L.attn_norm, l ? P.x[cur ^ 1] : nullptr, H));
         if (l) cur ^= 1;
-        juno_qmat *qkv_m[3] = {L.w[JUNO_T_ATTN_Q], L.w[JUNO_T_ATTN_K], L.w[JUNO_T_ATTN_V]};
-        JUNO_TRY(product(qkv_m, 3, GE_F32_ROW, P.qkv, m->qkv_ld));
+        JUNO_TRY(product(GE_F32_ROW, P.qkv, m->qkv_ld));
         if (L.bqkv) {
             const int width = Hl + 2 * KVl;
             qkv_bias_kernel<<<dim3((width + 255) / 256, n), 256, 0, st>>>(P.qkv, L.bqkv, n, width, m->qkv_ld);
@@ -1069,12 +1086,12 @@ static int enqueue_layers_prompt(juno_model *m, int n, int pos0, int &cur, cudaS
             }
         }
         JUNO_TRY(stage(P.att, nullptr, nullptr, nullptr, Hl));
-        JUNO_TRY(product(&L.w[JUNO_T_ATTN_OUT], 1, GE_F32_ROW, P.proj, H));
+        JUNO_TRY(product(GE_F32_ROW, P.proj, H));
         JUNO_TRY(stage(P.x[cur], P.proj, L.ffn_norm, P.x[cur ^ 1], H));
         cur ^= 1;
-        JUNO_TRY(product(&L.w[JUNO_T_FFN_GATE], 1, GE_SILU_ROW, P.hdn, I));
+        JUNO_TRY(product(GE_SILU_ROW, P.hdn, I));
         JUNO_TRY(stage(P.hdn, nullptr, nullptr, nullptr, I));
-        JUNO_TRY(product(&L.w[JUNO_T_FFN_DOWN], 1, GE_F32_ROW, P.proj, H));
+        JUNO_TRY(product(GE_F32_ROW, P.proj, H));
     }
     return JUNO_OK;
 }

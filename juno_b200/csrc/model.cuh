@@ -29,13 +29,13 @@ struct JunoGraph {
     int seen = 0;
 };
 
-// Workspace of a prompt pass of the quantised layers (prompt.cuh): rows of one pass, and one matrix in FP16.  Made by the first
+// Workspace of a prompt pass of the quantised layers (prompt.cuh): rows of one pass, and the matrices of two products in FP16.  Made by the first
 // prompt that needs it, grown by longer ones, kept until the model is freed.
 struct JunoPrompt {
     int rows = 0;
     uint8_t *dev = nullptr;  // one allocation, carved up below
     float *x[2], *qkv, *att, *proj, *hdn, *scale;
-    void *img, *w16;
+    void *img, *w16[2];
     float2 *cs;
     int32_t *step;           // tokens | positions | lengths | slots, `rows` each
     int32_t *h_step = nullptr;  // pinned mirror

@@ -123,36 +123,37 @@ struct DequantParams {
     int nseg, nb, K;
     __half *out;
 };
-// Bound by the writes of 2 bytes a weight: Q4_K takes about 5 instructions a weight, less than half of what an SM issues while it
-// writes them.  One warp per 16 x 256 tile; neighbouring warps take neighbouring tiles of a row tile, so a CTA writes whole 4 KB pieces of rows.
-__global__ void __launch_bounds__(256) dequant_rows_kernel(const DequantParams p) {
+// Runs beside the product before it, whose CTAs leave room for it on every SM: it writes the buffer that the product before that one
+// read, and waits for its predecessor at its end only, so that what follows it finds both complete.  Alone it is bound by the writes of 2 bytes a
+// weight.  One warp per 16 x 256 tile; neighbouring warps take neighbouring tiles of a row tile, so a CTA writes whole 4 KB pieces of rows.  Behind the product in turn:
+// TinyLlama Q8_0, 333 positions 3.55 ms; beside it 3.26 ms (Llama-3-8B, 2048 positions, where the tensor cores' power is the limit: 39.6 and 39.4 ms).
+constexpr int kDequantCtas = 2;  // per SM: with 64 registers a thread both fit beside a CTA of the product; one that did not would start after it
+template <int TYPE>
+__device__ __forceinline__ void dequant_one(const uint8_t *src, __half *row_r, __half *row_q, int lane) {
+    TileRegs<TYPE> R;
+    load_tile<TYPE>(R, src, lane);
+    dequant_tile(R, row_r, row_q, lane);
+}
+__global__ void __launch_bounds__(256, 4) dequant_rows_kernel(const DequantParams p) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int tile = blockIdx.x * 8 + warp;
-    int s = 0;
-    while (s < p.nseg && tile >= p.tiles[s]) s++;
-    pdl_launch_dependents();
-    if (s >= p.nseg) return;
-    const int t = tile - (s ? p.tiles[s - 1] : 0), rt = t / p.nb, sb = t - rt * p.nb;
-    const size_t row0 = (size_t)((s ? p.tiles[s - 1] / p.nb : 0) + rt) * 16 + (lane >> 2);
-    __half *row_r = p.out + row0 * p.K + sb * 256, *row_q = row_r + (size_t)8 * p.K;
-    const int type = p.seg[s].type;
-    const uint8_t *src = p.seg[s].w + (size_t)t * tile_bytes(type);
-    if (type == 12) {
-        TileRegs<12> R;
-        load_tile<12>(R, src, lane);
-        pdl_wait();  // the product before this one may still read the rows that are written here
-        dequant_tile(R, row_r, row_q, lane);
-    } else if (type == 14) {
-        TileRegs<14> R;
-        load_tile<14>(R, src, lane);
-        pdl_wait();
-        dequant_tile(R, row_r, row_q, lane);
-    } else {
-        TileRegs<8> R;
-        load_tile<8>(R, src, lane);
-        pdl_wait();
-        dequant_tile(R, row_r, row_q, lane);
+    const int total = p.tiles[p.nseg - 1];
+    for (int tile = blockIdx.x * 8 + warp; tile < total; tile += gridDim.x * 8) {
+        int s = 0;
+        while (tile >= p.tiles[s]) s++;
+        const int t = tile - (s ? p.tiles[s - 1] : 0), rt = t / p.nb, sb = t - rt * p.nb;
+        const size_t row0 = (size_t)((s ? p.tiles[s - 1] / p.nb : 0) + rt) * 16 + (lane >> 2);
+        __half *row_r = p.out + row0 * p.K + sb * 256, *row_q = row_r + (size_t)8 * p.K;
+        const int type = p.seg[s].type;
+        const uint8_t *src = p.seg[s].w + (size_t)t * tile_bytes(type);
+        if (type == 12)
+            dequant_one<12>(src, row_r, row_q, lane);
+        else if (type == 14)
+            dequant_one<14>(src, row_r, row_q, lane);
+        else
+            dequant_one<8>(src, row_r, row_q, lane);
     }
+    pdl_launch_dependents();
+    pdl_wait();
 }
 
 int launch_dequant_rows(juno_ctx *c, const DequantSeg *seg, int nseg, int K, void *out, cudaStream_t st) {
@@ -173,7 +174,7 @@ int launch_dequant_rows(juno_ctx *c, const DequantSeg *seg, int nseg, int K, voi
         bytes += (double)seg[s].row_tiles * p.nb * (tile_bytes(seg[s].type) + 8192);
     }
     ProfScope prof(c, st, PROF_OTHER, bytes);
-    JUNO_CUDA_TRY(launch_pdl(dequant_rows_kernel, dim3((unsigned)((tiles + 7) / 8)), dim3(256), 0, st, p));
+    JUNO_CUDA_TRY(launch_pdl(dequant_rows_kernel, dim3((unsigned)std::min((tiles + 7) / 8, kDequantCtas * c->sm_count)), dim3(256), 0, st, p));
     c->kernel_launches++;
     return JUNO_OK;
 }

@@ -55,6 +55,7 @@ __device__ __forceinline__ void put_head(const float *x, int dim, int dp, const 
 constexpr int kPrepWarps = 8;
 template <typename T>
 __global__ void __launch_bounds__(kPrepWarps * 32) grouped_prep_kernel(const __grid_constant__ GroupedParams p) {
+    row_start(gridDim.x);
     const GroupedAttnArgs &a = p.a;
     const int r = blockIdx.x, unit = blockIdx.y * kPrepWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (unit >= a.heads + 2 * a.kv_heads) return;
@@ -493,9 +494,9 @@ int launch_grouped_prep(juno_ctx *c, int dt, const GroupedAttnArgs &a, cudaStrea
     const dim3 grid((unsigned)a.rows.n, (unsigned)((units + kPrepWarps - 1) / kPrepWarps));
     ProfScope prof(c, st, PROF_ROWOPS, (double)a.rows.n * (a.heads * a.dp + a.kv_heads * (a.dp + a.vp)) * (4 + dt_bytes(dt)));
     if (dt == DT_F32)
-        grouped_prep_kernel<float><<<grid, kPrepWarps * 32, 0, st>>>(p);
+        JUNO_CUDA_TRY(launch_rows(a.rows.n, grouped_prep_kernel<float>, grid, dim3(kPrepWarps * 32), 0, st, p));
     else
-        grouped_prep_kernel<bf16><<<grid, kPrepWarps * 32, 0, st>>>(p);
+        JUNO_CUDA_TRY(launch_rows(a.rows.n, grouped_prep_kernel<bf16>, grid, dim3(kPrepWarps * 32), 0, st, p));
     JUNO_CUDA_TRY(cudaGetLastError());
     c->kernel_launches++;
     return JUNO_OK;

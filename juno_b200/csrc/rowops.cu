@@ -39,6 +39,7 @@ __global__ void __launch_bounds__(kRowThreads) embed_norm_kernel(const T *embed,
 
 template <typename T>
 __global__ void __launch_bounds__(kRowThreads) resid_norm_kernel(const ResidNormArgs a) {
+    row_start(a.n);
     extern __shared__ __align__(16) float row[];
     __shared__ float red[33];
     const int r = blockIdx.x;
@@ -82,6 +83,7 @@ __global__ void __launch_bounds__(kRowThreads) resid_norm_kernel(const ResidNorm
 template <typename T>
 __global__ void __launch_bounds__(kRowThreads) gather_norm_kernel(const float *x, int ldx, int width, const int32_t *row_idx, float g,
                                                                   float eps, T *out, int ldo) {
+    row_start(gridDim.x);
     __shared__ float red[33];
     const int i0 = blockIdx.x, r = row_idx ? row_idx[i0] : i0;
     const float *xr = x + (size_t)r * ldx;
@@ -98,11 +100,12 @@ __global__ void __launch_bounds__(kRowThreads) gather_norm_kernel(const float *x
     }
 }
 
-// Four channels per thread, kConvRows consecutive rows per block: a thread meets its own earlier inputs again in L1.
+// Four channels per thread.  A portion of one sequence: kConvRows consecutive rows per block, a thread meets its own earlier inputs again in
+// L1.  Rows of different sequences share nothing: one per block (eight of them one after the other took 16 us).
 constexpr int kConvRows = 8;
 struct ConvParams {
     const float *x;
-    int ldx, n, taps, one_seq;
+    int ldx, n, taps, one_seq, rows;  // rows: of a block of conv_kernel
     const float *row_scale;
     const void *w;
     float *state;  // this layer's rows of slot 0
@@ -114,10 +117,11 @@ struct ConvParams {
 };
 template <typename T>
 __global__ void __launch_bounds__(128) conv_kernel(const ConvParams p) {
+    row_start(p.n);
     const int col = (blockIdx.x * 128 + threadIdx.x) * 4;
     if (col >= p.ldx) return;
     const T *w = static_cast<const T *>(p.w);
-    const int r0 = blockIdx.y * kConvRows, r1 = min(p.n, r0 + kConvRows);
+    const int r0 = blockIdx.y * p.rows, r1 = min(p.n, r0 + p.rows);
     for (int r = r0; r < r1; r++) {
         const int pos = p.positions[r];
         float *ring = p.state ? p.state + (size_t)p.slots[r] * p.slot_stride + col : nullptr;
@@ -151,6 +155,7 @@ __global__ void __launch_bounds__(128) conv_kernel(const ConvParams p) {
 constexpr int kConvSeqRows = 16;
 template <typename T, int TAPS>
 __global__ void __launch_bounds__(128) conv_seq_kernel(const ConvParams p) {
+    row_start(p.n);
     const int col = (blockIdx.x * 128 + threadIdx.x) * 4;
     if (col >= p.ldx) return;
     const T *w = static_cast<const T *>(p.w);
@@ -192,6 +197,7 @@ __global__ void __launch_bounds__(128) conv_seq_kernel(const ConvParams p) {
 // After a portion: its last inputs into the state (a launch of its own, because the portion's first rows still read the
 // entries that its last rows replace).
 __global__ void __launch_bounds__(128) conv_state_kernel(const ConvParams p) {
+    row_start(p.n);
     const int col = (blockIdx.x * 128 + threadIdx.x) * 4;
     if (col >= p.ldx) return;
     const int r = p.n - 1 - (int)blockIdx.y;
@@ -209,6 +215,7 @@ struct LatentNormParams {
 };
 template <typename T>
 __global__ void __launch_bounds__(kRowThreads) latent_norm_kernel(const LatentNormParams p) {
+    row_start(gridDim.x);
     __shared__ float red[33];
     const int r = blockIdx.x, which = blockIdx.y;  // 0 = queries, 1 = key/value latent
     const LatentNormArgs &a = p.a;
@@ -251,10 +258,10 @@ int launch_resid_norm(juno_ctx *c, int dt, const ResidNormArgs &a, cudaStream_t 
     ProfScope prof(c, st, PROF_ROWOPS, (double)a.n * a.width * ((a.z ? 8 + dt_bytes(dt) : 4) + (a.h ? dt_bytes(dt) : 0)));
     if (dt == DT_F32) {
         JUNO_TRY(row_smem(resid_norm_kernel<float>, smem));
-        resid_norm_kernel<float><<<a.n, kRowThreads, smem, st>>>(a);
+        JUNO_CUDA_TRY(launch_rows(a.n, resid_norm_kernel<float>, dim3((unsigned)a.n), dim3(kRowThreads), smem, st, a));
     } else {
         JUNO_TRY(row_smem(resid_norm_kernel<bf16>, smem));
-        resid_norm_kernel<bf16><<<a.n, kRowThreads, smem, st>>>(a);
+        JUNO_CUDA_TRY(launch_rows(a.n, resid_norm_kernel<bf16>, dim3((unsigned)a.n), dim3(kRowThreads), smem, st, a));
     }
     JUNO_CUDA_TRY(cudaGetLastError());
     c->kernel_launches++;
@@ -266,9 +273,9 @@ int launch_gather_norm(juno_ctx *c, int dt, const float *x, int ldx, int width, 
     JUNO_REQUIRE(n > 0 && rows_ok(ldx, width) && ldo >= ldx, "row norm: bad arguments");
     ProfScope prof(c, st, PROF_ROWOPS, (double)n * width * (4 + dt_bytes(dt)));
     if (dt == DT_F32)
-        gather_norm_kernel<float><<<n, kRowThreads, 0, st>>>(x, ldx, width, row_idx, g, eps, static_cast<float *>(out), ldo);
+        JUNO_CUDA_TRY(launch_rows(n, gather_norm_kernel<float>, dim3((unsigned)n), dim3(kRowThreads), 0, st, x, ldx, width, row_idx, g, eps, static_cast<float *>(out), ldo));
     else
-        gather_norm_kernel<bf16><<<n, kRowThreads, 0, st>>>(x, ldx, width, row_idx, g, eps, static_cast<bf16 *>(out), ldo);
+        JUNO_CUDA_TRY(launch_rows(n, gather_norm_kernel<bf16>, dim3((unsigned)n), dim3(kRowThreads), 0, st, x, ldx, width, row_idx, g, eps, static_cast<bf16 *>(out), ldo));
     JUNO_CUDA_TRY(cudaGetLastError());
     c->kernel_launches++;
     return JUNO_OK;
@@ -294,23 +301,24 @@ int launch_conv(juno_ctx *c, int dt, const ConvArgs &a, const RowSet &rows, cuda
     p.out = a.out;
     p.ldo = a.ldo;
     const unsigned gx = (unsigned)((a.ldx + 511) / 512);
-    const dim3 grid(gx, (unsigned)((rows.n + kConvRows - 1) / kConvRows));
+    p.rows = rows.one_seq ? kConvRows : 1;
+    const dim3 grid(gx, (unsigned)((rows.n + p.rows - 1) / p.rows));
     ProfScope prof(c, st, PROF_ROWOPS, (double)rows.n * a.width * (4 + dt_bytes(dt)));
     const dim3 sgrid(gx, (unsigned)((rows.n + kConvSeqRows - 1) / kConvSeqRows));
     if (dt == DT_F32)
-        conv_kernel<float><<<grid, 128, 0, st>>>(p);
+        JUNO_CUDA_TRY(launch_rows(rows.n, conv_kernel<float>, grid, dim3(128), 0, st, p));
     else if (rows.one_seq && a.taps == 2)
-        conv_seq_kernel<bf16, 2><<<sgrid, 128, 0, st>>>(p);
+        JUNO_CUDA_TRY(launch_rows(rows.n, conv_seq_kernel<bf16, 2>, sgrid, dim3(128), 0, st, p));
     else if (rows.one_seq && a.taps == 3)
-        conv_seq_kernel<bf16, 3><<<sgrid, 128, 0, st>>>(p);
+        JUNO_CUDA_TRY(launch_rows(rows.n, conv_seq_kernel<bf16, 3>, sgrid, dim3(128), 0, st, p));
     else if (rows.one_seq && a.taps == 4)
-        conv_seq_kernel<bf16, 4><<<sgrid, 128, 0, st>>>(p);
+        JUNO_CUDA_TRY(launch_rows(rows.n, conv_seq_kernel<bf16, 4>, sgrid, dim3(128), 0, st, p));
     else
-        conv_kernel<bf16><<<grid, 128, 0, st>>>(p);
+        JUNO_CUDA_TRY(launch_rows(rows.n, conv_kernel<bf16>, grid, dim3(128), 0, st, p));
     JUNO_CUDA_TRY(cudaGetLastError());
     c->kernel_launches++;
     if (rows.one_seq && p.state) {
-        conv_state_kernel<<<dim3(gx, (unsigned)std::min(rows.n, pool->state_ring)), 128, 0, st>>>(p);
+        JUNO_CUDA_TRY(launch_rows(rows.n, conv_state_kernel, dim3(gx, (unsigned)std::min(rows.n, pool->state_ring)), dim3(128), 0, st, p));
         JUNO_CUDA_TRY(cudaGetLastError());
         c->kernel_launches++;
     }
@@ -330,9 +338,9 @@ int launch_latent_norm(juno_ctx *c, int dt, const LatentNormArgs &a, const RowSe
     JUNO_REQUIRE(a.kv_rank <= p.row_width, "latent norm: rows of %d do not fit pages of %d", a.kv_rank, p.row_width);
     ProfScope prof(c, st, PROF_ROWOPS, (double)rows.n * (a.q_rank + a.kv_rank) * (4 + dt_bytes(dt)));
     if (dt == DT_F32)
-        latent_norm_kernel<float><<<dim3(rows.n, 2), kRowThreads, 0, st>>>(p);
+        JUNO_CUDA_TRY(launch_rows(rows.n, latent_norm_kernel<float>, dim3((unsigned)rows.n, 2), dim3(kRowThreads), 0, st, p));
     else
-        latent_norm_kernel<bf16><<<dim3(rows.n, 2), kRowThreads, 0, st>>>(p);
+        JUNO_CUDA_TRY(launch_rows(rows.n, latent_norm_kernel<bf16>, dim3((unsigned)rows.n, 2), dim3(kRowThreads), 0, st, p));
     JUNO_CUDA_TRY(cudaGetLastError());
     c->kernel_launches++;
     return JUNO_OK;

@@ -14,6 +14,21 @@ inline int dt_bytes(int dt) { return dt == DT_F32 ? 4 : 2; }
 inline int pad16(int n) { return (n + 15) / 16 * 16; }
 inline int pad64(int n) { return (n + 63) / 64 * 64; }
 
+// Row kernels of a decode batch or a short portion start while their predecessor ends and let the product after them fetch its weights
+// meanwhile: Vosotar medium, 24 requests 0.87 -> 0.77 ms per step.  With the many blocks of a prompt the early starters get in the way (1000
+// positions, small: 2.54 -> 2.61 ms), so those are ordinary launches.
+constexpr int kEarlyRows = 128;
+__device__ __forceinline__ void row_start(int rows) {
+    pdl_wait();
+    if (rows <= kEarlyRows) pdl_launch_dependents();
+}
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_rows(int rows, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args &&...args) {
+    if (rows <= kEarlyRows) return launch_pdl(kernel, grid, block, smem, st, std::forward<Args>(args)...);
+    kernel<<<grid, block, smem, st>>>(std::forward<Args>(args)...);
+    return cudaGetLastError();
+}
+
 // The rows of one pass.  one_seq: consecutive positions of one sequence (a portion of a prompt); otherwise row i is the next
 // position of its own sequence.  Device pointers; positions[i] + 1 == lens[i].
 struct RowSet {

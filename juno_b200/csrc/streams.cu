@@ -27,6 +27,7 @@ __global__ void __launch_bounds__(kStThreads) stream_embed_kernel(const T *embed
 // S: the number of streams when it is a common one (the old streams stay in registers), else 0
 template <typename T, int S>
 __global__ void __launch_bounds__(kStThreads) stream_step_kernel(const StreamStepArgs a) {
+    row_start(a.n);
     extern __shared__ __align__(16) float row[];  // the sublayer's input
     __shared__ float red[33], mix[kMaxStreams * kMaxStreams], out[kMaxStreams], in[kMaxStreams];
     const int r = blockIdx.x, ns = S ? S : a.streams, tid = threadIdx.x;
@@ -79,6 +80,7 @@ __global__ void __launch_bounds__(kStThreads) stream_step_kernel(const StreamSte
 template <typename T>
 __global__ void __launch_bounds__(kStThreads) stream_gather_kernel(const float *x, int streams, int ldx, int width, const int32_t *row_idx, const float *w, float eps,
                                                                    T *out, float *sum, int ldo) {
+    row_start(gridDim.x);
     extern __shared__ __align__(16) float row[];
     __shared__ float red[33];
     const int i0 = blockIdx.x, r = row_idx ? row_idx[i0] : i0;
@@ -127,7 +129,7 @@ template <typename T, int S>
 static int step_inst(const StreamStepArgs &a, cudaStream_t st) {
     const size_t smem = (size_t)a.ldx * 4;
     JUNO_TRY(row_smem(stream_step_kernel<T, S>, smem));
-    stream_step_kernel<T, S><<<a.n, kStThreads, smem, st>>>(a);
+    JUNO_CUDA_TRY(launch_rows(a.n, stream_step_kernel<T, S>, dim3((unsigned)a.n), dim3(kStThreads), smem, st, a));
     return JUNO_OK;
 }
 template <typename T>
@@ -159,10 +161,10 @@ int launch_stream_gather(juno_ctx *c, int dt, const float *x, int streams, int l
     ProfScope prof(c, st, PROF_ROWOPS, (double)n * width * (4 * streams + dt_bytes(dt)));
     if (dt == DT_F32 || sum) {
         JUNO_TRY(row_smem(stream_gather_kernel<float>, smem));
-        stream_gather_kernel<float><<<n, kStThreads, smem, st>>>(x, streams, ldx, width, row_idx, w, eps, static_cast<float *>(out), sum, ldo);
+        JUNO_CUDA_TRY(launch_rows(n, stream_gather_kernel<float>, dim3((unsigned)n), dim3(kStThreads), smem, st, x, streams, ldx, width, row_idx, w, eps, static_cast<float *>(out), sum, ldo));
     } else {
         JUNO_TRY(row_smem(stream_gather_kernel<bf16>, smem));
-        stream_gather_kernel<bf16><<<n, kStThreads, smem, st>>>(x, streams, ldx, width, row_idx, w, eps, static_cast<bf16 *>(out), sum, ldo);
+        JUNO_CUDA_TRY(launch_rows(n, stream_gather_kernel<bf16>, dim3((unsigned)n), dim3(kStThreads), smem, st, x, streams, ldx, width, row_idx, w, eps, static_cast<bf16 *>(out), sum, ldo));
     }
     JUNO_CUDA_TRY(cudaGetLastError());
     c->kernel_launches++;

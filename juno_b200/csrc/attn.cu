@@ -586,17 +586,6 @@ __global__ void __launch_bounds__(kCombineParts * HD) attn_combine_kernel(const 
     p.out[(size_t)(seq * p.n_heads + h) * HD + d] = outv;
 }
 
-// cos/sin of pos * theta^(-2i/hd) in binary64, cast to float, as LlamaTransformerHandler.rope (:1662-1666).
-__global__ void rope_table_kernel(const int32_t *positions, int n, int hd, float theta, float2 *table) {
-    int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    int half = hd / 2;
-    if (idx >= n * half) return;
-    int seq = idx / half, i = idx - seq * half;
-    double freq = 1.0 / pow((double)theta, (2.0 * i) / hd);
-    double angle = positions[seq] * freq;
-    table[idx] = make_float2((float)cos(angle), (float)sin(angle));
-}
-
 struct RopeParams {
     void *k, *v;
     const int32_t *table;
@@ -842,15 +831,6 @@ int launch_attn(juno_ctx *ctx, const AttnArgs &a, cudaStream_t st) {
         launch_pdl(attn_combine_kernel<64>, cgrid, dim3(kCombineParts * 64), 0, st, p);
     JUNO_CUDA_TRY(cudaGetLastError());
     ctx->kernel_launches += 2;
-    return JUNO_OK;
-}
-
-int launch_rope_table(juno_ctx *ctx, const int32_t *positions, int n, int hd, float theta, float2 *table,
-                      cudaStream_t st) {
-    int total = n * hd / 2;
-    rope_table_kernel<<<(total + 127) / 128, 128, 0, st>>>(positions, n, hd, theta, table);
-    JUNO_CUDA_TRY(cudaGetLastError());
-    ctx->kernel_launches++;
     return JUNO_OK;
 }
 

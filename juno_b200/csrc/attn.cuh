@@ -60,7 +60,7 @@ struct AttnArgs {
     float *part_ml;      // [n][n_heads][n_splits][2]
     double algo_bytes = 0;  // K+V bytes the call has to read (for the profiler)
     // optional: fused RoPE + KV append.  q [n][ldq] is unrotated, knew/vnew [n][ldkv] hold this step's k and v,
-    // rope_cs the table of launch_rope_table; the newest position (seq_lens-1) is rotated, rounded and appended.
+    // rope_cs the step's table of rope_cos_sin; the newest position (seq_lens-1) is rotated, rounded and appended.
     const float2 *rope_cs = nullptr;
     const float *knew = nullptr, *vnew = nullptr;
     int ldkv = 0;
@@ -69,10 +69,16 @@ size_t attn_scratch_floats(int n, int n_heads, int hd, int n_splits);
 int attn_pick_splits(const juno_ctx *ctx, int n, int n_kv_heads, int max_len);
 int launch_attn(juno_ctx *ctx, const AttnArgs &a, cudaStream_t st);
 
+#if defined(__CUDACC__)
+// cos/sin of pos * theta^(-2i/hd) in binary64, cast to float, as LlamaTransformerHandler.rope (:1662-1666).
+__device__ __forceinline__ float2 rope_cos_sin(int pos, int i, int hd, float theta) {
+    const double freq = 1.0 / pow((double)theta, (2.0 * i) / hd);
+    const double angle = pos * freq;
+    return make_float2((float)cos(angle), (float)sin(angle));
+}
+#endif
 // RoPE on q and k (adjacent pairs, LlamaTransformerHandler.rope :1657-1671) and append of k, v at
-// position pos[i] of each sequence.  cs_table: [n][hd/2] (cos, sin) from launch_rope_table.
-int launch_rope_table(juno_ctx *ctx, const int32_t *positions, int n, int hd, float theta, float2 *table,
-                      cudaStream_t st);
+// position pos[i] of each sequence.  cs_table: [n][hd/2] of rope_cos_sin.
 int launch_rope_append(juno_ctx *ctx, const juno_kvpool *pool, int layer, int n, int n_heads, float *q, int ldq,
                        const float *k, const float *v, int ldkv, const int32_t *slots, const int32_t *positions,
                        const float2 *cs_table, cudaStream_t st);

@@ -84,22 +84,35 @@ static int nccl_load() {
     } while (0)
 
 // ───────────────────────────── small kernels ──────────────────────────────────────────────
-// Embedding row of the dequantised token_embd (getInitialActivation :651-660): token id clamped to
-// [0, vocab-1], values bit-exact with dequantizeQ4K & co.
-__global__ void embed_kernel(int type, int tiled, const uint8_t *w, int64_t nb, int64_t row_bytes, int hidden, int vocab,
-                             const int32_t *tokens, float *x) {
-    const int seq = blockIdx.y, col = blockIdx.x * blockDim.x + threadIdx.x;
-    if (col >= hidden) return;
-    int tok = tokens[seq];
-    tok = max(0, min(tok, vocab - 1));
-    float v;
-    if (tiled) {
-        const uint8_t *tile = w + (((int64_t)tok >> 4) * nb + (col >> 8)) * (int64_t)tile_bytes(type);
-        v = tile_elem_value(type, tile, tok & 15, col & 255);
-    } else {
-        v = raw_elem_value(type, w + (int64_t)tok * row_bytes, col);
+// Start of a pass.  Embedding row of the dequantised token_embd (getInitialActivation :651-660): token id clamped to
+// [0, vocab-1], values bit-exact with dequantizeQ4K & co.; and, in a block of its own per row, the rotation of the row's position.
+struct EmbedParams {
+    int type, tiled, hidden, vocab, hd;
+    const uint8_t *w;
+    int64_t nb, row_bytes;
+    const int32_t *tokens, *positions;
+    float theta;
+    float *x;
+    float2 *cs;
+};
+__global__ void __launch_bounds__(256) embed_kernel(const EmbedParams p) {
+    pdl_launch_dependents();  // the first product may fetch its weights
+    const int seq = blockIdx.y, half = p.hd / 2;
+    if (blockIdx.x == 0) {
+        if ((int)threadIdx.x < half) p.cs[(size_t)seq * half + threadIdx.x] = rope_cos_sin(p.positions[seq], threadIdx.x, p.hd, p.theta);
+        return;
     }
-    x[(size_t)seq * hidden + col] = v;
+    const int col = (blockIdx.x - 1) * 256 + threadIdx.x;
+    if (col >= p.hidden) return;
+    const int tok = max(0, min(p.tokens[seq], p.vocab - 1));
+    float v;
+    if (p.tiled) {
+        const uint8_t *tile = p.w + (((int64_t)tok >> 4) * p.nb + (col >> 8)) * (int64_t)tile_bytes(p.type);
+        v = tile_elem_value(p.type, tile, tok & 15, col & 255);
+    } else {
+        v = raw_elem_value(p.type, p.w + (int64_t)tok * p.row_bytes, col);
+    }
+    p.x[(size_t)seq * p.hidden + col] = v;
 }
 
 // Element (seq, v) of the logits: plain [n][V], or, after an all-gather of vocab slices, [world][n][V/world].
@@ -1360,10 +1373,36 @@ static int enqueue_pick(juno_model *m, int n, bool greedy_advance, bool want_log
     return JUNO_OK;
 }
 
-static int enqueue_step(juno_model *m, int n, int n_splits, bool greedy_advance, bool want_logits, cudaStream_t st) {
+// Embeddings of n tokens -> x, rotations of their positions -> cs.
+static int launch_embed(juno_model *m, int n, const int32_t *d_tok, const int32_t *d_pos, float *x, float2 *cs, cudaStream_t st) {
+    const juno_qmat *e = m->tok_embd;
+    EmbedParams p;
+    p.type = e->type;
+    p.tiled = e->tiled;
+    p.hidden = m->cfg.hidden;
+    p.vocab = m->cfg.vocab;
+    p.hd = m->hd;
+    p.w = e->dev;
+    p.nb = e->nb;
+    p.row_bytes = e->tiled ? 0 : e->cols / raw_block_elems(e->type) * raw_block_bytes(e->type);
+    p.tokens = d_tok;
+    p.positions = d_pos;
+    p.theta = m->cfg.rope_theta;
+    p.x = x;
+    p.cs = cs;
+    embed_kernel<<<dim3((unsigned)((p.hidden + 255) / 256 + 1), (unsigned)n), 256, 0, st>>>(p);
+    JUNO_CUDA_TRY(cudaGetLastError());
+    m->ctx->kernel_launches++;
+    return JUNO_OK;
+}
+
+// pick: the greedy pick is wanted (a step that returns logits only goes without; ranks that share the vocabulary gather there, so they
+// always take it).
+static int enqueue_step(juno_model *m, int n, int n_splits, bool greedy_advance, bool want_logits, bool pick, cudaStream_t st) {
     juno_ctx *c = m->ctx;
     const juno_model_cfg &f = m->cfg;
-    const int H = f.hidden, hd = m->hd, B = m->step_cap;
+    const int B = m->step_cap;
+    pick = pick || greedy_advance || m->vocab_sharded;
     const int32_t *d_tok = m->d_step, *d_pos = m->d_step + B, *d_slot = m->d_step + 2 * B, *d_len = m->d_step + 3 * B;
     if (m->stack) {
         RowSet rows;
@@ -1373,23 +1412,14 @@ static int enqueue_step(juno_model *m, int n, int n_splits, bool greedy_advance,
         rows.slots = d_slot;
         rows.lens = d_len;
         JUNO_TRY(stack_enqueue_step(c, m->stack, m->pool, rows, n_splits, f.max_ctx, m->logits_loc, st));
-        return enqueue_pick(m, n, greedy_advance, want_logits, st);
+        return pick ? enqueue_pick(m, n, greedy_advance, want_logits, st) : JUNO_OK;
     }
     if (m->tp_push) {
         epoch_kernel<<<1, 1, 0, st>>>(m->tp_epoch);
         JUNO_CUDA_TRY(cudaGetLastError());
         c->kernel_launches++;
     }
-    // embedding lookup -> x[0]
-    {
-        juno_qmat *e = m->tok_embd;
-        dim3 grid((H + 255) / 256, n);
-        int64_t rb = e->tiled ? 0 : e->cols / raw_block_elems(e->type) * raw_block_bytes(e->type);
-        embed_kernel<<<grid, 256, 0, st>>>(e->type, e->tiled, e->dev, e->nb, rb, H, f.vocab, d_tok, m->x[0]);
-        JUNO_CUDA_TRY(cudaGetLastError());
-        c->kernel_launches++;
-    }
-    JUNO_TRY(launch_rope_table(c, d_pos, n, hd, f.rope_theta, m->rope_cs, st));
+    JUNO_TRY(launch_embed(m, n, d_tok, d_pos, m->x[0], m->rope_cs, st));
     int cur = 0;          // x[cur] holds the residual stream
     // 9..64 sequences: one pass over the weights per product on the FP16 tensor-core kernels; otherwise the exact
     // integer-MMA GEMV (batches above 64 in chunks of up to eight sequences per pass)
@@ -1399,20 +1429,20 @@ static int enqueue_step(juno_model *m, int n, int n_splits, bool greedy_advance,
     else
         JUNO_TRY(enqueue_layers_q(m, n, d_slot, d_len, n_splits, cur, st));
     m->last_x = cur;
-    return enqueue_pick(m, n, greedy_advance, want_logits, st);
+    return pick ? enqueue_pick(m, n, greedy_advance, want_logits, st) : JUNO_OK;
 }
 
 // Runs one step: the first call for a (n, splits, mode) key runs eagerly (it also sizes every scratch
 // buffer); the second captures the same launches into a CUDA graph, later ones replay it.
-static int run_step(juno_model *m, int n, int n_splits, bool greedy_advance, bool want_logits) {
+static int run_step(juno_model *m, int n, int n_splits, bool greedy_advance, bool want_logits, bool pick) {
     juno_ctx *c = m->ctx;
     cudaStream_t st = c->stream;
     if (m->comm_failed) {
         set_error("the tensor-parallel communicator was aborted after a failed step: free the model and build a new group");
         return JUNO_ERR_NCCL;
     }
-    if (!m->use_graphs || c->profiling) return enqueue_step(m, n, n_splits, greedy_advance, want_logits, st);
-    const uint64_t key = ((uint64_t)n << 32) | ((uint64_t)n_splits << 2) | (want_logits ? 2u : 0u) | (greedy_advance ? 1u : 0u);
+    if (!m->use_graphs || c->profiling) return enqueue_step(m, n, n_splits, greedy_advance, want_logits, pick, st);
+    const uint64_t key = ((uint64_t)n << 32) | ((uint64_t)n_splits << 3) | (pick ? 4u : 0u) | (want_logits ? 2u : 0u) | (greedy_advance ? 1u : 0u);
     JunoGraph &g = m->graphs[key];
     if (g.exec) {
         JUNO_CUDA_TRY(cudaGraphLaunch(g.exec, st));
@@ -1421,11 +1451,11 @@ static int run_step(juno_model *m, int n, int n_splits, bool greedy_advance, boo
     }
     if (!g.seen) {
         g.seen = 1;
-        return enqueue_step(m, n, n_splits, greedy_advance, want_logits, st);
+        return enqueue_step(m, n, n_splits, greedy_advance, want_logits, pick, st);
     }
     const int64_t before = c->kernel_launches.load();
     JUNO_CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-    int rc = enqueue_step(m, n, n_splits, greedy_advance, want_logits, st);
+    int rc = enqueue_step(m, n, n_splits, greedy_advance, want_logits, pick, st);
     cudaGraph_t graph = nullptr;
     cudaError_t e = cudaStreamEndCapture(st, &graph);
     const int launches = (int)(c->kernel_launches.load() - before);
@@ -1634,13 +1664,7 @@ static int prefill_run(juno_model *m, juno_seq *seq, const int32_t *token_ids, i
             m->step_kv_bytes = 0;
             for (int i = 0; i < n; i++) m->step_kv_bytes += (double)(pos0 + i + 1) * m->kv_loc * m->hd * 2 * m->pool->elem_bytes;
             const int n_splits = attn_pick_splits(c, n, m->kv_loc, bucket_len(pos0 + n));
-            juno_qmat *e = m->tok_embd;
-            dim3 grid((f.hidden + 255) / 256, n);
-            int64_t rb = e->tiled ? 0 : e->cols / raw_block_elems(e->type) * raw_block_bytes(e->type);
-            embed_kernel<<<grid, 256, 0, st>>>(e->type, e->tiled, e->dev, e->nb, rb, f.hidden, V, d_tok, many ? m->prompt.x[0] : m->x[0]);
-            JUNO_CUDA_TRY(cudaGetLastError());
-            c->kernel_launches++;
-            JUNO_TRY(launch_rope_table(c, d_pos, n, m->hd, f.rope_theta, many ? m->prompt.cs : m->rope_cs, st));
+            JUNO_TRY(launch_embed(m, n, d_tok, d_pos, many ? m->prompt.x[0] : m->x[0], many ? m->prompt.cs : m->rope_cs, st));
             int cur = 0;
             if (many)
                 JUNO_TRY(enqueue_layers_prompt(m, n, pos0, cur, st));
@@ -1723,7 +1747,7 @@ int juno_forward(juno_model *m, int32_t n, juno_seq *const *seqs, const int32_t 
     JUNO_TRY(step_sync(m));
     int n_splits = 1;
     JUNO_TRY(prepare_step(m, n, seqs, token_ids, positions, 0, &n_splits));
-    JUNO_TRY(run_step(m, n, n_splits, false, logits_host != nullptr));
+    JUNO_TRY(run_step(m, n, n_splits, false, logits_host != nullptr, argmax_out != nullptr));
     // With collectives in the step the guarded wait comes first: a device-to-host copy into pageable memory blocks
     // the caller until the stream reaches it, and would sit behind a collective that never completes.
     if (m->world > 1) JUNO_TRY(step_sync(m));
@@ -1794,7 +1818,7 @@ int juno_decode_greedy(juno_model *m, int32_t n, juno_seq *const *seqs, const in
         }
     }
     JUNO_CUDA_TRY(cudaMemsetAsync(m->d_step_counter, 0, 4, c->stream));
-    for (int s = 0; s < steps; s++) JUNO_TRY(run_step(m, n, n_splits, true, false));
+    for (int s = 0; s < steps; s++) JUNO_TRY(run_step(m, n, n_splits, true, false, true));
     if (m->world > 1) JUNO_TRY(step_sync(m));  // before the copy of the ids, see juno_forward
     c->forward_calls += steps;
     JUNO_CUDA_TRY(cudaMemcpyAsync(out_ids, m->d_out_ids, (size_t)steps * n * 4, cudaMemcpyDeviceToHost, c->stream));

@@ -41,7 +41,7 @@ int launch_stage_rows(juno_ctx *c, const StageRowsArgs &a, cudaStream_t st);
 int launch_gather_rows(juno_ctx *c, const float *x, const float *add, const int32_t *rows, int row0, int n, int K, float *out, cudaStream_t st);
 
 // Attention of rows r < n at positions pos0 + r of one sequence over FP16 pages that already hold every one of them:
-// qkv [n][ld] unrotated, query heads first; cs: launch_rope_table of the rows.
+// qkv [n][ld] unrotated, query heads first; cs: rope_cos_sin of the rows.
 struct PromptAttnArgs {
     const juno_kvpool *pool = nullptr;
     int layer = 0, n = 0, pos0 = 0, n_heads = 0;

@@ -39,8 +39,8 @@ int launch_gemm_rows_tc(juno_ctx *c, const GemmArgs &a, unsigned *err, cudaStrea
 constexpr int kFewRows = 128;                                                              // most rows of launch_gemm_few_tc
 int launch_gemm_few_tc(juno_ctx *c, const GemmArgs &a, unsigned *err, cudaStream_t st);  // the same for few rows, BF16
 // The same on pairs of SMs, and whether a product does better there.
-bool gemm_pair_takes(const juno_ctx *c, const GemmArgs &a);
-int launch_gemm_pair_tc(juno_ctx *c, const GemmArgs &a, unsigned *err, cudaStream_t st);
+int gemm_pair_splits(const juno_ctx *c, const GemmArgs &a);
+int launch_gemm_pair_tc(juno_ctx *c, const GemmArgs &a, int splits, unsigned *err, cudaStream_t st);
 int launch_gemm_rows(juno_ctx *c, int dt, const GemmArgs &a, unsigned *err, cudaStream_t st);
 
 }  // namespace juno

@@ -206,7 +206,7 @@ static int gemm_tc_epi(juno_ctx *c, const GemmTcParams &p, cudaStream_t st) {
 }
 
 int launch_gemm_rows_tc(juno_ctx *c, const GemmArgs &a, unsigned *err, cudaStream_t st) {
-    if (gemm_pair_takes(c, a)) return launch_gemm_pair_tc(c, a, err, st);
+    if (const int splits = gemm_pair_splits(c, a)) return launch_gemm_pair_tc(c, a, splits, err, st);
     GemmTcParams p;
     memset(&p, 0, sizeof(p));
     p.g = a;

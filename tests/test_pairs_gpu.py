@@ -1,5 +1,5 @@
-"""Products of many rows on pairs of SMs: the last rows and columns of a tile missing, every epilogue that such a product has, K tails - in
-prompts whose feed-forwards are wide enough to take them."""
+"""Products of many rows on pairs of SMs: the last rows and columns of a tile missing, every epilogue that such a product has, K tails, K
+shared by two and four pairs - in prompts whose feed-forwards are wide enough to take them."""
 import numpy as np
 import pytest
 
@@ -11,17 +11,27 @@ from test_prompt_gpu import TOL, tame
 
 pytestmark = pytest.mark.gpu
 VOSOTAR = synth.vosotar_config(1000, 200, [vosotarutil.L(4, 64, 64, 64, 64, 4200)], taps=2)
+WIDE = synth.vosotar_config(2100, 200, [vosotarutil.L(2, 64, 64, 64, 64, 4200)], taps=1)
 DESILORN = synth.desilorn_config(1000, 200, [desilornutil.W(4, 2, 64, 64, 300, 2100)], streams=2)
 
 
 @pytest.mark.parametrize("util,cfg", [(vosotarutil, VOSOTAR), (desilornutil, DESILORN)], ids=["vosotar", "desilorn"])
-@pytest.mark.parametrize("n", [513, 700, 768])
+@pytest.mark.parametrize("n", [130, 300, 513, 700, 768])
 def test_prompts_match_the_oracle(tmp_path, util, cfg, n):
     p = util.Pair(tmp_path, cfg, seed=41)
     toks = p.tokens(n, 5)
     h = p.open("default", max_ctx=1024)
     places = list(range(0, n, 37)) + [n - 1]
     util.check(h.prefill_logits("a", toks, 0, places), p.oracle(toks)[places], "default", f"{n} positions")
+    h.release_gpu_resources()
+
+
+def test_two_pairs_share_k(tmp_path):
+    p = vosotarutil.Pair(tmp_path, WIDE, seed=42)
+    toks = p.tokens(768, 6)
+    h = p.open("default", max_ctx=1024)
+    places = list(range(0, 768, 51)) + [767]
+    vosotarutil.check(h.prefill_logits("a", toks, 0, places), p.oracle(toks)[places], "default")
     h.release_gpu_resources()
 
 

@@ -149,7 +149,8 @@ class B200MatVec:
             xb = xv.reshape(1, -1) if one else xv
             if xb.ndim != 2 or xb.shape[1] != A.cols:
                 raise ValueError(f"x.length must equal cols ({A.cols}), got {xb.shape[-1]}")
-            y = self.ctx.host_rows(xb.shape[0], A.rows)
+            n = xb.shape[0]
+            y = np.empty((n, A.rows), dtype=np.float32) if 4 * n * A.rows < PINNED_FROM else self.ctx.host_rows(n, A.rows)
             check(self._L.juno_gemv(self.ctx.handle, A.handle, _ptr(xb), xb.shape[0], _ptr(y)), "juno_gemv")
             return y[0] if one else y
         a = np.ascontiguousarray(A, dtype=np.float32).reshape(-1)

@@ -960,11 +960,11 @@ static int prompt_reserve(juno_model *m, int n) {
     if (P.h_step) cudaFreeHost(P.h_step);
     P = JunoPrompt();
     JUNO_TRY(dev_alloc((void **)&P.dev, total));
-    if (cudaMallocHost((void **)&P.h_step, 4 * R * 4) != cudaSuccess) {
+    if (cudaMallocHost((void **)&P.h_step, (4 * R + 1) * 4) != cudaSuccess) {
         cudaGetLastError();
         cudaFree(P.dev);
         P = JunoPrompt();
-        set_error("cudaMallocHost of %zu bytes failed", 4 * R * 4);
+        set_error("cudaMallocHost of %zu bytes failed", (4 * R + 1) * 4);
         return JUNO_ERR_OOM;
     }
     uint8_t *at = P.dev;
@@ -992,7 +992,7 @@ static int prompt_reserve(juno_model *m, int n) {
 
 // Layers of one pass of n consecutive positions of one sequence.  On return the residual stream is x[cur] + proj.
 // The next product's weights are turned into FP16 rows while this product runs: two buffers take turns.
-static int enqueue_layers_prompt(juno_model *m, int n, int pos0, int &cur, cudaStream_t st) {
+static int enqueue_layers_prompt(juno_model *m, int n, int pos0, bool guard, int &cur, cudaStream_t st) {
     juno_ctx *c = m->ctx;
     const juno_model_cfg &f = m->cfg;
     JunoPrompt &P = m->prompt;
@@ -1073,6 +1073,8 @@ static int enqueue_layers_prompt(juno_model *m, int n, int pos0, int &cur, cudaS
             at.ld = m->qkv_ld;
             at.cs = P.cs;
             at.slot = d_slot;
+            at.v_odd = P.h_step + 4 * R;
+            at.guard = guard;
             at.out = P.att;
             at.algo_bytes = (double)(pos0 + n) * KVl * 2 * m->pool->elem_bytes;
             JUNO_TRY(launch_prompt_append(c, at, st));
@@ -1614,8 +1616,9 @@ static int prepare_step(juno_model *m, int n, juno_seq *const *seqs, const int32
 
 // A portion of ONE sequence in passes of as many positions as the model's kernels take at once.  want[0..n_want): places
 // in the portion whose logits go to logits_host, in that order; argmax_out (optional): the greedy pick at the last of them.
+// guard: see PromptAttnArgs; a portion that turns out to need it is fed once more.
 static int prefill_run(juno_model *m, juno_seq *seq, const int32_t *token_ids, int n_tokens, int start_pos, int n_want, const int32_t *want,
-                       float *logits_host, int32_t *argmax_out) {
+                       float *logits_host, int32_t *argmax_out, bool guard = false) {
     JUNO_TRY(model_check(m));
     juno_ctx *c = m->ctx;
     std::lock_guard<std::recursive_mutex> lk(c->mu);
@@ -1630,6 +1633,8 @@ static int prefill_run(juno_model *m, juno_seq *seq, const int32_t *token_ids, i
     const int B = m->step_cap, chunk_max = m->stack ? B : std::min(B, kGemmMaxBatch), V = f.vocab;
     JUNO_REQUIRE(n_want == 0 || !m->vocab_sharded, "prefill logits are not implemented for a sharded vocabulary");
     cudaStream_t st = c->stream;
+    bool odd = false;
+    const int32_t *marked = nullptr;
     for (int done = 0; done < n_tokens;) {
         // without memory for the workspace of the many-row path the portion goes through the smaller passes
         const bool many = prompt_takes(m, n_tokens - done) && prompt_reserve(m, n_tokens - done) == JUNO_OK;
@@ -1638,6 +1643,11 @@ static int prefill_run(juno_model *m, juno_seq *seq, const int32_t *token_ids, i
         JUNO_TRY(seq_reserve(seq, pos0, pos0 + n, st));
         int32_t *h = many ? m->prompt.h_step : m->h_step, *d = many ? m->prompt.step : m->d_step;
         const int ld = many ? m->prompt.rows : B;
+        if (many) {  // the word may still hold what an earlier call left there
+            odd = odd || (done > 0 && h[4 * ld]);
+            h[4 * ld] = 0;
+            marked = h + 4 * ld;
+        }
         for (int i = 0; i < n; i++) {
             h[i] = token_ids[done + i];
             h[ld + i] = pos0 + i;
@@ -1667,7 +1677,7 @@ static int prefill_run(juno_model *m, juno_seq *seq, const int32_t *token_ids, i
             JUNO_TRY(launch_embed(m, n, d_tok, d_pos, many ? m->prompt.x[0] : m->x[0], many ? m->prompt.cs : m->rope_cs, st));
             int cur = 0;
             if (many)
-                JUNO_TRY(enqueue_layers_prompt(m, n, pos0, cur, st));
+                JUNO_TRY(enqueue_layers_prompt(m, n, pos0, guard, cur, st));
             else
                 JUNO_TRY(enqueue_layers_batched(m, n, d_slot, d_len, n_splits, cur, st, d_pos, !rows.empty()));
             m->last_x = cur;
@@ -1722,7 +1732,8 @@ static int prefill_run(juno_model *m, juno_seq *seq, const int32_t *token_ids, i
     JUNO_TRY(step_sync(m));
     JUNO_TRY(step_check(m));
     seq->len = std::max(seq->len, start_pos + n_tokens);
-    return JUNO_OK;
+    odd = odd || (marked && *marked);
+    return odd && !guard ? prefill_run(m, seq, token_ids, n_tokens, start_pos, n_want, want, logits_host, argmax_out, true) : JUNO_OK;
 }
 
 }  // namespace juno

@@ -37,8 +37,8 @@ struct JunoPrompt {
     float *x[2], *qkv, *att, *proj, *hdn, *scale;
     void *img, *w16[2];
     float2 *cs;
-    int32_t *step;           // tokens | positions | lengths | slots, `rows` each
-    int32_t *h_step = nullptr;  // pinned mirror
+    int32_t *step;           // tokens | positions | slots | lengths, `rows` each
+    int32_t *h_step = nullptr;  // pinned mirror, and behind it the word that PromptAttnArgs::v_odd points to
 };
 
 struct juno_model {

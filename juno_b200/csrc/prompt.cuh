@@ -51,6 +51,8 @@ struct PromptAttnArgs {
     const int32_t *slot = nullptr;  // device, one word
     float *out = nullptr;           // [n][n_heads * hd]
     double algo_bytes = 0;
+    int32_t *v_odd = nullptr;       // set to 1 by an append with values that are not finite in FP16
+    bool guard = false;             // such values may lie in the pages: rows are shielded from those of later positions
 };
 // Rotates k, rounds k and v to FP16 and writes them to the pages of their positions.
 int launch_prompt_append(juno_ctx *c, const PromptAttnArgs &a, cudaStream_t st);

@@ -94,3 +94,38 @@ def test_prompt_of_two_passes(ctx):
         for w, row in zip(inside, ref):
             assert rel_err(got[places.index(p + w)], row) < TOL, p + w
     h.release_gpu_resources()
+
+
+@pytest.mark.parametrize("arch,n,start,at", [(TINY, 80, 0, 40), (TINY, 70, 7, 63), (SMALL128, 200, 0, 130), (SMALL128, 65, 3, 1)])
+def test_values_beyond_fp16_stay_behind_their_position(ctx, arch, n, start, at):
+    """One position whose first-layer values overflow FP16 (infinite in its page, NaN from the next layer on): the positions before it
+    have the logits that they have without it, to the last bit."""
+    from juno_b200.handler import B200TransformerHandler
+    odd = arch.vocab - 1
+
+    def tensors():
+        for kind, layer, t, rows, cols, raw in tame(synth.random_model(arch, 53, MAPS["q8_0"], norm="ones")):
+            if kind == 0:  # the first column of the embeddings: of the odd token alone, which has no other
+                b = raw.reshape(rows, cols // 32, 34)
+                b[:, 0, 2] = 0
+                b[odd, :, 2:] = 0
+                b[odd, 0, 2] = 127
+            elif (kind, layer) == (7, 0):  # W_v reads it with a factor of 12,700
+                b = raw.reshape(rows, cols // 32, 34)
+                b[:, 0, :2] = np.full(1, 100, np.float16).view(np.uint8)
+                b[:, 0, 2:] = 0
+                b[:, 0, 2] = 127
+            yield kind, layer, t, rows, cols, raw
+
+    h = B200TransformerHandler(arch, ctx, max_batch=8, max_seqs=2, max_ctx=256)
+    h.load(tensors())
+    toks = np.random.default_rng(n).integers(0, odd, start + n)
+    got = {}
+    for name, tok in (("plain", toks[start + at]), ("odd", odd)):
+        toks[start + at] = tok
+        if start:
+            h.prefill(name, toks[:start], 0)
+        got[name] = h.prefill_logits(name, toks[start:], start, range(n))
+    assert np.isfinite(got["plain"]).all() and not np.isfinite(got["odd"][at]).any()
+    assert np.array_equal(got["odd"][:at], got["plain"][:at])
+    h.release_gpu_resources()

@@ -64,6 +64,8 @@ int juno_device_total_mem(int32_t device, int64_t *bytes);
 int juno_ctx_create(int32_t device, juno_ctx **out);
 int juno_ctx_destroy(juno_ctx *ctx); /* idempotent on a closed handle: returns JUNO_ERR_CLOSED */
 int juno_ctx_device(juno_ctx *ctx, int32_t *device);
+/* Waits for the context's stream.  JUNO_ERR_TIMEOUT, once, when a product of juno_gemv_device gave up a wait (its result is
+ * not valid); one on a stream of the caller's has to have finished before the call. */
 int juno_ctx_synchronize(juno_ctx *ctx);
 /* The cudaStream_t all work of this context is enqueued on (replaces the per-thread stream of
  * CudaMatVec.java:73-82); a host may record its own events on it. */
@@ -90,11 +92,12 @@ int juno_qmat_shape(juno_qmat *m, int64_t *rows, int64_t *cols, int32_t *ggml_ty
  * MatVec.sgemv(DeviceHalfMatrix, float[]) (MatVec.java:86-90, CudaMatVec.java:276-333)
  * on the quantised weights of LlamaTransformerHandler.matVec (:1200-1245):
  * inputs are not modified, JUNO_ERR_INVALID_ARG on a dimension mismatch,
- * JUNO_ERR_CLOSED on a freed matrix. */
+ * JUNO_ERR_CLOSED on a freed matrix, JUNO_ERR_TIMEOUT when a kernel gave up a wait (y is not valid). */
 int juno_gemv(juno_ctx *ctx, juno_qmat *m, const float *x_host, int32_t batch, float *y_host);
 
 /* Same product with x and y already in device memory, enqueued on `stream`
- * (a cudaStream_t, NULL = the context's stream) and not synchronised. */
+ * (a cudaStream_t, NULL = the context's stream) and not synchronised; a wait that its
+ * kernels gave up is reported by juno_ctx_synchronize. */
 int juno_gemv_device(juno_ctx *ctx, juno_qmat *m, const float *x_dev, int32_t batch, float *y_dev,
                      void *stream);
 

@@ -51,12 +51,15 @@ constexpr uint32_t kMagicSeq = 0x4A534551;    // "JSEQ"
 constexpr uint32_t kMagicPool = 0x4A4B5650;   // "JKVP"
 constexpr uint32_t kMagicDead = 0xDEADDEAD;
 
+// Whose kernels gave up a wait: calls that return when their work is done look at their own word then, and take the failure back, so
+// that it is reported once and by the call it belongs to; work that is only enqueued (juno_gemv_device) has another one.
+enum WaitWord { WAIT_BLOCKING = 0, WAIT_ENQUEUED = 1 };
 constexpr unsigned kErrStackWait = 8;  // code of a given-up wait in a layer stack's kernels (see GemvScratch::qerr)
 
 // Scratch of the host-level MatVec entry points and the word kernels report a given-up wait in.
 struct GemvScratch {
     unsigned *qerr = nullptr;       // device address of qerr_host
-    unsigned *qerr_host = nullptr;  // mapped host memory: code | warp << 8 | block << 16, 0 = no failure
+    unsigned *qerr_host = nullptr;  // mapped host memory, WaitWord words: code | warp << 8 | block << 16, 0 = no failure
     uint8_t *ximg = nullptr;        // FP16 staged activation (batched path)
     size_t ximg_bytes = 0;
     float *xscale = nullptr;        // per-row factors of an FP16 staged activation, 64 floats
@@ -101,6 +104,8 @@ int ctx_check(juno_ctx *c);
 // Grows a device buffer (never shrinks). Returns JUNO_OK / JUNO_ERR_OOM.
 int ensure_device(void **ptr, size_t *cur, size_t want);
 int ensure_pinned(juno_ctx *c, size_t want);
+// Once the work has drained: JUNO_ERR_TIMEOUT and the text, and the word cleared, when one of its kernels gave up a wait.
+int wait_status(juno_ctx *c, WaitWord which);
 
 // Brackets one launch (or a short group) with events when the context is profiling.
 struct ProfScope {

@@ -67,6 +67,19 @@ int ensure_pinned(juno_ctx *c, size_t want) {
     return JUNO_OK;
 }
 
+int wait_status(juno_ctx *c, WaitWord which) {
+    const unsigned code = __atomic_exchange_n(c->gemv_scratch.qerr_host + which, 0u, __ATOMIC_ACQ_REL);
+    if (!code) return JUNO_OK;
+    if ((code & 0xffu) == kErrStackWait)
+        set_error("a matrix product gave up waiting inside a kernel (stage %u of block %u)", (code >> 8) & 0xffu, code >> 16);
+    else if ((code & 0xffu) >= 3u)
+        set_error("tensor-parallel rank %u did not deliver its %s within a second (this rank gave up waiting)", (code >> 8) & 0xffu,
+                  (code & 0xffu) == 3u ? "partial products" : "greedy pick");
+    else
+        set_error("a GEMV warp gave up waiting for a weight tile (warp %u of block %u)", (code >> 8) & 0xffu, code >> 16);
+    return JUNO_ERR_TIMEOUT;
+}
+
 // Page-locked blocks for results that a host reads.  One pool for the process, because a result may outlive the context that wrote
 // it; blocks come in powers of two, at most kHostPoolBytes of them in all, and those that nobody holds are given back when a
 // context closes or another size needs the room.
@@ -237,7 +250,7 @@ int juno_ctx_synchronize(juno_ctx *c) {
     JUNO_TRY(ctx_check(c));
     DeviceGuard g(c->device);
     JUNO_CUDA_TRY(cudaStreamSynchronize(c->stream));
-    return JUNO_OK;
+    return wait_status(c, WAIT_ENQUEUED);
 }
 
 int juno_ctx_stream(juno_ctx *c, void **stream) {
@@ -424,7 +437,11 @@ int juno_gemv_device(juno_ctx *c, juno_qmat *m, const float *x_dev, int32_t batc
     std::lock_guard<std::recursive_mutex> lk(c->mu);
     DeviceGuard g(c->device);
     c->gemv_calls++;
-    return gemv_on_stream(c, m, x_dev, batch, y_dev, stream ? (cudaStream_t)stream : c->stream);
+    unsigned *const blocking = c->gemv_scratch.qerr;
+    c->gemv_scratch.qerr = blocking + WAIT_ENQUEUED;
+    const int rc = gemv_on_stream(c, m, x_dev, batch, y_dev, stream ? (cudaStream_t)stream : c->stream);
+    c->gemv_scratch.qerr = blocking;
+    return rc;
 }
 
 int juno_gemv(juno_ctx *c, juno_qmat *m, const float *x_host, int32_t batch, float *y_host) {
@@ -446,10 +463,12 @@ int juno_gemv(juno_ctx *c, juno_qmat *m, const float *x_host, int32_t batch, flo
     JUNO_TRY(gemv_on_stream(c, m, c->stage_x, batch, c->stage_y, c->stream));
     JUNO_CUDA_TRY(cudaMemcpyAsync(y_host, c->stage_y, yb, cudaMemcpyDeviceToHost, c->stream));
     JUNO_CUDA_TRY(cudaStreamSynchronize(c->stream));
+    JUNO_TRY(wait_status(c, WAIT_BLOCKING));
     if (c->gemv_scratch.xscale && batch >= gemm_min_batch()) {  // did a wait inside the tcgen05 kernel give up?
         unsigned code = 0;
         JUNO_CUDA_TRY(cudaMemcpy(&code, c->gemv_scratch.xscale + kGemmMaxBatch, 4, cudaMemcpyDeviceToHost));
         if (code) {
+            JUNO_CUDA_TRY(cudaMemset(c->gemv_scratch.xscale + kGemmMaxBatch, 0, 4));
             set_error("batched tensor-core product gave up waiting (code %u, block %u)", code & 0xffu, code >> 8);
             return JUNO_ERR_CUDA;
         }

@@ -1556,21 +1556,9 @@ static int step_check(juno_model *m) {
             return JUNO_ERR_CUDA;
         }
     }
-    juno_ctx *c = m->ctx;
-    const unsigned code = c->gemv_scratch.qerr_host ? *reinterpret_cast<volatile unsigned *>(c->gemv_scratch.qerr_host) : 0u;
-    if (code) {
-        *reinterpret_cast<volatile unsigned *>(c->gemv_scratch.qerr_host) = 0u;
-        if (m->tp_failed) cudaMemset(m->tp_failed, 0, 4);
-        if ((code & 0xffu) == kErrStackWait)
-            set_error("a matrix product gave up waiting inside a kernel (stage %u of block %u)", (code >> 8) & 0xffu, code >> 16);
-        else if ((code & 0xffu) >= 3u)
-            set_error("tensor-parallel rank %u did not deliver its %s within a second (this rank gave up waiting)", (code >> 8) & 0xffu,
-                      (code & 0xffu) == 3u ? "partial products" : "greedy pick");
-        else
-            set_error("a GEMV warp gave up waiting for a weight tile (warp %u of block %u)", (code >> 8) & 0xffu, code >> 16);
-        return JUNO_ERR_TIMEOUT;
-    }
-    return JUNO_OK;
+    const int rc = wait_status(m->ctx, WAIT_BLOCKING);
+    if (rc != JUNO_OK && m->tp_failed) cudaMemset(m->tp_failed, 0, 4);
+    return rc;
 }
 
 static int bucket_len(int len) {

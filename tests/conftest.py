@@ -63,6 +63,20 @@ def layout_host():
 
 
 @pytest.fixture(scope="session")
+def wait_words(ctx):
+    """The words of mapped host memory in which kernels of this context report a wait that they gave up."""
+    import ctypes as C
+    import subprocess
+    src, so = (os.path.join(ROOT, "tests", "native", f) for f in ("wait_words.cpp", "libwait_words.so"))
+    header = os.path.join(ROOT, "juno_b200", "csrc", "common.cuh")
+    if not os.path.exists(so) or os.path.getmtime(so) < max(os.path.getmtime(src), os.path.getmtime(header)):
+        subprocess.check_call(["g++", "-O2", "-std=c++17", "-I/usr/local/cuda/include", "-shared", "-fPIC", "-o", so, src])
+    L = C.CDLL(so)
+    L.wait_words.restype, L.wait_words.argtypes = C.POINTER(C.c_uint32), [C.c_void_p]
+    return L.wait_words(ctx.handle)
+
+
+@pytest.fixture(scope="session")
 def ctx():
     from juno_b200.matvec import GpuContext
     return GpuContext.shared(0)

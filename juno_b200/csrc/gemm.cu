@@ -22,6 +22,7 @@
 #include "bulk.cuh"
 #include "gemv.cuh"
 #include "layout.cuh"
+#include "ring.cuh"
 #include "tile_math.cuh"
 
 namespace juno {
@@ -246,17 +247,19 @@ __global__ void __launch_bounds__(kGemmThreads, 2) gemm_kernel(const __grid_cons
     pdl_wait();
     pdl_launch_dependents();
     bool failed = false;
+    int issued = 0;  // copies of this warp's slots, or of the stages (lane 0)
     float acc[NT][4];
 #pragma unroll
     for (int nt = 0; nt < NT; nt++) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
     if (warp == kGemmWarps) {
         if (lane == 0) {
-            for (int i = 0; i < 2 * (s1 - s0); i++) {
-                const int st = i % p.stages, use = i / p.stages;
-                if (use > 0) mbar_wait_bounded(freed + st * 8, (unsigned)(use - 1) & 1u, 0, p.err, failed);
+            for (; issued < 2 * (s1 - s0); issued++) {
+                const int st = issued % p.stages;
+                if (issued >= p.stages) mbar_wait_bounded(freed + st * 8, ring_parity(issued - p.stages, p.stages), 0, p.err, failed);
+                if (failed) break;
                 mbar_expect_tx(full + st * 8, stage_bytes);
                 asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(act + st * stage_bytes),
-                             "l"(p.ximg + (size_t)(2 * s0 + i) * stage_bytes), "r"(stage_bytes), "r"(full + st * 8)
+                             "l"(p.ximg + (size_t)(2 * s0 + issued) * stage_bytes), "r"(stage_bytes), "r"(full + st * 8)
                              : "memory");
             }
         }
@@ -264,6 +267,7 @@ __global__ void __launch_bounds__(kGemmThreads, 2) gemm_kernel(const __grid_cons
     } else if (warp < active) {
         const uint32_t xs = (uint32_t)NC * 32u;
         int slot = 0, st = 0;
+        issued = min(p.ring, s1 - s0);
         unsigned tpar = 0, spar = 0;
         for (int i = 0; i < s1 - s0; i++) {
             mbar_wait_bounded(tile_bar + slot * 8, tpar, 0, p.err, failed);
@@ -296,14 +300,26 @@ __global__ void __launch_bounds__(kGemmThreads, 2) gemm_kernel(const __grid_cons
                 }
             }
             __syncwarp();  // every lane has used the slot's bytes before they are overwritten
-            if (lane == 0 && s0 + i + p.ring < s1) fetch(i + p.ring);
+            if (lane == 0 && !failed && s0 + i + p.ring < s1) {
+                fetch(i + p.ring);
+                issued++;
+            }
             if (++slot == p.ring) {
                 slot = 0;
                 tpar ^= 1u;
             }
         }
     }
-    __syncthreads();  // the stages are done with: their memory takes the partial sums, [sequence][row of the unit]
+    // the stages are done with: their memory takes the partial sums, [sequence][row of the unit]
+    if (__syncthreads_or(failed)) {  // somebody gave up waiting: what is still on its way has to land first
+        if (failed) *reinterpret_cast<volatile unsigned *>(p.err) = 1u | (unsigned)warp << 8 | blockIdx.x << 16;
+        if (lane == 0 && (warp < active || warp == kGemmWarps)) {
+            const int slots = warp == kGemmWarps ? p.stages : p.ring;
+            const uint32_t bar = warp == kGemmWarps ? full : tile_bar;
+            for (int j = ring_open(issued, 0, slots); j < issued; j++) mbar_wait_bounded(bar + j % slots * 8, ring_parity(j, slots), 0, p.err, failed);
+        }
+        __syncthreads();
+    }
     if (warp < active) {
         const uint32_t at = act + (uint32_t)((2 * (lane & 3)) * kGemmOutLd + warp * 16 + (lane >> 2)) * 4;
 #pragma unroll

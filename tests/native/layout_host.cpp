@@ -113,3 +113,27 @@ extern "C" int qsplit_check(int total_rt, int NB, int grid, int *max_tiles_per_w
     if (max_tiles_per_warp) *max_tiles_per_warp = busiest;
     return 0;
 }
+
+// ── rings of copies (ring.cuh) ───────────────────────────────────────────────────────────
+#include "../../juno_b200/csrc/ring.cuh"
+
+// A user of a ring takes n copies in turn, arming copy i + slots after copy i, and gives up at copy `fail` (n: never).  0 when the copies to
+// wait for at the end are those that were armed and not waited for, one per slot, each in the phase its slot is in.
+extern "C" int ring_check(int n, int slots, int fail) {
+    int issued = n < slots ? n : slots, used = 0;
+    int armed[64] = {0};  // copies that each slot was armed for
+    for (int j = 0; j < issued; j++) armed[j % slots]++;
+    for (; used < n && used != fail; used++)
+        if (used + slots < n) {
+            issued++;
+            armed[(used + slots) % slots]++;
+        }
+    bool waited[64] = {false};
+    int open = 0;
+    for (int j = ring_open(issued, used, slots); j < issued; j++, open++) {
+        const int s = j % slots;
+        if (j < used || waited[s] || ring_parity(j, slots) != ((unsigned)(armed[s] - 1) & 1u)) return 1;
+        waited[s] = true;
+    }
+    return open != issued - used;
+}

@@ -108,3 +108,10 @@ def test_gemv_work_split_covers_every_tile_once(layout_host):
         per_cta = -(-rt // grid)  # row tiles of the busiest CTA
         chunks = -(-per_cta // 16)
         assert busiest.value <= -(-per_cta * nb // 16) + chunks, (rt, nb, grid, busiest.value)
+
+
+@pytest.mark.parametrize("slots", [2, 3, 4, 6])
+def test_rings_know_the_copies_that_are_in_flight(layout_host, slots):
+    for n in range(1, 30):
+        for fail in range(n + 1):
+            assert layout_host.ring_check(n, slots, fail) == 0, (n, fail)

@@ -320,6 +320,7 @@ static void free_qmat(juno_qmat *&q) {
     }
 }
 
+static void prompt_release(JunoPrompt &P);
 static void model_release(juno_model *m) {
     juno_ctx *c = m->ctx;
     DeviceGuard g(c->device);
@@ -362,8 +363,7 @@ static void model_release(juno_model *m) {
     for (void *b : bufs)
         if (b) cudaFree(b);
     if (m->h_step) cudaFreeHost(m->h_step);
-    if (m->prompt.dev) cudaFree(m->prompt.dev);
-    if (m->prompt.h_step) cudaFreeHost(m->prompt.h_step);
+    prompt_release(m->prompt);
     stack_free(m->stack);
     m->stack = nullptr;
     m->magic = kMagicDead;
@@ -927,7 +927,7 @@ static int enqueue_layers_batched(juno_model *m, int n, const int32_t *d_slot, c
 }
 
 // ───────────────────────────── prompt passes of many positions ────────────────────────────
-constexpr int kPromptRows = 2048;  // most positions per pass
+constexpr int kPromptMinRows = 128, kPromptRows = 2048;  // least and most positions per pass that the workspace is made for
 
 static int step_sync(juno_model *m);
 
@@ -940,38 +940,44 @@ static bool prompt_takes(const juno_model *m, int n) {
     return n > (chunk >= 8 ? chunk : 2 * chunk);
 }
 
-// Room for n rows; JUNO_ERR_OOM leaves the model without the workspace (the caller then uses the smaller passes).
-static int prompt_reserve(juno_model *m, int n) {
-    JunoPrompt &P = m->prompt;
-    const int rows = (std::min(n, kPromptRows) + 127) / 128 * 128;
-    if (rows <= P.rows) return JUNO_OK;
-    const size_t H = m->cfg.hidden, R = rows, I = m->inter_loc;
-    size_t w16 = 0;  // elements of the largest group of matrices that one product takes
-    for (const JunoLayer &L : m->layers) {
-        auto elems = [&](int k) { return (size_t)L.w[k]->row_tiles * 16 * (size_t)L.w[k]->cols; };
-        w16 = std::max({w16, elems(JUNO_T_ATTN_Q) + elems(JUNO_T_ATTN_K) + elems(JUNO_T_ATTN_V), elems(JUNO_T_ATTN_OUT), elems(JUNO_T_FFN_GATE), elems(JUNO_T_FFN_DOWN)});
-    }
-    const size_t sizes[] = {R * H * 4, R * H * 4, R * m->qkv_ld * 4, R * H * 4, R * H * 4, R * I * 4, R * 4, R * std::max(H, I) * 2, w16 * 2, w16 * 2,
-                            R * (m->hd / 2) * sizeof(float2), 4 * R * 4};
-    size_t total = 0;
-    for (size_t s : sizes) total += (s + 1023) & ~(size_t)1023;
-    JUNO_TRY(step_sync(m));
+static void prompt_release_rows(JunoPrompt &P) {
     if (P.dev) cudaFree(P.dev);
     if (P.h_step) cudaFreeHost(P.h_step);
+    P.dev = nullptr;
+    P.h_step = nullptr;
+    P.rows = 0;
+}
+
+static void prompt_release(JunoPrompt &P) {
+    prompt_release_rows(P);
+    if (P.weights) cudaFree(P.weights);
     P = JunoPrompt();
-    JUNO_TRY(dev_alloc((void **)&P.dev, total));
-    if (cudaMallocHost((void **)&P.h_step, (4 * R + 1) * 4) != cudaSuccess) {
+}
+
+// The row buffers of passes of up to `rows` positions, in place of those that are there, which stay if there is no memory for both.
+static int prompt_alloc_rows(juno_model *m, int rows) {
+    JunoPrompt &P = m->prompt;
+    const size_t H = m->cfg.hidden, R = rows, I = m->inter_loc;
+    const size_t sizes[] = {R * H * 4, R * H * 4, R * m->qkv_ld * 4, R * H * 4, R * H * 4, R * I * 4, R * 4, R * std::max(H, I) * 2, R * (m->hd / 2) * sizeof(float2), 4 * R * 4};
+    size_t total = 0;
+    for (size_t s : sizes) total += (s + 1023) & ~(size_t)1023;
+    uint8_t *dev = nullptr;
+    int32_t *h_step = nullptr;
+    JUNO_TRY(dev_alloc((void **)&dev, total));
+    if (cudaMallocHost((void **)&h_step, (4 * R + 1) * 4) != cudaSuccess) {
         cudaGetLastError();
-        cudaFree(P.dev);
-        P = JunoPrompt();
+        cudaFree(dev);
         set_error("cudaMallocHost of %zu bytes failed", (4 * R + 1) * 4);
         return JUNO_ERR_OOM;
     }
-    uint8_t *at = P.dev;
+    prompt_release_rows(P);
+    P.dev = dev;
+    P.h_step = h_step;
+    P.rows = rows;
     int k = 0;
     auto take = [&]() {
-        uint8_t *p = at;
-        at += (sizes[k++] + 1023) & ~(size_t)1023;
+        uint8_t *p = dev;
+        dev += (sizes[k++] + 1023) & ~(size_t)1023;
         return p;
     };
     P.x[0] = (float *)take();
@@ -982,11 +988,39 @@ static int prompt_reserve(juno_model *m, int n) {
     P.hdn = (float *)take();
     P.scale = (float *)take();
     P.img = take();
-    P.w16[0] = take();
-    P.w16[1] = take();
     P.cs = (float2 *)take();
     P.step = (int32_t *)take();
-    P.rows = rows;
+    return JUNO_OK;
+}
+
+// Room for passes of n positions.  Rows come in powers of two, so that prompts that grow longer ask seldom; when memory is short
+// there is room for fewer (m->prompt.rows), at least for those of before.  JUNO_ERR_OOM: for none.
+static int prompt_reserve(juno_model *m, int n) {
+    JunoPrompt &P = m->prompt;
+    int rows = kPromptMinRows;
+    while (rows < std::min(n, kPromptRows)) rows *= 2;
+    if (rows <= P.rows) return JUNO_OK;
+    JUNO_TRY(step_sync(m));
+    if (!P.weights) {
+        size_t w16 = 0;  // elements of the largest group of matrices that one product takes
+        for (const JunoLayer &L : m->layers) {
+            auto elems = [&](int k) { return (size_t)L.w[k]->row_tiles * 16 * (size_t)L.w[k]->cols; };
+            w16 = std::max({w16, elems(JUNO_T_ATTN_Q) + elems(JUNO_T_ATTN_K) + elems(JUNO_T_ATTN_V), elems(JUNO_T_ATTN_OUT), elems(JUNO_T_FFN_GATE), elems(JUNO_T_FFN_DOWN)});
+        }
+        JUNO_TRY(dev_alloc((void **)&P.weights, 2 * w16 * 2));
+        P.w16[0] = P.weights;
+        P.w16[1] = P.weights + w16 * 2;
+    }
+    while (prompt_alloc_rows(m, rows) != JUNO_OK) {
+        if (P.dev) {  // the old rows make room
+            prompt_release_rows(P);
+        } else if (rows == kPromptMinRows) {
+            prompt_release(P);
+            return JUNO_ERR_OOM;
+        } else {
+            rows /= 2;
+        }
+    }
     return JUNO_OK;
 }
 
@@ -1623,14 +1657,15 @@ static int prefill_run(juno_model *m, juno_seq *seq, const int32_t *token_ids, i
     cudaStream_t st = c->stream;
     bool odd = false;
     const int32_t *marked = nullptr;
+    // without memory for the workspace of the many-row path the portion goes through the smaller passes
+    const int prompt_rows = prompt_takes(m, n_tokens) && prompt_reserve(m, n_tokens) == JUNO_OK ? m->prompt.rows : 0;
     for (int done = 0; done < n_tokens;) {
-        // without memory for the workspace of the many-row path the portion goes through the smaller passes
-        const bool many = prompt_takes(m, n_tokens - done) && prompt_reserve(m, n_tokens - done) == JUNO_OK;
-        const int n = std::min(many ? std::min(m->prompt.rows, kPromptRows) : chunk_max, n_tokens - done), pos0 = start_pos + done;
+        const bool many = prompt_rows > 0 && prompt_takes(m, n_tokens - done);
+        const int n = std::min(many ? prompt_rows : chunk_max, n_tokens - done), pos0 = start_pos + done;
         JUNO_TRY(step_sync(m));  // the pinned step buffer is reused
         JUNO_TRY(seq_reserve(seq, pos0, pos0 + n, st));
         int32_t *h = many ? m->prompt.h_step : m->h_step, *d = many ? m->prompt.step : m->d_step;
-        const int ld = many ? m->prompt.rows : B;
+        const int ld = many ? prompt_rows : B;
         if (many) {  // the word may still hold what an earlier call left there
             odd = odd || (done > 0 && h[4 * ld]);
             h[4 * ld] = 0;

@@ -33,11 +33,12 @@ struct JunoGraph {
 // prompt that needs it, grown by longer ones, kept until the model is freed.
 struct JunoPrompt {
     int rows = 0;
-    uint8_t *dev = nullptr;  // one allocation, carved up below
+    uint8_t *weights = nullptr;  // w16: the same size for every pass
+    uint8_t *dev = nullptr;      // the row buffers below, one allocation
     float *x[2], *qkv, *att, *proj, *hdn, *scale;
     void *img, *w16[2];
     float2 *cs;
-    int32_t *step;           // tokens | positions | slots | lengths, `rows` each
+    int32_t *step;              // tokens | positions | slots | lengths, `rows` each
     int32_t *h_step = nullptr;  // pinned mirror, and behind it the word that PromptAttnArgs::v_odd points to
 };
 

@@ -129,3 +129,46 @@ def test_values_beyond_fp16_stay_behind_their_position(ctx, arch, n, start, at):
     assert np.isfinite(got["plain"]).all() and not np.isfinite(got["odd"][at]).any()
     assert np.array_equal(got["odd"][:at], got["plain"][:at])
     h.release_gpu_resources()
+
+
+# rows of a pass take 71 KB each, the FP16 matrices 67 MB: what is left decides how many positions go in one
+@pytest.mark.parametrize("before,left_mb,passes", [(200, 40, 4), (0, 100, 8), (0, 60, None)])
+def test_prompts_with_little_memory_left(ctx, before, left_mb, passes):
+    """2,000 positions where memory is short: passes of as many rows as there is room for (not fewer than an earlier prompt had), or the
+    small passes; and whole again when memory is back."""
+    import torch
+    from juno_b200.handler import B200TransformerHandler
+    arch = synth.Arch(1024, 2, 16, 4, 8192, 512, 1e-5, 10000.0)
+    toks = np.random.default_rng(4).integers(0, arch.vocab, 2000)
+    places = [0, 700, 1999]
+
+    def opened():
+        h = B200TransformerHandler(arch, ctx, max_batch=64, max_seqs=2, max_ctx=2048)
+        return h.load(tame(synth.random_model(arch, 54, MAPS["q8_0"], norm="random")))
+
+    def launches(h):
+        n = ctx.counters()["kernel_launches"]
+        rows = h.prefill_logits("a", toks, 0, places)
+        return rows, ctx.counters()["kernel_launches"] - n
+
+    h = opened()
+    h.prefill("a", toks[:60], 0)
+    want, whole = launches(h)
+    h.release_gpu_resources()
+    h = opened()
+    if before:
+        h.prefill("a", toks[:before], 0)
+    torch.cuda.empty_cache()
+    held = torch.empty(torch.cuda.mem_get_info()[0] - (left_mb << 20), dtype=torch.uint8, device="cuda")
+    got, count = launches(h)
+    del held
+    torch.cuda.empty_cache()
+    again, count_again = launches(h)
+    h.release_gpu_resources()
+    assert max(rel_err(g, w) for g, w in zip(got, want)) < TOL
+    assert np.array_equal(again, want) and count_again == whole
+    per_pass, logits, hidden = whole - 3, 2, 1
+    if passes is None:
+        assert count > 500  # 32 small passes
+    else:
+        assert count == passes * per_pass + 3 * logits + hidden, (count, whole)

@@ -70,9 +70,9 @@ int juno_ctx_synchronize(juno_ctx *ctx);
 /* The cudaStream_t all work of this context is enqueued on (replaces the per-thread stream of
  * CudaMatVec.java:73-82); a host may record its own events on it. */
 int juno_ctx_stream(juno_ctx *ctx, void **stream);
-/* Page-locked host memory for results: a copy into it runs at the rate of the link, and its pages are mapped already.  Blocks are kept
- * for the next allocation (at most 96 MB in all, held and idle); JUNO_ERR_OOM when there is no room, then any memory will do.
- * A block stays valid after the context closed. */
+/* Page-locked host memory for results: a copy into it runs at the rate of the link, and its pages are mapped already.  Freed blocks are
+ * kept for the next allocation of about their size (at most 96 MB in all, held and idle); JUNO_ERR_OOM when there is no room, then any
+ * memory will do.  A block stays valid after the context closed. */
 int juno_host_alloc(juno_ctx *ctx, int64_t bytes, void **block);
 int juno_host_free(void *block);
 

@@ -1,5 +1,6 @@
 // Context, device discovery, error text and the MatVec-operator entry points of the C ABI.
 #include <cstring>
+#include <iterator>
 #include <map>
 #include <mutex>
 #include <string>
@@ -81,20 +82,32 @@ int wait_status(juno_ctx *c, WaitWord which) {
 }
 
 // Page-locked blocks for results that a host reads.  One pool for the process, because a result may outlive the context that wrote
-// it; blocks come in powers of two, at most kHostPoolBytes of them in all, and those that nobody holds are given back when a
-// context closes or another size needs the room.
+// it.  A block is at most an eighth longer than asked for (short ones: a multiple of 256 KB), all of them together have at most
+// kHostPoolBytes; those that nobody holds are given back when a context closes, and as many of them as it takes when another size needs
+// the room.
 constexpr size_t kHostPoolBytes = (size_t)96 << 20, kHostBlockMin = (size_t)256 << 10;
 struct HostPool {
     std::mutex mu;
     std::map<void *, size_t> held;
     std::multimap<size_t, void *> idle;
-    size_t total = 0;
-    void release_idle() {
-        for (auto &b : idle) {
-            cudaFreeHost(b.second);
-            total -= b.first;
+    size_t held_bytes = 0, idle_bytes = 0;
+    static size_t block_size(size_t bytes) {
+        size_t unit = kHostBlockMin;
+        while (unit * 16 <= bytes) unit *= 2;
+        return (bytes + unit - 1) / unit * unit;
+    }
+    void hold(void *p, size_t size) {
+        held[p] = size;
+        held_bytes += size;
+    }
+    // Gives idle blocks back, the longest first, until at most `most` bytes of them are left.
+    void release_idle(size_t most) {
+        while (idle_bytes > most) {
+            const auto it = std::prev(idle.end());
+            cudaFreeHost(it->second);
+            idle_bytes -= it->first;
+            idle.erase(it);
         }
-        idle.clear();
     }
 };
 static HostPool &host_pool() {
@@ -111,27 +124,30 @@ extern "C" {
 int juno_host_alloc(juno_ctx *c, int64_t bytes, void **out) {
     JUNO_TRY(ctx_check(c));
     JUNO_REQUIRE(out && bytes > 0, "bad host allocation (%lld bytes)", (long long)bytes);
-    size_t size = kHostBlockMin;
-    while (size < (size_t)bytes && size < kHostPoolBytes) size *= 2;
+    const size_t size = HostPool::block_size((size_t)std::min<int64_t>(bytes, kHostPoolBytes + 1));
     HostPool &h = host_pool();
     std::lock_guard<std::mutex> lk(h.mu);
-    const auto it = h.idle.find(size);
-    if (it != h.idle.end() && size >= (size_t)bytes) {
+    const auto it = h.idle.lower_bound(size);
+    if (it != h.idle.end() && it->first <= size + size / 4) {
         *out = it->second;
-        h.held[it->second] = size;
+        h.hold(it->second, it->first);
+        h.idle_bytes -= it->first;
         h.idle.erase(it);
         return JUNO_OK;
     }
-    DeviceGuard g(c->device);
-    if (h.total + size > kHostPoolBytes) h.release_idle();
     void *p = nullptr;
-    if (size < (size_t)bytes || h.total + size > kHostPoolBytes || cudaHostAlloc(&p, size, cudaHostAllocPortable) != cudaSuccess) {
-        cudaGetLastError();
+    bool ok = h.held_bytes + size <= kHostPoolBytes;  // otherwise giving back would not help
+    if (ok) {
+        DeviceGuard g(c->device);
+        h.release_idle(kHostPoolBytes - h.held_bytes - size);
+        ok = cudaHostAlloc(&p, size, cudaHostAllocPortable) == cudaSuccess;
+        if (!ok) cudaGetLastError();
+    }
+    if (!ok) {
         set_error("no page-locked block of %lld bytes is free", (long long)bytes);
         return JUNO_ERR_OOM;
     }
-    h.total += size;
-    h.held[p] = size;
+    h.hold(p, size);
     *out = p;
     return JUNO_OK;
 }
@@ -142,6 +158,8 @@ int juno_host_free(void *block) {
     const auto it = h.held.find(block);
     JUNO_REQUIRE(it != h.held.end(), "not a block of juno_host_alloc");
     h.idle.emplace(it->second, block);
+    h.idle_bytes += it->second;
+    h.held_bytes -= it->second;
     h.held.erase(it);
     return JUNO_OK;
 }
@@ -233,7 +251,7 @@ int juno_ctx_destroy(juno_ctx *c) {
     {
         HostPool &h = host_pool();
         std::lock_guard<std::mutex> hk(h.mu);
-        h.release_idle();
+        h.release_idle(0);
     }
     c->magic = kMagicDead;  // record kept: a second destroy reports CLOSED
     return JUNO_OK;

@@ -72,7 +72,8 @@ int launch_gemm_rows(juno_ctx *c, int dt, const GemmArgs &a, unsigned *err, cuda
                      (a.epi != GE_GEGLU || (a.N % 16 == 0 && a.groups == 1)),
                  "matrix product: bad arguments (M %d, N %d, K %d)", a.M, a.N, a.K);
     const double es = dt_bytes(dt);
-    const double algo = a.groups * ((double)a.M * a.K + (double)a.N * a.K) * es + (double)a.groups * a.M * a.N * (a.epi == GE_F32 ? 4.0 : es);
+    const bool f32_out = a.epi == GE_F32 || a.epi == GE_F32_ROW || a.epi == GE_SILU_ROW, half_out = a.epi == GE_GEGLU || a.epi == GE_SILU_ROW;
+    const double algo = a.groups * ((double)a.M * a.K + (double)a.N * a.K) * es + (double)a.groups * a.M * (half_out ? a.N / 2 : a.N) * (f32_out ? 4.0 : es);
     ProfScope prof(c, st, PROF_GEMM_ROWS, algo);
     // Up to kFewRows rows the weights' way from memory is the bound, above them the MMAs.  A pass of Vosotar medium through the one
     // and the other: 20 rows 0.75 and 1.34 ms, 100 rows 0.94 and 1.35, 128 rows 0.99 and 1.36; Desilorn small, 100 rows: 0.95 and 1.20.

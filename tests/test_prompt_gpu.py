@@ -172,3 +172,21 @@ def test_prompts_with_little_memory_left(ctx, before, left_mb, passes):
         assert count > 500  # 32 small passes
     else:
         assert count == passes * per_pass + 3 * logits + hidden, (count, whole)
+
+
+def test_profiled_bytes_of_the_products(ctx):
+    """What the profile counts for the products of a prompt: 16-bit operands, FP32 results, one column per gate and up row."""
+    from juno_b200.handler import B200TransformerHandler
+    a, n = SMALL128, 100
+    h = B200TransformerHandler(a, ctx, max_batch=64, max_seqs=1, max_ctx=128)
+    h.load(synth.random_model(a, 55))
+    ctx.profile(True)
+    ctx.profile_read()
+    h.prefill("a", np.arange(n), 0)
+    got = ctx.profile_read()["gemm_rows"]
+    ctx.profile(False)
+    kv = a.hidden // a.n_heads * a.n_kv_heads
+    shapes = [(a.hidden, a.hidden + 2 * kv, 1), (a.hidden, a.hidden, 1), (a.hidden, 2 * a.inter, 2), (a.inter, a.hidden, 1)]  # columns, rows, rows per result
+    want = sum(2 * k * (n + rows) + 4 * n * rows // per for k, rows, per in shapes)
+    assert got["launches"] == 4 * a.n_layers and got["algo_bytes"] == want * a.n_layers
+    h.release_gpu_resources()

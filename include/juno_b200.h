@@ -312,10 +312,12 @@ int juno_model_seq_create(juno_model *m, juno_seq **out);
 int juno_forward(juno_model *m, int32_t n, juno_seq *const *seqs, const int32_t *token_ids,
                  const int32_t *positions, float *logits_host, int32_t *argmax_out);
 /* Prompt prefill in chunks: feeds token_ids[0..n_tokens) of ONE sequence at positions start_pos.. and fills its KV
- * pages (causal attention inside a pass).  Portions of more than min(max_batch, 64) positions go in passes of up to 2048
- * through FP16 copies of the weights, made matrix by matrix; shorter ones, tensor-parallel models and devices without memory
- * for that workspace in passes of up to min(max_batch, 64) through the batched dequant-GEMM kernels.  Replaces the token-by-token prefill loop of GenerationLoop.java:306-317 (same positions, same
- * cache contents up to the FP16 rounding of the batched path).  logits_host ([vocab]) and argmax_out (one id) are
+ * pages (causal attention inside a pass).  Portions of more than min(max_batch, 64) positions (twice that where it is below
+ * eight) go in passes of up to 2048 through FP16 copies of the weights, made matrix by matrix, fewer where memory is short; shorter
+ * ones, tensor-parallel models and devices without memory for that workspace in passes of up to min(max_batch, 64) through the
+ * batched dequant-GEMM kernels.  The workspace stays with the model.  A portion whose values do not all fit FP16 pages is fed twice
+ * (later positions must not reach earlier ones).  Replaces the token-by-token prefill loop of GenerationLoop.java:306-317 (same
+ * positions, same cache contents up to the FP16 rounding of the batched path).  logits_host ([vocab]) and argmax_out (one id) are
  * optional and refer to the LAST position fed.  Tensor parallel models: logits only with an unsharded vocabulary. */
 int juno_prefill(juno_model *m, juno_seq *seq, const int32_t *token_ids, int32_t n_tokens, int32_t start_pos,
                  float *logits_host, int32_t *argmax_out);

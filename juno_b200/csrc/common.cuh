@@ -130,7 +130,9 @@ struct ProfScope {
 
 // Programmatic dependent launch: a kernel launched with the attribute may be scheduled while the previous kernel of
 // the stream is still running; it must execute pdl_wait() before it touches anything that kernel (or an earlier one)
-// produces.  Here only weight prefetches and a launch-private work counter happen before the wait.
+// produces.  Before the wait kernels here fetch weights and count work of their own.  One writes: dequant_rows_kernel (prompt.cu) fills the
+// buffer that the product before its predecessor read.  That is safe as long as the row products trigger their dependents only after
+// their own wait, and every kernel waits before it ends: what runs beside a product then knows that everything before that one is done.
 inline bool pdl_enabled() {
     static const bool on = [] {
         const char *v = getenv("JUNO_NO_PDL");

@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) gemm_pair_kernel(const __grid
     const uint32_t tmem = *reinterpret_cast<volatile uint32_t *>(&tmem_slot);
     const GemmArgs &g = p.g;
     pdl_wait();
-    pdl_launch_dependents();
+    pdl_launch_dependents();  // not before the wait: dequant_rows_kernel (prompt.cu) may be next and write what the product before this one read
 
     if (warp == 0) {
         if (lane == 0) {
@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) gemm_pair_split_kernel(const 
     const uint32_t tmem = *reinterpret_cast<volatile uint32_t *>(&tmem_slot);
     const GemmArgs &g = p.g;
     pdl_wait();
-    pdl_launch_dependents();
+    pdl_launch_dependents();  // not before the wait: dequant_rows_kernel (prompt.cu) may be next and write what the product before this one read
     int ok = 0;  // epilogue warps: the accumulator is complete
     const int quad = warp & 3;
     const uint32_t acc = tmem + ((uint32_t)(quad * 32) << 16), mine = stage0 + (uint32_t)(quad * 32 + lane) * 4;  // partial sums: [column][row]

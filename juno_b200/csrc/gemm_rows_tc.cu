@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) gemm_rows_tc_kernel(const __g
     const uint32_t tmem = *reinterpret_cast<volatile uint32_t *>(&tmem_slot);
     const GemmArgs &g = p.g;
     pdl_wait();
-    pdl_launch_dependents();
+    pdl_launch_dependents();  // not before the wait: dequant_rows_kernel (prompt.cu) may be next and write what the product before this one read
 
     if (warp == 0) {
         if (lane == 0) {

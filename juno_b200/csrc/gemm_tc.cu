@@ -535,9 +535,10 @@ bool gemm_tc_enabled() {
 }
 int gemm_tc_padded_batch(int batch) { return (batch + 15) / 16 * 16; }
 size_t gemm_tc_image_bytes(int K, int batch) { return (size_t)K * gemm_tc_padded_batch(batch) * 2; }
-// Shapes this kernel takes: enough 128-row blocks to occupy the GPU, and a batch from which it measured faster than the
-// mma.sync kernel (its time hardly depends on the batch: 185-209 us on 128256 x 4096 Q4_K for 16-64 sequences, against
-// 138-294 us).
+// Shapes this kernel takes: enough 128-row blocks to occupy the GPU, and a batch from which it pays on Q4_K, the format of most large
+// matrices.  This kernel / the mma.sync kernel on 128256 x 4096, us with the staging of the input: Q4_K 32 rows 204 / 185, 48 rows
+// 214 / 220, 64 rows 226 / 249; Q6_K 48 rows 282 / 230, 64 rows 292 / 265; Q8_0 48 rows 306 / 210, 64 rows 322 / 245.  Q6_K and Q8_0
+// matrices of this size would be better off over there; the line does not tell the formats apart.
 bool gemm_tc_shape_ok(const juno_ctx *ctx, int row_tiles, int batch) {
     static const int min_batch = [] {
         const char *e = getenv("JUNO_GEMM_TC_MIN_BATCH");

@@ -124,7 +124,9 @@ struct DequantParams {
     __half *out;
 };
 // Runs beside the product before it, whose CTAs leave room for it on every SM: it writes the buffer that the product before that one
-// read, and waits for its predecessor at its end only, so that what follows it finds both complete.  Alone it is bound by the writes of 2 bytes a
+// read, and waits for its predecessor at its end only, so that what follows it finds both complete.  It may write before the wait because
+// it cannot start before the product beside it has passed its own (the row products trigger their dependents after it), and by then all
+// that came before that product is done.  Alone it is bound by the writes of 2 bytes a
 // weight.  One warp per 16 x 256 tile; neighbouring warps take neighbouring tiles of a row tile, so a CTA writes whole 4 KB pieces of rows.  Behind the product in turn:
 // TinyLlama Q8_0, 333 positions 3.55 ms; beside it 3.26 ms (Llama-3-8B, 2048 positions, where the tensor cores' power is the limit: 39.6 and 39.4 ms).
 constexpr int kDequantCtas = 2;  // per SM: with 64 registers a thread both fit beside a CTA of the product; one that did not would start after it

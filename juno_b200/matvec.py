@@ -20,9 +20,10 @@ def _ptr(a: np.ndarray):
     return a.ctypes.data_as(C.c_void_p)
 
 
-# Results from this size on are returned in page-locked memory: a copy into fresh pages runs at 6-25 GB/s (3 MB: 120-530 us), into these at
-# 50 GB/s.  Around a hundred kilobytes the gain reaches what the array costs to make (TinyLlama's 128 KB: 0.789 -> 0.786 ms per step; 256 KB
-# of Desilorn medium: 0.578 -> 0.565).
+# Logits and products from this size on are returned in page-locked memory (GpuContext.host_rows): a copy into fresh pages runs at 6-25 GB/s
+# (3 MB: 120-530 us), into these at 50 GB/s.  Around a hundred kilobytes the gain reaches what the array costs to make: 256 KB of Desilorn
+# medium 0.578 -> 0.565 ms per step; the 128,000 bytes of a vocabulary of 32,000, just below, 0.789 -> 0.786.  `prefill` and
+# `PagedKvCache.attention` return ordinary arrays.
 PINNED_FROM = 1 << 17
 
 

@@ -364,7 +364,7 @@ def main():
     peak, peak_kind = measured_peaks()
     g = prof["gemv_q4k"]
     kname = ("qgemv_kernel<Q4_K> (integer tensor-core fused dequant-GEMV)" if B < 9 else
-             "gemm_kernel<Q4_K> / gemm_tc_kernel<Q4_K> (one-pass batched dequant-GEMM)")
+             "gemm_quant_kernel (one-pass batched dequant-GEMM)")
     # Profiling mode runs the step eagerly with events round every launch: its times include launch gaps the CUDA graph
     # does not have.  What is reported for the dominant kernel is its SHARE of the event-timed step applied to the
     # graph's step time, so that the kernel times of a step add up to ms_per_step.

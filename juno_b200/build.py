@@ -16,7 +16,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "libjuno_b200.so")
-SOURCES = ["context.cu", "gemv.cu", "qgemv.cu", "gemm.cu", "gemm_tc.cu", "attn.cu", "model.cu", "gguf_file.cu",
+SOURCES = ["context.cu", "gemv.cu", "qgemv.cu", "gemm_quant_tc.cu", "attn.cu", "model.cu", "gguf_file.cu",
            "safetensors_file.cu", "registry.cu", "stack_loader.cu", "vosotar.cu", "desilorn.cu", "stack.cu", "stack_decode.cu", "gemv_rows.cu",
            "rowops.cu", "streams.cu", "gemm_rows.cu", "gemm_rows_tc.cu", "gemm_few_tc.cu", "gemm_pair_tc.cu", "latent_attn.cu", "latent_attn_mma.cu", "flash_attn.cu",
            "grouped_attn.cu", "prompt.cu"]

@@ -1,4 +1,4 @@
-// Shared-memory loads, mbarriers with bounded waits and bulk copies of the quantised products (qgemv.cu, gemm.cu).
+// Shared-memory loads, mbarriers with bounded waits and bulk copies of the quantised products (qgemv.cu, gemm_quant_tc.cu).
 #pragma once
 #include <stdint.h>
 

@@ -8,7 +8,9 @@
 #include "common.cuh"
 #include <algorithm>
 
+#include "gemm_quant.cuh"
 #include "gemv.cuh"
+#include "prompt.cuh"
 #include "qgemv.cuh"
 
 namespace juno {
@@ -395,54 +397,41 @@ static int gemv_on_stream(juno_ctx *c, juno_qmat *m, const float *x, int batch, 
         q.ldx = (int)m->cols;
         return launch_qgemv(c, q, st);
     }
-    const size_t need = gemm_image_bytes((int)m->cols, std::min(batch, kGemmMaxBatch));
+    const size_t need = (size_t)m->cols * 2 * std::min(batch, kGemmMaxBatch);
     void *pi = c->gemv_scratch.ximg;
     JUNO_TRY(ensure_device(&pi, &c->gemv_scratch.ximg_bytes, need));
     c->gemv_scratch.ximg = (uint8_t *)pi;
-    GemvArgs a;
-    a.nseg = 1;
-    a.seg[0].w = m->dev;
-    a.seg[0].rows = (int)m->rows;
-    a.seg[0].row_tiles = (int)m->row_tiles;
-    a.type = m->type;
-    a.K = (int)m->cols;
-    a.ld_out = (int)m->rows;
-    a.ximg = c->gemv_scratch.ximg;
-    StageArgs sa;
-    sa.mode = STAGE_PLAIN;
-    sa.ldx = (int)m->cols;
-    sa.K = (int)m->cols;
-    sa.img = c->gemv_scratch.ximg;
-    // one pass over the weights per group of up to kGemmMaxBatch rows
     if (!c->gemv_scratch.xscale) {
-        cudaError_t e = cudaMalloc((void **)&c->gemv_scratch.xscale, (kGemmMaxBatch + 4) * sizeof(float));  // + an error word for the tcgen05 kernel
+        cudaError_t e = cudaMalloc((void **)&c->gemv_scratch.xscale, kGemmMaxBatch * sizeof(float));
         if (e != cudaSuccess) {
             cudaGetLastError();
             set_error("cudaMalloc of %zu bytes failed: %s", kGemmMaxBatch * sizeof(float), cudaGetErrorString(e));
             return JUNO_ERR_OOM;
         }
-        JUNO_CUDA_TRY(cudaMemset(c->gemv_scratch.xscale, 0, (kGemmMaxBatch + 4) * sizeof(float)));
     }
+    // one pass over the weights per group of up to kGemmMaxBatch rows
     for (int b0 = 0; b0 < batch; b0 += kGemmMaxBatch) {
-        const int bc = std::min(kGemmMaxBatch, batch - b0);
-        if (gemm_tc_enabled() && gemm_tc_shape_ok(c, (int)m->row_tiles, bc)) {  // tcgen05/TMEM kernel (opt-in)
-            void *pt = c->gemv_scratch.ximg;
-            JUNO_TRY(ensure_device(&pt, &c->gemv_scratch.ximg_bytes, gemm_tc_image_bytes((int)m->cols, bc) + 16));
-            c->gemv_scratch.ximg = (uint8_t *)pt;
-            unsigned *err = reinterpret_cast<unsigned *>(c->gemv_scratch.xscale + kGemmMaxBatch);
-            JUNO_TRY(launch_stage_tc(c, x + (size_t)b0 * m->cols, (int)m->cols, (int)m->cols, bc, c->gemv_scratch.ximg,
-                                     c->gemv_scratch.xscale, st));
-            JUNO_TRY(launch_gemm_tc(c, m->dev, m->type, (int)m->rows, (int)m->row_tiles, (int)m->cols, bc, c->gemv_scratch.ximg,
-                                    c->gemv_scratch.xscale, y + (size_t)b0 * m->rows, (int)m->rows, EPI_STORE, err, st));
-            continue;
-        }
-        sa.x = x + (size_t)b0 * m->cols;
-        sa.batch = bc;
-        JUNO_TRY(launch_stage_f16(c, sa, c->gemv_scratch.xscale, st));
+        StageRowsArgs s;
+        s.x = x + (size_t)b0 * m->cols;
+        s.n = std::min(kGemmMaxBatch, batch - b0);
+        s.K = (int)m->cols;
+        s.out = c->gemv_scratch.ximg;
+        s.scale = c->gemv_scratch.xscale;
+        s.quant_order = true;
+        JUNO_TRY(launch_stage_rows(c, s, st));
+        GemmQuantArgs a;
+        a.seg[0].w = m->dev;
         a.seg[0].out = y + (size_t)b0 * m->rows;
-        a.batch = bc;
-        a.xscale = c->gemv_scratch.xscale;
-        JUNO_TRY(launch_gemm(c, a, st));
+        a.seg[0].rows = (int)m->rows;
+        a.seg[0].row_tiles = (int)m->row_tiles;
+        a.seg[0].type = m->type;
+        a.seg[0].row_pow = m->row_pow;
+        a.K = s.K;
+        a.n = s.n;
+        a.x = s.out;
+        a.scale = s.scale;
+        a.ld_out = (int)m->rows;
+        JUNO_TRY(launch_gemm_quant(c, a, st));
     }
     return JUNO_OK;
 }
@@ -482,15 +471,6 @@ int juno_gemv(juno_ctx *c, juno_qmat *m, const float *x_host, int32_t batch, flo
     JUNO_CUDA_TRY(cudaMemcpyAsync(y_host, c->stage_y, yb, cudaMemcpyDeviceToHost, c->stream));
     JUNO_CUDA_TRY(cudaStreamSynchronize(c->stream));
     JUNO_TRY(wait_status(c, WAIT_BLOCKING));
-    if (c->gemv_scratch.xscale && batch >= gemm_min_batch()) {  // did a wait inside the tcgen05 kernel give up?
-        unsigned code = 0;
-        JUNO_CUDA_TRY(cudaMemcpy(&code, c->gemv_scratch.xscale + kGemmMaxBatch, 4, cudaMemcpyDeviceToHost));
-        if (code) {
-            JUNO_CUDA_TRY(cudaMemset(c->gemv_scratch.xscale + kGemmMaxBatch, 0, 4));
-            set_error("batched tensor-core product gave up waiting (code %u, block %u)", code & 0xffu, code >> 8);
-            return JUNO_ERR_CUDA;
-        }
-    }
     c->h2d_bytes += (int64_t)xb;
     c->d2h_bytes += (int64_t)yb;
     return JUNO_OK;

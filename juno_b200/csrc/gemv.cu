@@ -1,6 +1,6 @@
 // Resident quantised matrices: repack of raw GGUF blocks into the 16x256 tile layout (layout.cuh), bit-exact
 // dequantisation (LlamaTransformerHandler.dequantize :873-1135) and the plain kernels for shapes the tile layout
-// does not cover.  The fused dequant-GEMV itself lives in qgemv.cu (1..8 sequences) and gemm.cu / gemm_tc.cu
+// does not cover.  The fused dequant-GEMV itself lives in qgemv.cu (1..8 sequences) and gemm_quant_tc.cu
 // (9..64 sequences).
 #include <cuda_fp16.h>
 
@@ -125,6 +125,30 @@ int launch_dequant(juno_ctx *ctx, const juno_qmat *m, int64_t row_start, int64_t
 }
 
 // ───────────────────────────── resident matrix ─────────────────────────────────────────────
+// The power of two of every row (tile_f16.cuh): what brings the largest scale of the row, times what it is multiplied with, into
+// [2^14, 2^15), as two FP16 factors.  One warp per row tile: 16 rows x two super-blocks at a time.
+__global__ void row_pow_kernel(int type, const uint8_t *tiles, int64_t nb, uint32_t *pow) {
+    const int lane = threadIdx.x, row = lane & 15;
+    const uint8_t *t0 = tiles + (size_t)blockIdx.x * nb * tile_bytes(type);
+    auto half_at = [](const uint8_t *p) { return fabsf(__half2float(*reinterpret_cast<const __half *>(p))); };
+    float top = 0.f;
+    for (int64_t sb = lane >> 4; sb < nb; sb += 2) {
+        const uint8_t *t = t0 + sb * tile_bytes(type);
+        if (type == 12)
+            top = fmaxf(top, fmaxf(63.f * half_at(t + row * 4), half_at(t + row * 4 + 2)));
+        else if (type == 14)
+            top = fmaxf(top, 128.f * half_at(t + 3328 + row * 2));
+        else
+            for (int j = 0; j < 8; j++) top = fmaxf(top, half_at(t + 4096 + row * 16 + j * 2));
+    }
+    top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 16));
+    int e = 15;
+    if (top > 0.f && top < 3.0e38f) frexpf(top, &e);
+    const int p = min(15 - e, 30), a = min(p, 15);
+    if (lane < 16)
+        pow[blockIdx.x * 16 + row] = (uint32_t)__half_as_ushort(__float2half_rn(ldexpf(1.f, a))) | (uint32_t)__half_as_ushort(__float2half_rn(ldexpf(1.f, p - a))) << 16;
+}
+
 int qmat_create(juno_ctx *ctx, const void *blocks, int type, int64_t rows_total, int64_t cols_total, int64_t row0,
                 int64_t nrows, int64_t sb0, int64_t nsb, juno_qmat **out) {
     JUNO_REQUIRE(type == 0 || type == 8 || type == 12 || type == 14, "unsupported GGML type %d", type);
@@ -182,7 +206,7 @@ int qmat_create(juno_ctx *ctx, const void *blocks, int type, int64_t rows_total,
     } else {
         m->bytes = (size_t)m->row_tiles * m->nb * tile_bytes(type);
         uint8_t *tmp = nullptr;
-        if (cudaMalloc((void **)&m->dev, m->bytes) != cudaSuccess || cudaMalloc((void **)&tmp, raw_bytes) != cudaSuccess) {
+        if (cudaMalloc((void **)&m->dev, m->bytes + (size_t)m->row_tiles * 64) != cudaSuccess || cudaMalloc((void **)&tmp, raw_bytes) != cudaSuccess) {
             cudaGetLastError();
             set_error("cudaMalloc of %zu + %zu bytes failed", m->bytes, raw_bytes);
             return fail(JUNO_ERR_OOM);
@@ -198,8 +222,10 @@ int qmat_create(juno_ctx *ctx, const void *blocks, int type, int64_t rows_total,
                 repack_q6k_kernel<<<blocks_n, threads, 0, st>>>(tmp, (size_t)rrb, (int)nrows, (int)sb0, (int)nsb, m->dev);
             else
                 repack_q80_kernel<<<blocks_n, threads, 0, st>>>(tmp, (size_t)rrb, (int)nrows, (int)sb0, (int)nsb, m->dev);
+            m->row_pow = reinterpret_cast<uint32_t *>(m->dev + m->bytes);
+            row_pow_kernel<<<(unsigned)m->row_tiles, 32, 0, st>>>(type, m->dev, m->nb, m->row_pow);
             e = cudaGetLastError();
-            ctx->kernel_launches++;
+            ctx->kernel_launches += 2;
         }
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
         cudaFree(tmp);

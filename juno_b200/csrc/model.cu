@@ -17,7 +17,7 @@
 #include "attn.cuh"
 #include "common.cuh"
 #include "dequant.cuh"
-#include "gemv.cuh"
+#include "gemm_quant.cuh"
 #include "gemm_rows.cuh"
 #include "model.cuh"
 #include "prompt.cuh"
@@ -357,7 +357,7 @@ static void model_release(juno_model *m) {
         m->pool->owned_by_model = 0;
         kvpool_destroy(m->pool);
     }
-    void *bufs[] = {m->x[0], m->x[1], m->qkv, m->att, m->proj, m->proj2, m->hdn, m->xsc, m->img_h_tc, m->tc_err, m->img_h, m->img_att, m->img_i, m->logits_loc, m->logits_gather, m->logits_full,
+    void *bufs[] = {m->x[0], m->x[1], m->qkv, m->att, m->proj, m->proj2, m->hdn, m->xsc, m->img_h, m->img_att, m->img_i, m->logits_loc, m->logits_gather, m->logits_full,
                     m->attn_scratch, m->rope_cs, m->d_step, m->d_argmax, m->d_pidx, m->d_out_ids, m->d_step_counter,
                     m->d_pval, m->output_norm};
     for (void *b : bufs)
@@ -763,14 +763,11 @@ extern "C" int juno_model_finalize(juno_model *m) {
     JUNO_TRY(dev_alloc((void **)&m->proj, (size_t)B * H * 4));
     JUNO_TRY(dev_alloc((void **)&m->proj2, (size_t)B * H * 4));
     const int Bg = std::min(B, kGemmMaxBatch);
-    JUNO_TRY(dev_alloc((void **)&m->img_h, gemm_image_bytes(H, Bg)));
-    JUNO_TRY(dev_alloc((void **)&m->img_att, gemm_image_bytes(m->heads_loc * hd, Bg)));
-    JUNO_TRY(dev_alloc((void **)&m->img_i, gemm_image_bytes(m->inter_loc, Bg)));
+    JUNO_TRY(dev_alloc((void **)&m->img_h, (size_t)H * Bg * 2));
+    JUNO_TRY(dev_alloc((void **)&m->img_att, (size_t)m->heads_loc * hd * Bg * 2));
+    JUNO_TRY(dev_alloc((void **)&m->img_i, (size_t)m->inter_loc * Bg * 2));
     JUNO_TRY(dev_alloc((void **)&m->hdn, (size_t)B * m->inter_loc * 4));
     JUNO_TRY(dev_alloc((void **)&m->xsc, (size_t)3 * B * 4));
-    JUNO_TRY(dev_alloc((void **)&m->img_h_tc, gemm_tc_image_bytes(H, Bg)));
-    JUNO_TRY(dev_alloc((void **)&m->tc_err, 4));
-    JUNO_CUDA_TRY(cudaMemset(m->tc_err, 0, 4));
     JUNO_TRY(dev_alloc((void **)&m->logits_loc, (size_t)B * m->vocab_loc * 4));
     if (m->vocab_sharded) {
         JUNO_TRY(dev_alloc((void **)&m->logits_gather, (size_t)B * f.vocab * 4));
@@ -788,39 +785,31 @@ extern "C" int juno_model_finalize(juno_model *m) {
 namespace juno {
 
 // ───────────────────────────── one decode step, enqueued on the context stream ────────────
-static int gemv_group(juno_model *m, juno_qmat *const *mats, float *const *outs, int count, const GemvArgs &proto,
-                      cudaStream_t st) {
-    // matrices that share the staged activation share a launch: one block format, or Q4_K mixed with Q6_K
-    int i = 0;
-    while (i < count) {
-        int j = i + 1;
-        bool mixed = false;
-        while (j < count && j - i < 3) {
-            const int ta = mats[i]->type, tb = mats[j]->type;
-            const bool k_quant = m->mix_formats && (ta == 12 || ta == 14) && (tb == 12 || tb == 14);
-            if (tb != ta && !k_quant) break;
-            if (tb != mats[j - 1]->type || tb != ta) mixed = mixed || (tb != ta);
-            j++;
-        }
-        GemvArgs a = proto;
-        a.nseg = j - i;
-        for (int s = 0; s < a.nseg; s++) {
-            a.seg[s].w = mats[i + s]->dev;
-            a.seg[s].out = outs[i + s];
-            a.seg[s].rows = a.epi == EPI_SILU_PAIR ? (int)mats[i + s]->rows / 2 : (int)mats[i + s]->rows;
-            a.seg[s].row_tiles = (int)mats[i + s]->row_tiles;
-            a.seg[s].type = mats[i + s]->type;
-        }
-        a.type = mixed ? 0 : mats[i]->type;
-        a.K = (int)mats[i]->cols;
-        JUNO_TRY(launch_gemm(m->ctx, a, st));
-        i = j;
+// Product of matrices that share the staged rows x [n][K].
+static int quant_group(juno_model *m, juno_qmat *const *mats, float *const *outs, int count, int epi, int n, const void *x, const float *scale, int ld_out,
+                       cudaStream_t st, bool precise = false) {
+    GemmQuantArgs a;
+    a.nseg = count;
+    for (int s = 0; s < count; s++) {
+        a.seg[s].w = mats[s]->dev;
+        a.seg[s].out = outs[s];
+        a.seg[s].rows = epi == EPI_SILU_PAIR ? (int)mats[s]->rows / 2 : (int)mats[s]->rows;
+        a.seg[s].row_tiles = (int)mats[s]->row_tiles;
+        a.seg[s].type = mats[s]->type;
+        a.seg[s].row_pow = mats[s]->row_pow;
     }
-    return JUNO_OK;
+    a.K = (int)mats[0]->cols;
+    a.n = n;
+    a.x = x;
+    a.scale = scale;
+    a.ld_out = ld_out;
+    a.epi = epi;
+    a.precise = precise;
+    return launch_gemm_quant(m->ctx, a, st);
 }
 
 // Layers and output projection of one step on the batched path (n >= gemm_min_batch()): every product is ONE pass
-// over its weights for all n sequences (launch_gemm), with separate staging kernels in between (they need the
+// over its weights for all n sequences (launch_gemm_quant), with separate staging kernels in between (they need the
 // whole row for its power-of-two factor).  x[0] holds the embeddings on entry; the residual stream ends in x[cur].
 static int enqueue_layers_batched(juno_model *m, int n, const int32_t *d_slot, const int32_t *d_len, int n_splits, int &cur,
                                   cudaStream_t st, const int32_t *d_prefill_pos = nullptr, bool want_logits = true) {
@@ -829,37 +818,23 @@ static int enqueue_layers_batched(juno_model *m, int n, const int32_t *d_slot, c
     const int H = f.hidden, hd = m->hd, B = f.max_batch;
     const int Hl = m->heads_loc * hd, KVl = m->kv_loc * hd, Il = m->inter_loc;
     float *sc_h = m->xsc, *sc_att = m->xsc + B, *sc_i = m->xsc + 2 * B;
-    m->tc_used = true;
-    auto stage = [&](int mode, const float *x, int ldx, const float *add, float *x_out, const float *normw, int K, uint8_t *img,
-                     float *sc) {
-        StageArgs a;
-        a.mode = mode;
+    auto stage = [&](const float *x, const float *add, float *x_out, const float *normw, int K, uint8_t *img, float *sc) {
+        StageRowsArgs a;
         a.x = x;
-        a.ldx = ldx;
-        a.x_add = add;
-        a.x_out = x_out;
+        a.add = add;
         a.normw = normw;
+        a.x_out = x_out;
         a.eps = f.rms_eps;
+        a.n = n;
         a.K = K;
-        a.batch = n;
-        a.img = img;
-        return launch_stage_f16(c, a, sc, st, img == m->img_h ? m->img_h_tc : nullptr);
+        a.out = img;
+        a.scale = sc;
+        a.quant_order = true;
+        return launch_stage_rows(c, a, st);
     };
     auto product = [&](juno_qmat *const *mats, float *const *outs, int count, int epi, int ld_out, const uint8_t *img,
-                       const float *sc) {
-        GemvArgs a;
-        a.batch = n;
-        a.ximg = img;
-        a.xscale = sc;
-        a.epi = epi;
-        a.ld_out = ld_out;
-        if (img == m->img_h) {
-            a.ximg_tc = m->img_h_tc;
-            a.tc_err = m->tc_err;
-        }
-        return gemv_group(m, mats, outs, count, a, st);
-    };
-    JUNO_TRY(stage(STAGE_RMSNORM, m->x[0], H, nullptr, nullptr, m->layers[0].attn_norm, H, m->img_h, sc_h));
+                       const float *sc) { return quant_group(m, mats, outs, count, epi, n, img, sc, ld_out, st); };
+    JUNO_TRY(stage(m->x[0], nullptr, nullptr, m->layers[0].attn_norm, H, m->img_h, sc_h));
     cur = 0;
     for (int l = 0; l < f.n_layers; l++) {
         JunoLayer &L = m->layers[l];
@@ -898,26 +873,26 @@ static int enqueue_layers_batched(juno_model *m, int n, const int32_t *d_slot, c
             at.ldkv = m->qkv_ld;
         }
         JUNO_TRY(launch_attn(c, at, st));
-        JUNO_TRY(stage(STAGE_PLAIN, m->att, Hl, nullptr, nullptr, nullptr, Hl, m->img_att, sc_att));
+        JUNO_TRY(stage(m->att, nullptr, nullptr, nullptr, Hl, m->img_att, sc_att));
         // x2 = x + Wo att (summed over ranks first when tensor parallel), staged rmsNorm(x2, ffn_norm)
         juno_qmat *wo[1] = {L.w[JUNO_T_ATTN_OUT]};
         float *po[1] = {m->proj};
         JUNO_TRY(product(wo, po, 1, EPI_STORE, H, m->img_att, sc_att));
         if (m->world > 1)
             JUNO_NCCL_TRY(g_nccl.AllReduce(m->proj, m->proj, (size_t)n * H, kNcclFloat, kNcclSum, m->comm, st));
-        JUNO_TRY(stage(STAGE_RMSNORM, m->x[cur], H, m->proj, m->x[cur ^ 1], L.ffn_norm, H, m->img_h, sc_h));
+        JUNO_TRY(stage(m->x[cur], m->proj, m->x[cur ^ 1], L.ffn_norm, H, m->img_h, sc_h));
         cur ^= 1;
         // hdn = silu(Wgate xn2) * (Wup xn2)
         juno_qmat *gu[1] = {L.w[JUNO_T_FFN_GATE]};
         float *pg[1] = {m->hdn};
         JUNO_TRY(product(gu, pg, 1, EPI_SILU_PAIR, Il, m->img_h, sc_h));
-        JUNO_TRY(stage(STAGE_PLAIN, m->hdn, Il, nullptr, nullptr, nullptr, Il, m->img_i, sc_i));
+        JUNO_TRY(stage(m->hdn, nullptr, nullptr, nullptr, Il, m->img_i, sc_i));
         juno_qmat *wd[1] = {L.w[JUNO_T_FFN_DOWN]};
         JUNO_TRY(product(wd, po, 1, EPI_STORE, H, m->img_i, sc_i));
         if (m->world > 1)
             JUNO_NCCL_TRY(g_nccl.AllReduce(m->proj, m->proj, (size_t)n * H, kNcclFloat, kNcclSum, m->comm, st));
         const float *next_norm = (l + 1 < f.n_layers) ? m->layers[l + 1].attn_norm : m->output_norm;
-        JUNO_TRY(stage(STAGE_RMSNORM, m->x[cur], H, m->proj, m->x[cur ^ 1], next_norm, H, m->img_h, sc_h));
+        JUNO_TRY(stage(m->x[cur], m->proj, m->x[cur ^ 1], next_norm, H, m->img_h, sc_h));
         cur ^= 1;
     }
     if (!want_logits) return JUNO_OK;
@@ -938,6 +913,20 @@ static bool prompt_takes(const juno_model *m, int n) {
     if (m->stack || m->world > 1) return false;
     const int chunk = std::min(m->cfg.max_batch, kGemmMaxBatch);
     return n > (chunk >= 8 ? chunk : 2 * chunk);
+}
+
+// Do the products of a portion of n positions unpack the quantised tiles themselves (gemm_quant_tc.cu)?  That costs an unpacking per 224 rows,
+// where FP16 rows of the weights cost one for all of them, a write and a read, and the product itself runs on pairs of SMs.  FP16 rows / unpacking: Llama-3-8B
+// 70 / 200 / 333 / 500 positions 10.3 / 9.8 / 13.5 / 13.8 and 4.2 / 5.5 / 8.6 / 12.9 ms; TinyLlama Q4_K_M 70 / 200 / 333 / 500 positions 2.70 / 3.31 / 3.17 / 3.64 and
+// 1.77 / 2.23 / 2.74 / 3.33 ms, 600 positions 3.39 and 3.59.  Layers with fewer tiles than there are warps to unpack them are all launches: two layers of width 512, 250
+// positions 145 and 165 us (four of width 1024, 2752 tiles each: 381 and 342).
+constexpr int kFusedRows = 512, kFusedTiles = 2368;
+static bool prompt_fused(const juno_model *m, int n) {
+    if (m->stack || n > kFusedRows) return false;
+    int64_t tiles = 0;
+    for (const juno_qmat *w : m->layers[0].w)
+        if (w) tiles += w->row_tiles * w->nb;
+    return tiles >= kFusedTiles;
 }
 
 static void prompt_release_rows(JunoPrompt &P) {
@@ -1025,8 +1014,9 @@ static int prompt_reserve(juno_model *m, int n) {
 }
 
 // Layers of one pass of n consecutive positions of one sequence.  On return the residual stream is x[cur] + proj.
-// The next product's weights are turned into FP16 rows while this product runs: two buffers take turns.
-static int enqueue_layers_prompt(juno_model *m, int n, int pos0, bool guard, int &cur, cudaStream_t st) {
+// fused: the products unpack the quantised tiles themselves.  Otherwise the next product's weights are turned into FP16 rows while this
+// product runs: two buffers take turns.
+static int enqueue_layers_prompt(juno_model *m, int n, int pos0, bool fused, bool guard, int &cur, cudaStream_t st) {
     juno_ctx *c = m->ctx;
     const juno_model_cfg &f = m->cfg;
     JunoPrompt &P = m->prompt;
@@ -1043,6 +1033,7 @@ static int enqueue_layers_prompt(juno_model *m, int n, int pos0, bool guard, int
         a.K = K;
         a.out = P.img;
         a.scale = P.scale;
+        a.quant_order = fused;
         return launch_stage_rows(c, a, st);
     };
     // product k of the pass: q|k|v, W_o, gate|up, W_down of layer k / 4
@@ -1067,6 +1058,11 @@ static int enqueue_layers_prompt(juno_model *m, int n, int pos0, bool guard, int
     auto product = [&](int epi, float *out, int ldo) -> int {
         juno_qmat *const *mats;
         const int count = matrices(k, &mats);
+        if (fused) {
+            float *outs[3] = {out, out + mats[0]->rows, out + mats[0]->rows + (count > 1 ? mats[1]->rows : 0)};
+            k++;
+            return quant_group(m, mats, outs, count, epi == GE_SILU_ROW ? EPI_SILU_PAIR : EPI_STORE, n, P.img, P.scale, ldo, st, true);
+        }
         GemmArgs a;
         a.K = (int)mats[0]->cols;
         for (int i = 0; i < count; i++) a.N += (int)mats[i]->rows;
@@ -1083,7 +1079,7 @@ static int enqueue_layers_prompt(juno_model *m, int n, int pos0, bool guard, int
         JUNO_TRY(launch_gemm_rows(c, DT_BF16, a, c->gemv_scratch.qerr, st));
         return ++k < 4 * f.n_layers ? rows_of(k) : JUNO_OK;
     };
-    JUNO_TRY(rows_of(0));
+    if (!fused) JUNO_TRY(rows_of(0));
     cur = 0;
     for (int l = 0; l < f.n_layers; l++) {
         JunoLayer &L = m->layers[l];
@@ -1170,25 +1166,17 @@ static int prompt_logits(juno_model *m, const std::pair<int, int> *rows, int cou
         a.ld_out = m->vocab_loc;
         return q_group(m, lm, lo, 1, a, st);
     }
-    StageArgs s;
-    s.mode = STAGE_RMSNORM;
+    StageRowsArgs s;
     s.x = m->x[0];
-    s.ldx = H;
     s.normw = m->output_norm;
     s.eps = m->cfg.rms_eps;
+    s.n = count;
     s.K = H;
-    s.batch = count;
-    s.img = m->img_h;
-    JUNO_TRY(launch_stage_f16(c, s, m->xsc, st, m->img_h_tc));
-    GemvArgs a;
-    a.batch = count;
-    a.ximg = m->img_h;
-    a.xscale = m->xsc;
-    a.ximg_tc = m->img_h_tc;
-    a.tc_err = m->tc_err;
-    a.ld_out = m->vocab_loc;
-    m->tc_used = true;
-    return gemv_group(m, lm, lo, 1, a, st);
+    s.out = m->img_h;
+    s.scale = m->xsc;
+    s.quant_order = true;
+    JUNO_TRY(launch_stage_rows(c, s, st));
+    return quant_group(m, lm, lo, 1, EPI_STORE, count, m->img_h, m->xsc, m->vocab_loc, st);
 }
 
 // ───────────────────────────── decode step on the integer-MMA GEMV (1..8 sequences) ───────
@@ -1581,15 +1569,6 @@ static int step_sync(juno_model *m) {
 
 // After the step has drained: did one of its kernels give up on a wait?
 static int step_check(juno_model *m) {
-    if (m->tc_err && m->tc_used) {
-        m->tc_used = false;
-        unsigned code = 0;
-        if (cudaMemcpy(&code, m->tc_err, 4, cudaMemcpyDeviceToHost) == cudaSuccess && code) {
-            cudaMemset(m->tc_err, 0, 4);
-            set_error("batched tensor-core product gave up waiting (code %u, block %u)", code & 0xffu, code >> 8);
-            return JUNO_ERR_CUDA;
-        }
-    }
     const int rc = wait_status(m->ctx, WAIT_BLOCKING);
     if (rc != JUNO_OK && m->tp_failed) cudaMemset(m->tp_failed, 0, 4);
     return rc;
@@ -1659,6 +1638,7 @@ static int prefill_run(juno_model *m, juno_seq *seq, const int32_t *token_ids, i
     const int32_t *marked = nullptr;
     // without memory for the workspace of the many-row path the portion goes through the smaller passes
     const int prompt_rows = prompt_takes(m, n_tokens) && prompt_reserve(m, n_tokens) == JUNO_OK ? m->prompt.rows : 0;
+    const bool fused = prompt_fused(m, n_tokens);
     for (int done = 0; done < n_tokens;) {
         const bool many = prompt_rows > 0 && prompt_takes(m, n_tokens - done);
         const int n = std::min(many ? prompt_rows : chunk_max, n_tokens - done), pos0 = start_pos + done;
@@ -1700,7 +1680,7 @@ static int prefill_run(juno_model *m, juno_seq *seq, const int32_t *token_ids, i
             JUNO_TRY(launch_embed(m, n, d_tok, d_pos, many ? m->prompt.x[0] : m->x[0], many ? m->prompt.cs : m->rope_cs, st));
             int cur = 0;
             if (many)
-                JUNO_TRY(enqueue_layers_prompt(m, n, pos0, guard, cur, st));
+                JUNO_TRY(enqueue_layers_prompt(m, n, pos0, fused, guard, cur, st));
             else
                 JUNO_TRY(enqueue_layers_batched(m, n, d_slot, d_len, n_splits, cur, st, d_pos, !rows.empty()));
             m->last_x = cur;

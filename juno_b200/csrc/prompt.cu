@@ -3,8 +3,8 @@
 // A pass takes up to some thousand positions, so a product is bound by the tensor cores and a weight is met by every row of the
 // pass: the quantised tiles are turned into FP16 rows once per pass and matrix (one read of the blocks, one write of 2 bytes a
 // weight) and the product itself is the one of the dense layers (gemm_rows_tc.cu).  Measured on whole prompts against passes of
-// 64 positions through the batched kernels (gemm.cu, gemm_tc.cu, decode attention), which read every block 32 times: Llama-3-8B
-// Q4_K_M, 2048 positions 368.9 -> 41.9 ms; TinyLlama Q8_0, 333 positions 22.8 -> 3.51 ms.
+// 64 positions through the batched products and the decode attention, which read every block 32 times: Llama-3-8B Q4_K_M, 2048 positions
+// 368.9 -> 41.9 ms.  Portions of up to 512 positions leave the tiles to the product (gemm_quant_tc.cu).
 #include <cuda_fp16.h>
 
 #include <algorithm>
@@ -182,8 +182,99 @@ int launch_dequant_rows(juno_ctx *c, const DequantSeg *seg, int nseg, int K, voi
 }
 
 // ───────────────────────────── activations ────────────────────────────────────────────────
-constexpr int kStageThreads = 256;
-__global__ void __launch_bounds__(kStageThreads) stage_rows_kernel(const StageRowsArgs a) {
+__device__ __forceinline__ void put_staged(const StageRowsArgs &a, __half *out, int i, const float4 &v, float down) {
+    const float4 h = make_float4(v.x * down, v.y * down, v.z * down, v.w * down);
+    if (a.quant_order)
+        *reinterpret_cast<uint2 *>(out + i) = make_uint2(pack_f16(h.x, h.z), pack_f16(h.y, h.w));
+    else
+        *reinterpret_cast<uint2 *>(out + prompt_col(i)) = make_uint2(pack_f16(h.x, h.y), pack_f16(h.z, h.w));
+}
+
+// One CTA per row.  The row stays in registers between the pass that finds its norm and its largest magnitude and the pass that writes
+// it: read once, written once, bound by memory for many rows and by one round trip for a few.  V: groups of four columns per thread.
+constexpr int kStageThreads = 512, kStageCols = kStageThreads * 4;
+template <int V>
+__global__ void __launch_bounds__(kStageThreads, V <= 4 ? 3 : 2) stage_rows_kernel(const StageRowsArgs a) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, K = a.K;
+    const size_t row = blockIdx.x;
+    constexpr int kWarps = kStageThreads / 32;
+    __shared__ float red[kWarps], redm[kWarps];
+    float4 v[V];
+    pdl_wait();
+    pdl_launch_dependents();
+    const float *x = a.x + row * K, *add = a.add ? a.add + row * K : nullptr;
+#pragma unroll
+    for (int k = 0; k < V; k++) {
+        const int i = k * kStageCols + tid * 4;
+        v[k] = i < K ? *reinterpret_cast<const float4 *>(x + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    if (add) {
+#pragma unroll
+        for (int k = 0; k < V; k++) {
+            const int i = k * kStageCols + tid * 4;
+            if (i >= K) break;
+            const float4 b = *reinterpret_cast<const float4 *>(add + i);
+            v[k] = make_float4(__fadd_rn(v[k].x, b.x), __fadd_rn(v[k].y, b.y), __fadd_rn(v[k].z, b.z), __fadd_rn(v[k].w, b.w));
+        }
+    }
+    if (a.x_out) {
+#pragma unroll
+        for (int k = 0; k < V; k++) {
+            const int i = k * kStageCols + tid * 4;
+            if (i < K) *reinterpret_cast<float4 *>(a.x_out + row * K + i) = v[k];
+        }
+    }
+    float ss = 0.f, vmax = 0.f;
+#pragma unroll
+    for (int k = 0; k < V; k++) {
+        const int i = k * kStageCols + tid * 4;
+        if (i >= K) break;
+        if (a.normw) {
+            ss = fmaf(v[k].x, v[k].x, fmaf(v[k].y, v[k].y, fmaf(v[k].z, v[k].z, fmaf(v[k].w, v[k].w, ss))));
+            const float4 w = *reinterpret_cast<const float4 *>(a.normw + i);
+            v[k] = make_float4(__fmul_rn(w.x, v[k].x), __fmul_rn(w.y, v[k].y), __fmul_rn(w.z, v[k].z), __fmul_rn(w.w, v[k].w));
+        }
+        vmax = fmaxf(fmaxf(fmaxf(fabsf(v[k].x), fabsf(v[k].y)), fmaxf(fabsf(v[k].z), fabsf(v[k].w))), vmax);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        vmax = fmaxf(vmax, __shfl_xor_sync(0xffffffffu, vmax, o));
+    }
+    if (lane == 0) {
+        red[warp] = ss;
+        redm[warp] = vmax;
+    }
+    __syncthreads();
+    ss = 0.f;
+#pragma unroll
+    for (int w = 0; w < kWarps; w++) {
+        ss += red[w];
+        vmax = fmaxf(vmax, redm[w]);
+    }
+    const float inv = a.normw ? __fdiv_rn(1.f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, (float)K), a.eps))) : 1.f;
+    vmax *= inv;
+    // power of two that brings vmax into [256, 512) (1 for an all-zero or non-finite row)
+    float down = 1.f, up = 1.f;
+    if (vmax > 0.f && vmax < 3.0e38f) {
+        int e;
+        frexpf(vmax, &e);
+        down = ldexpf(1.f, 9 - e);
+        up = ldexpf(1.f, e - 9);
+    }
+    if (tid == 0) a.scale[row] = up;
+    __half *out = static_cast<__half *>(a.out) + row * K;
+#pragma unroll
+    for (int k = 0; k < V; k++) {
+        const int i = k * kStageCols + tid * 4;
+        if (i >= K) break;
+        if (a.normw) v[k] = make_float4(__fmul_rn(v[k].x, inv), __fmul_rn(v[k].y, inv), __fmul_rn(v[k].z, inv), __fmul_rn(v[k].w, inv));
+        put_staged(a, out, i, v[k], down);
+    }
+}
+
+// Rows that do not fit the registers are read twice.
+__global__ void __launch_bounds__(256) stage_wide_rows_kernel(const StageRowsArgs a) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, K = a.K;
     const size_t row = blockIdx.x;
     __shared__ float red[8], redm[8];
@@ -192,7 +283,7 @@ __global__ void __launch_bounds__(kStageThreads) stage_rows_kernel(const StageRo
     const float *x = a.x + row * K, *add = a.add ? a.add + row * K : nullptr;
     float *xo = a.x_out ? a.x_out + row * K : nullptr;
     float ss = 0.f, vmax = 0.f;
-    for (int i = tid * 4; i < K; i += kStageThreads * 4) {
+    for (int i = tid * 4; i < K; i += 256 * 4) {
         float4 v = *reinterpret_cast<const float4 *>(x + i);
         if (add) {
             const float4 b = *reinterpret_cast<const float4 *>(add + i);
@@ -218,7 +309,7 @@ __global__ void __launch_bounds__(kStageThreads) stage_rows_kernel(const StageRo
     __syncthreads();
     ss = 0.f;
 #pragma unroll
-    for (int w = 0; w < kStageThreads / 32; w++) {
+    for (int w = 0; w < 8; w++) {
         ss += red[w];
         vmax = fmaxf(vmax, redm[w]);
     }
@@ -235,7 +326,7 @@ __global__ void __launch_bounds__(kStageThreads) stage_rows_kernel(const StageRo
     if (tid == 0) a.scale[row] = up;
     __half *out = static_cast<__half *>(a.out) + row * K;
     const float *src = xo ? xo : x;  // this thread's own stores
-    for (int i = tid * 4; i < K; i += kStageThreads * 4) {
+    for (int i = tid * 4; i < K; i += 256 * 4) {
         float4 v = *reinterpret_cast<const float4 *>(src + i);
         if (add && !xo) {
             const float4 b = *reinterpret_cast<const float4 *>(add + i);
@@ -246,14 +337,20 @@ __global__ void __launch_bounds__(kStageThreads) stage_rows_kernel(const StageRo
             v = make_float4(__fmul_rn(__fmul_rn(w.x, v.x), inv), __fmul_rn(__fmul_rn(w.y, v.y), inv), __fmul_rn(__fmul_rn(w.z, v.z), inv),
                             __fmul_rn(__fmul_rn(w.w, v.w), inv));
         }
-        *reinterpret_cast<uint2 *>(out + prompt_col(i)) = make_uint2(pack_f16(v.x * down, v.y * down), pack_f16(v.z * down, v.w * down));
+        put_staged(a, out, i, v, down);
     }
 }
 
 int launch_stage_rows(juno_ctx *c, const StageRowsArgs &a, cudaStream_t st) {
     JUNO_REQUIRE(a.n > 0 && a.K > 0 && a.K % 32 == 0 && a.x && a.out && a.scale, "stage rows: bad arguments (K=%d, n=%d)", a.K, a.n);
     ProfScope prof(c, st, PROF_OTHER, (double)a.n * a.K * 6);
-    JUNO_CUDA_TRY(launch_pdl(stage_rows_kernel, dim3((unsigned)a.n), dim3(kStageThreads), 0, st, a));
+    void (*const kernels[])(const StageRowsArgs) = {stage_rows_kernel<1>, stage_rows_kernel<2>, stage_rows_kernel<4>, stage_rows_kernel<8>, stage_rows_kernel<16>};
+    int k = 0;
+    while (k < 5 && (1 << k) * kStageCols < a.K) k++;
+    if (k < 5)
+        JUNO_CUDA_TRY(launch_pdl(kernels[k], dim3((unsigned)a.n), dim3(kStageThreads), 0, st, a));
+    else
+        JUNO_CUDA_TRY(launch_pdl(stage_wide_rows_kernel, dim3((unsigned)a.n), dim3(256), 0, st, a));
     c->kernel_launches++;
     return JUNO_OK;
 }

@@ -34,6 +34,7 @@ struct StageRowsArgs {
     int n = 0, K = 0;
     void *out = nullptr;
     float *scale = nullptr;
+    bool quant_order = false;  // columns as quant_col has them (gemm_quant.cuh), else as prompt_col
 };
 int launch_stage_rows(juno_ctx *c, const StageRowsArgs &a, cudaStream_t st);
 

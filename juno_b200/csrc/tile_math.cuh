@@ -1,5 +1,4 @@
-// Register image of one 16x256 weight tile (layout.cuh) and small helpers, shared by the batched dequant-GEMM
-// kernels (gemm.cu, gemm_tc.cu).
+// Register image of one 16x256 weight tile (layout.cuh) and small helpers of the kernels that turn tiles into FP16.
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -93,14 +92,6 @@ __device__ __forceinline__ void load_tile<8>(TileRegs<8> &r, const uint8_t *tile
 }
 
 
-// Nibbles of one word as four register pairs: (w & mask) | magic in one instruction each.
-__device__ __forceinline__ void q4_unpack(uint32_t w, uint32_t M, uint32_t K, uint32_t &lo_a, uint32_t &lo_b,
-                                          uint32_t &hi_a, uint32_t &hi_b) {
-    lo_a = and_or(w, M, K);        // (byte0.lo, byte2.lo)
-    hi_a = and_or(w >> 4, M, K);   // (byte0.hi, byte2.hi)
-    lo_b = and_or(w >> 8, M, K);   // (byte1.lo, byte3.lo)
-    hi_b = and_or(w >> 12, M, K);  // (byte1.hi, byte3.hi)
-}
 __device__ __forceinline__ float i8_to_f32(uint32_t w, int k) { return (float)(int)(signed char)((w >> (8 * k)) & 0xFFu); }
 
 }  // namespace juno

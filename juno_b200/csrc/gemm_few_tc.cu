@@ -135,21 +135,27 @@ __global__ void __launch_bounds__(kFewThreads, 2) gemm_few_kernel(const __grid_c
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            // D FP32, A and B BF16, both K-major
-            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(p.cols >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
-            bool ok = true;
-            for (int k = 0; k < steps; k++) {
-                const int s = k % S;
-                if (!(ok = bar_wait(full0 + 8 * s, (unsigned)(k / S) & 1u, fail))) break;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint64_t wd = sw128_desc(stage0 + s * stage_bytes), ad = sw128_desc(stage0 + s * stage_bytes + w_bytes);
+        // D FP32, A and B BF16, both K-major
+        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(p.cols >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
+        const bool leader = elect_one();
+        bool ok = true;
+        for (int k = 0, s = 0, par = 0; k < steps; k++) {
+            ok = bar_wait(full0 + 8 * s, (unsigned)par, fail) && ok;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint64_t wd = sw128_desc(stage0 + s * stage_bytes), ad = sw128_desc(stage0 + s * stage_bytes + w_bytes);
+            if (leader && ok) {
 #pragma unroll
                 for (int j = 0; j < kBK / 16; j++) mma_bf16(tmem, wd + 2 * j, ad + 2 * j, idesc, (k > 0 || j > 0) ? 1u : 0u);
                 mma_commit(empty0 + 8 * s);
             }
-            if (ok) mma_commit(ready);
+            __syncwarp();
+            if (++s == S) {
+                s = 0;
+                par ^= 1;
+            }
         }
+        if (leader && ok) mma_commit(ready);
+        __syncwarp();
     } else {
         const int quad = warp & 3;  // TMEM lanes a warp can read: 32 * (warp % 4) ..
         int ok = 0;

@@ -108,26 +108,34 @@ __global__ void __launch_bounds__(kPairThreads, 1) gemm_pair_kernel(const __grid
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {
             // D FP32, A and B BF16 or both FP16, both K-major, M 256
             const uint32_t idesc = (1u << 4) | (g.half ? 0u : (1u << 7) | (1u << 10)) | ((uint32_t)(kPairN >> 3) << 17) | ((uint32_t)(2 * kBM >> 4) << 24);
-            unsigned it = 0, tile = 0;
+            const bool leader = elect_one();
+            unsigned s = 0, par = 0, tile = 0;
             bool ok = true;
-            for (int work = pair; ok && work < p.n_work; work += pairs, tile++) {
+            for (int work = pair; work < p.n_work; work += pairs, tile++) {
                 const unsigned acc = tile & 1u;
-                if (!(ok = bar_wait(acce0 + 8 * acc, ((tile >> 1) & 1u) ^ 1u, fail))) break;
+                ok = bar_wait(acce0 + 8 * acc, ((tile >> 1) & 1u) ^ 1u, fail) && ok;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t d = tmem + acc * kPairN;
-                for (int k = 0; k < p.k_steps; k++, it++) {
-                    const unsigned s = it % kPairStages, use = it / kPairStages;
-                    if (!(ok = bar_wait(full0 + 8 * s, use & 1u, fail))) break;
+                for (int k = 0; k < p.k_steps; k++) {
+                    ok = bar_wait(full0 + 8 * s, par, fail) && ok;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint64_t ad = sw128_desc(stage0 + s * kPairStageBytes), bd = sw128_desc(stage0 + s * kPairStageBytes + kPairHalf);
+                    if (leader && ok) {
 #pragma unroll
-                    for (int j = 0; j < kBK / 16; j++) pair_mma(d, ad + 2 * j, bd + 2 * j, idesc, (k > 0 || j > 0) ? 1u : 0u);
-                    pair_commit(empty0 + 8 * s);
+                        for (int j = 0; j < kBK / 16; j++) pair_mma(d, ad + 2 * j, bd + 2 * j, idesc, (k > 0 || j > 0) ? 1u : 0u);
+                        pair_commit(empty0 + 8 * s);
+                    }
+                    __syncwarp();
+                    if (++s == kPairStages) {
+                        s = 0;
+                        par ^= 1u;
+                    }
                 }
-                if (ok) pair_commit(accf0 + 8 * acc);
+                if (leader && ok) pair_commit(accf0 + 8 * acc);
+                __syncwarp();
             }
         }
     } else {
@@ -223,19 +231,27 @@ __global__ void __launch_bounds__(kPairThreads, 1) gemm_pair_split_kernel(const 
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {
             const uint32_t idesc = (1u << 4) | (g.half ? 0u : (1u << 7) | (1u << 10)) | ((uint32_t)(kPairN >> 3) << 17) | ((uint32_t)(2 * kBM >> 4) << 24);
+            const bool leader = elect_one();
             bool good = true;
-            for (int k = 0; k < steps; k++) {
-                const int s = k % kPairStages;
-                if (!(good = bar_wait(full0 + 8 * s, (unsigned)(k / kPairStages) & 1u, fail))) break;
+            for (int k = 0, s = 0, par = 0; k < steps; k++) {
+                good = bar_wait(full0 + 8 * s, (unsigned)par, fail) && good;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint64_t ad = sw128_desc(stage0 + s * kPairStageBytes), bd = sw128_desc(stage0 + s * kPairStageBytes + kPairHalf);
+                if (leader && good) {
 #pragma unroll
-                for (int j = 0; j < kBK / 16; j++) pair_mma(tmem, ad + 2 * j, bd + 2 * j, idesc, (k > 0 || j > 0) ? 1u : 0u);
-                pair_commit(empty0 + 8 * s, q);
+                    for (int j = 0; j < kBK / 16; j++) pair_mma(tmem, ad + 2 * j, bd + 2 * j, idesc, (k > 0 || j > 0) ? 1u : 0u);
+                    pair_commit(empty0 + 8 * s, q);
+                }
+                __syncwarp();
+                if (++s == kPairStages) {
+                    s = 0;
+                    par ^= 1;
+                }
             }
-            if (good) pair_commit(ready, q);
+            if (leader && good) pair_commit(ready, q);
+            __syncwarp();
         }
     } else {
         if (lane == 0) ok = bar_wait(ready, 0u, fail) ? 1 : 0;

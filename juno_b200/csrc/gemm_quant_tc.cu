@@ -117,11 +117,6 @@ __device__ __forceinline__ float4 qt_peer_sum(uint32_t addr, int splits) {
     }
     return v;
 }
-__device__ __forceinline__ bool elect_one() {
-    uint32_t ok;
-    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(ok));
-    return ok != 0;
-}
 __device__ __forceinline__ void qt_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
 
 // The next tile of an unpacking warp, in the hands of a lane of the copying warp.
@@ -348,8 +343,6 @@ __global__ void __launch_bounds__((kQtWarps + 4) * 32, 2) gemm_quant_kernel(cons
         }
         __syncwarp();
     } else if (warp == kQtWarps + 1) {
-        // The whole warp walks and waits, one lane issues: operands of the MMAs stay in uniform registers (with the loop in one lane's
-        // branch eight of them took 830 cycles to issue).
         // D FP32, A and B FP16, M 128; A from the tensor memory, B K-major
         const uint32_t idesc = (1u << 4) | ((uint32_t)(p.N >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
         const bool leader = elect_one();

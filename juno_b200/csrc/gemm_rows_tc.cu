@@ -88,27 +88,33 @@ __global__ void __launch_bounds__(kTileThreads, 1) gemm_rows_tc_kernel(const __g
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            // D FP32, A and B BF16 or both FP16, both K-major
-            const uint32_t idesc = (1u << 4) | (g.half ? 0u : (1u << 7) | (1u << 10)) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
-            unsigned it = 0, tile = 0;
-            bool ok = true;
-            for (int work = blockIdx.x; ok && work < p.n_work; work += gridDim.x, tile++) {
-                const unsigned acc = tile & 1u;
-                if (!(ok = bar_wait(acce0 + 8 * acc, ((tile >> 1) & 1u) ^ 1u, fail))) break;
+        // D FP32, A and B BF16 or both FP16, both K-major
+        const uint32_t idesc = (1u << 4) | (g.half ? 0u : (1u << 7) | (1u << 10)) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
+        const bool leader = elect_one();
+        unsigned s = 0, par = 0, tile = 0;
+        bool ok = true;
+        for (int work = blockIdx.x; work < p.n_work; work += gridDim.x, tile++) {
+            const unsigned acc = tile & 1u;
+            ok = bar_wait(acce0 + 8 * acc, ((tile >> 1) & 1u) ^ 1u, fail) && ok;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t d = tmem + acc * BN;
+            for (int k = 0; k < p.k_steps; k++) {
+                ok = bar_wait(full0 + 8 * s, par, fail) && ok;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t d = tmem + acc * BN;
-                for (int k = 0; k < p.k_steps; k++, it++) {
-                    const unsigned s = it % S, use = it / S;
-                    if (!(ok = bar_wait(full0 + 8 * s, use & 1u, fail))) break;
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint64_t ad = sw128_desc(stage0 + s * kStageBytes), bd = sw128_desc(stage0 + s * kStageBytes + kABytes);
+                const uint64_t ad = sw128_desc(stage0 + s * kStageBytes), bd = sw128_desc(stage0 + s * kStageBytes + kABytes);
+                if (leader && ok) {
 #pragma unroll
                     for (int j = 0; j < kBK / 16; j++) mma_bf16(d, ad + 2 * j, bd + 2 * j, idesc, (k > 0 || j > 0) ? 1u : 0u);
                     mma_commit(empty0 + 8 * s);
                 }
-                if (ok) mma_commit(accf0 + 8 * acc);
+                __syncwarp();
+                if (++s == S) {
+                    s = 0;
+                    par ^= 1u;
+                }
             }
+            if (leader && ok) mma_commit(accf0 + 8 * acc);
+            __syncwarp();
         }
     } else {
         const int quad = warp & 3;  // TMEM lanes a warp can read: 32 * (warp % 4) ..

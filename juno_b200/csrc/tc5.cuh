@@ -52,6 +52,14 @@ __device__ __forceinline__ void mma_bf16(uint32_t d, uint64_t a, uint64_t b, uin
         "l"(a), "l"(b), "r"(idesc), "r"(acc)
         : "memory");
 }
+// One lane of a converged warp.  A warp that issues MMAs walks and waits as a whole and issues from this lane: addresses and descriptors stay
+// in uniform registers then.  From a lane's own branch four MMAs and their commit took 415 cycles to issue, more than tiles of up to 128 columns take
+// to multiply.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t ok;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(ok));
+    return ok != 0;
+}
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }

@@ -66,6 +66,8 @@ __global__ void __launch_bounds__(kPairThreads, 1) gemm_pair_kernel(const __grid
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rank = (int)(blockIdx.x & 1u), pair = (int)(blockIdx.x >> 1), pairs = (int)(gridDim.x >> 1);
     const uint32_t full0 = s_u32(bars), empty0 = full0 + 8 * kPairStages, accf0 = empty0 + 8 * kPairStages, acce0 = accf0 + 16;
     if (threadIdx.x == 0) {
+        prefetch_map(&p.tw);
+        prefetch_map(&p.ta);
         for (int s = 0; s < kPairStages; s++) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(full0 + 8 * s) : "memory");
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(empty0 + 8 * s) : "memory");
@@ -92,18 +94,23 @@ __global__ void __launch_bounds__(kPairThreads, 1) gemm_pair_kernel(const __grid
     pdl_launch_dependents();  // not before the wait: dequant_rows_kernel (prompt.cu) may be next and write what the product before this one read
 
     if (warp == 0) {
-        if (lane == 0) {
-            unsigned it = 0;
-            bool ok = true;
-            for (int work = pair; ok && work < p.n_work; work += pairs) {
-                const int mt = work % p.m_tiles, nt = work / p.m_tiles;
-                for (int k = 0; k < p.k_steps; k++, it++) {
-                    const unsigned s = it % kPairStages, use = it / kPairStages;
-                    if (!(ok = bar_wait(empty0 + 8 * s, (use & 1u) ^ 1u, fail))) break;
+        const bool leader = elect_one();
+        unsigned s = 0, par = 0;
+        bool ok = true;
+        for (int work = pair; work < p.n_work; work += pairs) {
+            const int mt = work % p.m_tiles, nt = work / p.m_tiles;
+            for (int k = 0; k < p.k_steps; k++) {
+                ok = bar_wait(empty0 + 8 * s, par ^ 1u, fail) && ok;
+                if (leader && ok) {
                     if (rank == 0) asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full0 + 8 * s), "r"(2 * kPairStageBytes) : "memory");
                     const uint32_t bar = in_cta(full0 + 8 * s, 0), a_s = stage0 + s * kPairStageBytes;
                     pair_tma(a_s, &p.ta, k * kBK, mt * 2 * kBM + rank * kBM, bar);
                     pair_tma(a_s + kPairHalf, &p.tw, k * kBK, nt * kPairN + rank * kBM, bar);
+                }
+                __syncwarp();
+                if (++s == kPairStages) {
+                    s = 0;
+                    par ^= 1u;
                 }
             }
         }
@@ -194,6 +201,8 @@ __global__ void __launch_bounds__(kPairThreads, 1) gemm_pair_split_kernel(const 
     const int k0 = p.k_steps * q / p.splits, steps = p.k_steps * (q + 1) / p.splits - k0;
     const uint32_t full0 = s_u32(bars), empty0 = full0 + 8 * kPairStages, ready = empty0 + 8 * kPairStages;
     if (threadIdx.x == 0) {
+        prefetch_map(&p.tw);
+        prefetch_map(&p.ta);
         for (int s = 0; s < kPairStages; s++) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(full0 + 8 * s) : "memory");
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(empty0 + 8 * s) : "memory");
@@ -220,14 +229,20 @@ __global__ void __launch_bounds__(kPairThreads, 1) gemm_pair_split_kernel(const 
     const uint32_t acc = tmem + ((uint32_t)(quad * 32) << 16), mine = stage0 + (uint32_t)(quad * 32 + lane) * 4;  // partial sums: [column][row]
     const int share = kPairN / p.splits;
     if (warp == 0) {
-        if (lane == 0) {
-            for (int k = 0; k < steps; k++) {
-                const int s = k % kPairStages, use = k / kPairStages;
-                if (use > 0 && !bar_wait(empty0 + 8 * s, (unsigned)(use - 1) & 1u, fail)) break;
+        const bool leader = elect_one();
+        bool good = true;
+        for (int k = 0, s = 0, par = 0; k < steps; k++) {
+            good = bar_wait(empty0 + 8 * s, (unsigned)par ^ 1u, fail) && good;
+            if (leader && good) {
                 if (rank == 0) asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full0 + 8 * s), "r"(2 * kPairStageBytes) : "memory");
                 const uint32_t bar = in_cta(full0 + 8 * s, 2 * q), a_s = stage0 + s * kPairStageBytes;
                 pair_tma(a_s, &p.ta, (k0 + k) * kBK, mt * 2 * kBM + rank * kBM, bar);
                 pair_tma(a_s + kPairHalf, &p.tw, (k0 + k) * kBK, nt * kPairN + rank * kBM, bar);
+            }
+            __syncwarp();
+            if (++s == kPairStages) {
+                s = 0;
+                par ^= 1;
             }
         }
     } else if (warp == 1) {

@@ -235,7 +235,7 @@ __global__ void __launch_bounds__((kQtWarps + 4) * 32, 2) gemm_quant_kernel(cons
         __syncwarp();
     } else if (warp == kQtWarps) {
         if (lane == 0) {
-            asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&p.tx)) : "memory");
+            prefetch_map(&p.tx);
             for (int i = 0; i < p.stages; i++) {
                 mbar_init(full + i * 8, kQtWarps + 1);
                 mbar_init(free + i * 8, 1);

@@ -40,6 +40,8 @@ __global__ void __launch_bounds__(kTileThreads, 1) gemm_rows_tc_kernel(const __g
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, S = p.stages;
     const uint32_t full0 = s_u32(bars), empty0 = full0 + 8 * kMaxStages, accf0 = empty0 + 8 * kMaxStages, acce0 = accf0 + 16;
     if (threadIdx.x == 0) {
+        prefetch_map(&p.tw);
+        prefetch_map(&p.ta);
         for (int s = 0; s < S; s++) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(full0 + 8 * s) : "memory");
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(empty0 + 8 * s) : "memory");
@@ -65,28 +67,36 @@ __global__ void __launch_bounds__(kTileThreads, 1) gemm_rows_tc_kernel(const __g
     pdl_launch_dependents();  // not before the wait: dequant_rows_kernel (prompt.cu) may be next and write what the product before this one read
 
     if (warp == 0) {
-        if (lane == 0) {
-            unsigned it = 0;
-            bool ok = true;
-            for (int work = blockIdx.x; ok && work < p.n_work; work += gridDim.x) {
-                const int mt = work % p.m_tiles, t = work / p.m_tiles, nt = t % p.n_tiles, z = t / p.n_tiles;
-                for (int k = 0; k < p.k_steps; k++, it++) {
-                    const unsigned s = it % S, use = it / S;
-                    if (!(ok = bar_wait(empty0 + 8 * s, (use & 1u) ^ 1u, fail))) break;
+        const bool leader = elect_one();
+        unsigned s = 0, par = 0, it = 0;  // it: stages that were filled
+        bool ok = true;
+        for (int work = blockIdx.x; work < p.n_work; work += gridDim.x) {
+            const int mt = work % p.m_tiles, t = work / p.m_tiles, nt = t % p.n_tiles, z = t / p.n_tiles;
+            for (int k = 0; k < p.k_steps; k++) {
+                ok = bar_wait(empty0 + 8 * s, par ^ 1u, fail) && ok;
+                if (leader && ok) {
                     const uint32_t bar = full0 + 8 * s, a_s = stage0 + s * kStageBytes;
                     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(kStageBytes) : "memory");
                     tma_2d(a_s, &p.ta, z * g.a_step + k * kBK, mt * kBM, bar);
                     tma_2d(a_s + kABytes, &p.tw, k * kBK, z * g.w_step + nt * BN, bar);
+                    it++;
                 }
-            }
-            // the last copies of every stage: nothing may be in flight when the CTA leaves
-            for (int b = 0; b < S && b < (int)it; b++) {
-                const unsigned j = it - 1 - b, s = j % S;
-                const long long t0 = clock64();
-                while (!bar_test(full0 + 8 * s, (j / S) & 1u) && clock64() - t0 < kWaitClocks) {
+                __syncwarp();
+                if (++s == S) {
+                    s = 0;
+                    par ^= 1u;
                 }
             }
         }
+        // the last copies of every stage: nothing may be in flight when the CTA leaves
+        if (leader)
+            for (int b = 0; b < S && b < (int)it; b++) {
+                const unsigned j = it - 1 - b, last = j % S;
+                const long long t0 = clock64();
+                while (!bar_test(full0 + 8 * last, (j / S) & 1u) && clock64() - t0 < kWaitClocks) {
+                }
+            }
+        __syncwarp();
     } else if (warp == 1) {
         // D FP32, A and B BF16 or both FP16, both K-major
         const uint32_t idesc = (1u << 4) | (g.half ? 0u : (1u << 7) | (1u << 10)) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);

@@ -40,6 +40,7 @@ __device__ __forceinline__ void tma_2d(uint32_t dst, const CUtensorMap *map, int
                  "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar)
                  : "memory");
 }
+__device__ __forceinline__ void prefetch_map(const CUtensorMap *map) { asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory"); }
 // K-major operand with 128-byte swizzle: rows of 128 bytes, groups of eight rows 1024 bytes apart.
 __device__ __forceinline__ uint64_t sw128_desc(uint32_t saddr) {
     return (uint64_t)((saddr >> 4) & 0x3FFFu) | (uint64_t)1 << 16 | (uint64_t)(1024 >> 4) << 32 | (uint64_t)1 << 46 | (uint64_t)2 << 61;

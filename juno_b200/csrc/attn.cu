@@ -33,6 +33,7 @@ struct AttnParams {
     // the context splits of a (sequence, kv head) form one thread-block cluster (cluster dimension y = n_splits): the
     // splits are merged through distributed shared memory inside attn_mma_kernel and no merge kernel is launched
     int cluster_merge;
+    int wide;  // FP16 pages, one split: eight warps per CTA
 };
 
 template <typename T>
@@ -227,8 +228,15 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attn_split_kernel(const AttnP
 //   S = Q K^T   : A = q as two FP16 limbs (hi + lo, so the scores keep FP32-level accuracy), B = K via ldmatrix
 //   online softmax on the FP32 fragment (row max / sum across the four lanes that share a row)
 //   O += P V    : A = P (the score fragment re-used as an A fragment, FP16), B = V via ldmatrix.trans
-// Rows of the 16-row MMA tile are the G query heads of the group (G <= 8; rows 8..15 stay zero).
+// Rows 0..7 of the 16-row MMA tile are the high limbs of the G query heads of the group (G <= 8), rows 8..15 their low limbs: one MMA multiplies
+// both, and the two sums lie in the same lane.  (With the limbs in MMAs of their own, rows 8..15 zero, a page took twice as many.)
 constexpr int kMmaWarps = 4;
+template <int HD>
+constexpr int kMmaCtas = HD == 128 ? 3 : 4;  // CTAs on an SM: what registers and shared memory hold
+// A context that one CTA takes alone, without a merge, has eight warps for it as long as there are few such CTAs.
+constexpr int kWideWarps = 8;
+template <int HD>
+constexpr int kWideCtas = HD == 128 ? 1 : 2;
 
 __device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t addr) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
@@ -256,8 +264,8 @@ __device__ __forceinline__ uint32_t pack_h2(float a, float b) {
     return *reinterpret_cast<uint32_t *>(&h);
 }
 
-template <int HD, int G>
-__global__ void __launch_bounds__(kMmaWarps * 32, 2) attn_mma_kernel(const AttnParams p) {
+template <int HD, int G, int W>
+__global__ void __launch_bounds__(W * 32, W == kMmaWarps ? kMmaCtas<HD> : kWideCtas<HD>) attn_mma_kernel(const AttnParams p) {
     constexpr int LDT = HD + 8;             // tile row stride in halfs (the pad keeps ldmatrix rows on distinct banks)
     constexpr int TILE = 16 * LDT;          // halfs per K or V tile
     constexpr int KS = HD / 16, DN = HD / 8;
@@ -306,12 +314,12 @@ __global__ void __launch_bounds__(kMmaWarps * 32, 2) attn_mma_kernel(const AttnP
             pml[(size_t)tid * p.n_splits * 2 + 0] = -INFINITY;
             pml[(size_t)tid * p.n_splits * 2 + 1] = 0.f;
         }
-        for (int idx = tid; idx < G * HD; idx += kMmaWarps * 32) po[(size_t)(idx / HD) * p.n_splits * HD + (idx % HD)] = 0.f;
+        for (int idx = tid; idx < G * HD; idx += W * 32) po[(size_t)(idx / HD) * p.n_splits * HD + (idx % HD)] = 0.f;
         return;
     }
     // q of the group: rotate (rope :1657-1671), scale into the log2 domain, split into two FP16 limbs
     const float scale = (float)(1.0 / sqrt((double)HD)) * 1.4426950408889634f;
-    for (int idx = tid; idx < 8 * (HD / 2); idx += kMmaWarps * 32) {
+    for (int idx = tid; idx < 8 * (HD / 2); idx += W * 32) {
         const int g = idx / (HD / 2), i = idx - g * (HD / 2);
         float y0 = 0.f, y1 = 0.f;
         if (g < G) {
@@ -346,9 +354,9 @@ __global__ void __launch_bounds__(kMmaWarps * 32, 2) attn_mma_kernel(const AttnP
     float o[DN][2], m_run = -INFINITY, l_run = 0.f;  // row r8: output columns dn*8 + 2c, +1; running max; this lane's share of the sum
 #pragma unroll
     for (int dn = 0; dn < DN; dn++) o[dn][0] = o[dn][1] = 0.f;
-    for (; pg < pg1; pg += kMmaWarps, stage ^= 1) {
-        const bool more = pg + kMmaWarps < pg1;
-        if (more) issue(pg + kMmaWarps, stage ^ 1);
+    for (; pg < pg1; pg += W, stage ^= 1) {
+        const bool more = pg + W < pg1;
+        if (more) issue(pg + W, stage ^ 1);
         if (more)
             asm volatile("cp.async.wait_group 1;" ::: "memory");
         else
@@ -397,14 +405,12 @@ __global__ void __launch_bounds__(kMmaWarps * 32, 2) attn_mma_kernel(const AttnP
             for (int ks = 0; ks < KS; ks++) {
                 uint32_t b[4];  // (pos 0-7, k lo), (pos 0-7, k hi), (pos 8-15, k lo), (pos 8-15, k hi)
                 ldmatrix_x4(b, kts + (uint32_t)(rr * LDT + ks * 16 + cc) * 2u);
-                mma_f16(s0, qh[ks][0], 0u, qh[ks][1], 0u, b[0], b[1]);
-                mma_f16(s1, qh[ks][0], 0u, qh[ks][1], 0u, b[2], b[3]);
-                mma_f16(s0, ql[ks][0], 0u, ql[ks][1], 0u, b[0], b[1]);
-                mma_f16(s1, ql[ks][0], 0u, ql[ks][1], 0u, b[2], b[3]);
+                mma_f16(s0, qh[ks][0], ql[ks][0], qh[ks][1], ql[ks][1], b[0], b[1]);
+                mma_f16(s1, qh[ks][0], ql[ks][0], qh[ks][1], ql[ks][1], b[2], b[3]);
             }
         }
         // this lane holds row r8, positions pos0 + 2c, +1 (s0) and pos0 + 8 + 2c, +1 (s1)
-        float sc[4] = {s0[0], s0[1], s1[0], s1[1]};
+        float sc[4] = {s0[0] + s0[2], s0[1] + s0[3], s1[0] + s1[2], s1[1] + s1[3]};
         if (pos0 + 16 > t1) {
             if (pos0 + 2 * c >= t1) sc[0] = -INFINITY;
             if (pos0 + 2 * c + 1 >= t1) sc[1] = -INFINITY;
@@ -444,14 +450,12 @@ __global__ void __launch_bounds__(kMmaWarps * 32, 2) attn_mma_kernel(const AttnP
                 uint32_t b[4];  // (pos 0-7, dims dn), (pos 8-15, dims dn), (pos 0-7, dims dn+1), (pos 8-15, dims dn+1), transposed
                 ldmatrix_x4_trans(b, vts + (uint32_t)(rr * LDT + dn * 8 + cc) * 2u);
                 float acc0[4] = {o[dn][0], o[dn][1], 0.f, 0.f}, acc1[4] = {o[dn + 1][0], o[dn + 1][1], 0.f, 0.f};
-                mma_f16(acc0, pa0, 0u, pa2, 0u, b[0], b[1]);
-                mma_f16(acc1, pa0, 0u, pa2, 0u, b[2], b[3]);
-                mma_f16(acc0, pb0, 0u, pb2, 0u, b[0], b[1]);
-                mma_f16(acc1, pb0, 0u, pb2, 0u, b[2], b[3]);
-                o[dn][0] = acc0[0];
-                o[dn][1] = acc0[1];
-                o[dn + 1][0] = acc1[0];
-                o[dn + 1][1] = acc1[1];
+                mma_f16(acc0, pa0, pb0, pa2, pb2, b[0], b[1]);
+                mma_f16(acc1, pa0, pb0, pa2, pb2, b[2], b[3]);
+                o[dn][0] = acc0[0] + acc0[2];
+                o[dn][1] = acc0[1] + acc0[3];
+                o[dn + 1][0] = acc1[0] + acc1[2];
+                o[dn + 1][1] = acc1[1] + acc1[3];
             }
         }
         __syncwarp();  // everybody is done with this stage before it is refilled two pages later
@@ -462,9 +466,9 @@ __global__ void __launch_bounds__(kMmaWarps * 32, 2) attn_mma_kernel(const AttnP
     // merge the four warps through shared memory (the K/V tiles are dead)
     __syncthreads();
     float *mg_o = reinterpret_cast<float *>(sm_kv);       // [warp][G][HD]
-    float *mg_m = mg_o + kMmaWarps * G * HD;               // [warp][G]
-    float *mg_l = mg_m + kMmaWarps * G;                    // [warp][G]
-    float *cl_o = mg_l + kMmaWarps * G;                    // [G][HD]   this CTA's merged split, read by the cluster
+    float *mg_m = mg_o + W * G * HD;               // [warp][G]
+    float *mg_l = mg_m + W * G;                    // [warp][G]
+    float *cl_o = mg_l + W * G;                    // [G][HD]   this CTA's merged split, read by the cluster
     float *cl_m = cl_o + G * HD, *cl_l = cl_m + G;
     if (r8 < G) {
 #pragma unroll
@@ -476,14 +480,14 @@ __global__ void __launch_bounds__(kMmaWarps * 32, 2) attn_mma_kernel(const AttnP
         }
     }
     __syncthreads();
-    for (int idx = tid; idx < G * HD; idx += kMmaWarps * 32) {
+    for (int idx = tid; idx < G * HD; idx += W * 32) {
         const int g = idx / HD, d = idx - g * HD;
         float M = -INFINITY;
 #pragma unroll
-        for (int w = 0; w < kMmaWarps; w++) M = fmaxf(M, mg_m[w * G + g]);
+        for (int w = 0; w < W; w++) M = fmaxf(M, mg_m[w * G + g]);
         float L = 0.f, acc = 0.f;
 #pragma unroll
-        for (int w = 0; w < kMmaWarps; w++) {
+        for (int w = 0; w < W; w++) {
             const float lw = mg_l[w * G + g];
             if (lw > 0.f) {
                 const float f = exp2f(mg_m[w * G + g] - M);
@@ -497,6 +501,8 @@ __global__ void __launch_bounds__(kMmaWarps * 32, 2) attn_mma_kernel(const AttnP
                 cl_m[g] = M;
                 cl_l[g] = L;
             }
+        } else if (p.n_splits == 1) {  // nothing to merge with
+            p.out[(size_t)(seq * p.n_heads + h0 + g) * HD + d] = (L > 0.f) ? acc / L : 0.f;
         } else {
             po[(size_t)g * p.n_splits * HD + d] = acc;
             if (d == 0) {
@@ -515,7 +521,7 @@ __global__ void __launch_bounds__(kMmaWarps * 32, 2) attn_mma_kernel(const AttnP
     {
         const int S = (int)cluster.num_blocks(), r = (int)cluster.block_rank();
         const int per = (G * HD) / S;
-        for (int idx = r * per + tid; idx < (r + 1) * per; idx += kMmaWarps * 32) {
+        for (int idx = r * per + tid; idx < (r + 1) * per; idx += W * 32) {
             const int g = idx / HD, d = idx - g * HD;
             float M = -INFINITY;
             for (int sp = 0; sp < S; sp++) M = fmaxf(M, *cluster.map_shared_rank(cl_m + g, sp));
@@ -653,15 +659,27 @@ static int attn_cluster_max() {
     return std::max(0, std::min(m, 16));
 }
 
-int attn_pick_splits(const juno_ctx *ctx, int n, int n_kv_heads, int max_len) {
-    const int target = ctx->sm_count * 4;  // CTAs of 128 threads wanted in flight
-    int by_occupancy = (target + n * n_kv_heads - 1) / std::max(1, n * n_kv_heads);
-    // at least 128 positions per split (two pages per warp): in the batch-1 step at context 2048, 16-32 splits
-    // measured 2.27 ms/step against 2.36 ms with 64 (fewer partials to merge, same occupancy where it matters)
-    int by_length = std::max(1, (max_len + 127) / 128);
-    int s = std::max(1, std::min(by_occupancy, by_length));
+static bool attn_wide(const juno_ctx *ctx, int pairs, int hd) { return pairs <= ctx->sm_count * (hd == 128 ? kWideCtas<128> : kWideCtas<64>); }
+// How many CTAs share the context of a (sequence, kv head).  A CTA takes about three page times beside the pages of its busiest warp, CTAs
+// run in rounds of as many as the GPU holds, and more than one split cost a merge.  Every round counts in full: Llama-3-8B, six requests of
+// 512 to 1024 positions, 6 splits (one round of two CTAs per SM, which was what registers allowed) 7.9 us a layer, 8 splits (1.3 rounds) 11.9; eight requests of
+// up to 4096 positions, 4 splits 25 + 10 us, 10 splits 32 + 12.
+int attn_pick_splits(const juno_ctx *ctx, int n, int n_kv_heads, int hd, int max_len) {
+    const int pairs = std::max(1, n * n_kv_heads), slots = ctx->sm_count * (hd == 128 ? kMmaCtas<128> : kMmaCtas<64>), pages = (max_len + kPageTokens - 1) / kPageTokens;
+    // at least 128 positions per split (two pages per warp), and no more partial results than the callers have room for
+    const int most = std::min({std::max(1, (max_len + 127) / 128), (ctx->sm_count * 4 + pairs - 1) / pairs, 64});
+    int s = 1;
+    double best = 1e30;
+    for (int k = 1; k <= most; k++) {
+        const bool wide = k == 1 && attn_wide(ctx, pairs, hd);
+        const int rounds = wide ? 1 : (pairs * k + slots - 1) / slots, warps = wide ? kWideWarps : kMmaWarps, per_warp = ((pages + k - 1) / k + warps - 1) / warps;
+        const double cost = rounds * (per_warp + 3.0) + (k > 1 ? 1.5 + k / 16.0 : 0.0);
+        if (cost < best) {
+            best = cost;
+            s = k;
+        }
+    }
     if (const char *e = getenv("JUNO_ATTN_SPLITS")) s = std::max(1, std::min(s, atoi(e)));
-    s = std::min(s, 64);
     // Up to twice the cluster limit the count is rounded down to a power of two within it, so that the splits of a
     // (sequence, kv head) can be one thread-block cluster and merge on chip; longer contexts keep their many splits
     // and the separate merge kernel.
@@ -682,9 +700,9 @@ static bool attn_use_mma() {
     return on;
 }
 
-template <int HD, int G>
+template <int HD, int G, int W = kMmaWarps>
 static size_t attn_mma_smem() {
-    return ((size_t)2 * 8 * (HD + 8) + (size_t)kMmaWarps * 4 * 16 * (HD + 8)) * sizeof(__half);
+    return ((size_t)2 * 8 * (HD + 8) + (size_t)W * 4 * 16 * (HD + 8)) * sizeof(__half);
 }
 
 // Whether a cluster of `splits` CTAs of the tensor-core kernel can be co-scheduled on this device (asked once per size).
@@ -697,8 +715,8 @@ static bool attn_cluster_fits(int splits) {
     int &f = fits[dev & 63][lg];
     if (f == 0) {
         const size_t smem = attn_mma_smem<HD, G>();
-        cudaFuncSetAttribute(attn_mma_kernel<HD, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        cudaFuncSetAttribute(attn_mma_kernel<HD, G>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        cudaFuncSetAttribute(attn_mma_kernel<HD, G, kMmaWarps>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaFuncSetAttribute(attn_mma_kernel<HD, G, kMmaWarps>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(1, splits, 1);
         cfg.blockDim = dim3(kMmaWarps * 32);
@@ -711,7 +729,7 @@ static bool attn_cluster_fits(int splits) {
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         int n = 0;
-        const cudaError_t e = cudaOccupancyMaxActiveClusters(&n, attn_mma_kernel<HD, G>, &cfg);
+        const cudaError_t e = cudaOccupancyMaxActiveClusters(&n, attn_mma_kernel<HD, G, kMmaWarps>, &cfg);
         if (e != cudaSuccess) cudaGetLastError();
         f = (e == cudaSuccess && n > 0) ? 1 : 2;
     }
@@ -732,13 +750,13 @@ static void attn_launch_inst(const AttnParams &p, int n, cudaStream_t st) {
             int dev = 0;
             cudaGetDevice(&dev);
             if (!configured[dev & 63]) {
-                cudaFuncSetAttribute(attn_mma_kernel<HD, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+                cudaFuncSetAttribute(attn_mma_kernel<HD, G, kMmaWarps>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
                 configured[dev & 63] = true;
             }
             if (p.cluster_merge) {
                 static bool np_set[64] = {false};
                 if (!np_set[dev & 63]) {
-                    cudaFuncSetAttribute(attn_mma_kernel<HD, G>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+                    cudaFuncSetAttribute(attn_mma_kernel<HD, G, kMmaWarps>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
                     np_set[dev & 63] = true;
                 }
                 cudaLaunchConfig_t cfg = {};
@@ -755,10 +773,20 @@ static void attn_launch_inst(const AttnParams &p, int n, cudaStream_t st) {
                 attr[1].val.programmaticStreamSerializationAllowed = 1;
                 cfg.attrs = attr;
                 cfg.numAttrs = pdl_enabled() ? 2 : 1;
-                cudaLaunchKernelEx(&cfg, attn_mma_kernel<HD, G>, p);
+                cudaLaunchKernelEx(&cfg, attn_mma_kernel<HD, G, kMmaWarps>, p);
                 return;
             }
-            launch_pdl(attn_mma_kernel<HD, G>, grid, dim3(kMmaWarps * 32), smem, st, p);
+            if (p.wide) {
+                const size_t wide = attn_mma_smem<HD, G, kWideWarps>();
+                static bool wide_set[64] = {false};
+                if (!wide_set[dev & 63]) {
+                    cudaFuncSetAttribute(attn_mma_kernel<HD, G, kWideWarps>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wide);
+                    wide_set[dev & 63] = true;
+                }
+                launch_pdl(attn_mma_kernel<HD, G, kWideWarps>, grid, dim3(kWideWarps * 32), wide, st, p);
+                return;
+            }
+            launch_pdl(attn_mma_kernel<HD, G, kMmaWarps>, grid, dim3(kMmaWarps * 32), smem, st, p);
             return;
         }
     }
@@ -812,6 +840,7 @@ int launch_attn(juno_ctx *ctx, const AttnArgs &a, cudaStream_t st) {
     if (pool->dtype == 0 && attn_use_mma() && a.n_splits <= attn_cluster_max() &&
         (a.n_splits & (a.n_splits - 1)) == 0 && (G * hd) % a.n_splits == 0 && attn_cluster_fits_any(hd, G, a.n_splits))
         p.cluster_merge = 1;
+    p.wide = !p.cluster_merge && a.n_splits == 1 && attn_wide(ctx, a.n * pool->n_kv_heads, hd) ? 1 : 0;
     ProfScope prof(ctx, st, PROF_ATTN, a.algo_bytes);
     int rc;
     if (pool->dtype == 0)
@@ -820,7 +849,7 @@ int launch_attn(juno_ctx *ctx, const AttnArgs &a, cudaStream_t st) {
         rc = hd == 128 ? attn_launch_g<float, 128>(p, a.n, G, st) : attn_launch_g<float, 64>(p, a.n, G, st);
     JUNO_TRY(rc);
     JUNO_CUDA_TRY(cudaGetLastError());
-    if (p.cluster_merge) {
+    if (p.cluster_merge || (p.n_splits == 1 && pool->dtype == 0 && attn_use_mma())) {  // the kernel has stored the results
         ctx->kernel_launches += 1;
         return JUNO_OK;
     }
@@ -1269,7 +1298,7 @@ int juno_attn_decode(juno_ctx *c, juno_kvpool *p, int32_t layer, int32_t n, juno
         max_len = std::max(max_len, seqs[i]->len);
     }
     const int hd = p->head_dim, qdim = n_heads * hd;
-    const int n_splits = attn_pick_splits(c, n, p->n_kv_heads, max_len);
+    const int n_splits = attn_pick_splits(c, n, p->n_kv_heads, p->head_dim, max_len);
     const size_t qbytes = (size_t)n * qdim * sizeof(float);
     const size_t scratch = attn_scratch_floats(n, n_heads, hd, n_splits) * sizeof(float);
     const size_t meta_bytes = meta.size() * sizeof(int32_t);
@@ -1369,7 +1398,7 @@ int juno_attn_decode_static(juno_ctx *c, juno_kvpool *p, int32_t layer, int32_t 
                   "entry point has %zu", n, n_heads, hd, per_split, room);
         return JUNO_ERR_INVALID_ARG;
     }
-    int n_splits = attn_pick_splits(c, n, p->n_kv_heads, max_len);
+    int n_splits = attn_pick_splits(c, n, p->n_kv_heads, p->head_dim, max_len);
     n_splits = (int)std::min<size_t>((size_t)n_splits, room / per_split);
     int32_t *d_meta = static_cast<int32_t *>(base);
     float *sc = reinterpret_cast<float *>(static_cast<unsigned char *>(base) + meta_bytes);

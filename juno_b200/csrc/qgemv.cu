@@ -519,6 +519,16 @@ __device__ __forceinline__ float qpeer_ld(uint32_t addr, int rank) {
     asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
     return v;
 }
+// The sum over the cluster's CTAs in rank order, the loads all on their way before the first is used.
+__device__ __forceinline__ float qpeer_sum(uint32_t addr, int splits) {
+    float part[8], v = 0.f;
+#pragma unroll
+    for (int r = 0; r < 8; r++) part[r] = r < splits ? qpeer_ld(addr, r) : 0.f;
+#pragma unroll
+    for (int r = 0; r < 8; r++)
+        if (r < splits) v += part[r];
+    return v;
+}
 // Floats of the exchange of a SPLIT kernel: two buffers of a chunk's sums (all sixteen rows of its row tiles), then the sums of squares.
 __host__ __device__ constexpr int qexchange_floats(int bc) { return 2 * kQChunk * 16 * bc + 8; }
 
@@ -730,8 +740,7 @@ __global__ void __launch_bounds__(kQThreads, OCC) qgemv_kernel(const __grid_cons
             if (tid < 8) {
                 float sc = 1.f;
                 if (p.normw) {
-                    float s = 0.f;
-                    for (int r = 0; r < p.splits; r++) s += qpeer_ld(xs + (2 * kQChunk * 16 * p.bc + tid) * 4, r);
+                    const float s = qpeer_sum(xs + (2 * kQChunk * 16 * p.bc + tid) * 4, p.splits);
                     sc = __fdiv_rn(1.f, __fsqrt_rn(__fadd_rn(__fdiv_rn(s, (float)p.K), p.eps)));
                 }
                 rs_s[tid] = sc;
@@ -745,11 +754,8 @@ __global__ void __launch_bounds__(kQThreads, OCC) qgemv_kernel(const __grid_cons
             const int b = idx / per_b, rg = idx - b * per_b, l = rg >> rows_sh, row = rg & (rows_out - 1);
             const uint32_t at = xb + (uint32_t)((b * crt + l) * 16 + row) * 4;
             const int Rg = lo + l, s = qseg_of(p, Rg), orow = (Rg - p.rt_begin[s]) * rows_out + row;
-            float v = 0.f, v2 = 0.f;
-            for (int r = 0; r < p.splits; r++) {
-                v += qpeer_ld(at, r);
-                if (p.epi == QEPI_SILU_PAIR) v2 += qpeer_ld(at + 32, r);
-            }
+            float v = qpeer_sum(at, p.splits);
+            const float v2 = p.epi == QEPI_SILU_PAIR ? qpeer_sum(at + 32, p.splits) : 0.f;
             if (orow >= p.rows[s]) continue;
             v = __fmul_rn(v, rs_s[b]);
             if (p.epi == QEPI_SILU_PAIR) v = __fmul_rn(silu_f(v), __fmul_rn(v2, rs_s[b]));

@@ -662,15 +662,18 @@ static int attn_cluster_max() {
 static bool attn_wide(const juno_ctx *ctx, int pairs, int hd) { return pairs <= ctx->sm_count * (hd == 128 ? kWideCtas<128> : kWideCtas<64>); }
 // How many CTAs share the context of a (sequence, kv head).  A CTA takes about three page times beside the pages of its busiest warp, CTAs
 // run in rounds of as many as the GPU holds, and more than one split cost a merge.  Every round counts in full: Llama-3-8B, six requests of
-// 512 to 1024 positions, 6 splits (one round of two CTAs per SM, which was what registers allowed) 7.9 us a layer, 8 splits (1.3 rounds) 11.9; eight requests of
-// up to 4096 positions, 4 splits 25 + 10 us, 10 splits 32 + 12.
-int attn_pick_splits(const juno_ctx *ctx, int n, int n_kv_heads, int hd, int max_len) {
-    const int pairs = std::max(1, n * n_kv_heads), slots = ctx->sm_count * (hd == 128 ? kMmaCtas<128> : kMmaCtas<64>), pages = (max_len + kPageTokens - 1) / kPageTokens;
+// 512 to 1024 positions, 6 splits (one round of two CTAs per SM, which was what registers allowed) 7.9 us a layer, 8 splits (1.3 rounds) 11.9, with
+// three CTAs per SM 7.1; eight requests of up to 4096 positions, 4 splits 25 + 10 us, 10 splits 32 + 12.  A context of one split has no merge: TinyLlama, 150
+// positions 0.787 -> 0.761 ms a step, Llama-3-8B, 100 positions 1.85 -> 1.73; 450 positions of TinyLlama in one split of eight warps 0.811, in four of four 0.798.
+// FP32 pages have a kernel of their own, always with a merge: as many splits as fill the GPU with four CTAs per SM.
+int attn_pick_splits(const juno_ctx *ctx, const juno_kvpool *pool, int n, int max_len) {
+    const int hd = pool->head_dim;
+    const int pairs = std::max(1, n * pool->n_kv_heads), slots = ctx->sm_count * (hd == 128 ? kMmaCtas<128> : kMmaCtas<64>), pages = (max_len + kPageTokens - 1) / kPageTokens;
     // at least 128 positions per split (two pages per warp), and no more partial results than the callers have room for
     const int most = std::min({std::max(1, (max_len + 127) / 128), (ctx->sm_count * 4 + pairs - 1) / pairs, 64});
-    int s = 1;
+    int s = pool->dtype == 0 ? 1 : most;
     double best = 1e30;
-    for (int k = 1; k <= most; k++) {
+    for (int k = 1; pool->dtype == 0 && k <= most; k++) {
         const bool wide = k == 1 && attn_wide(ctx, pairs, hd);
         const int rounds = wide ? 1 : (pairs * k + slots - 1) / slots, warps = wide ? kWideWarps : kMmaWarps, per_warp = ((pages + k - 1) / k + warps - 1) / warps;
         const double cost = rounds * (per_warp + 3.0) + (k > 1 ? 1.5 + k / 16.0 : 0.0);
@@ -1298,7 +1301,7 @@ int juno_attn_decode(juno_ctx *c, juno_kvpool *p, int32_t layer, int32_t n, juno
         max_len = std::max(max_len, seqs[i]->len);
     }
     const int hd = p->head_dim, qdim = n_heads * hd;
-    const int n_splits = attn_pick_splits(c, n, p->n_kv_heads, p->head_dim, max_len);
+    const int n_splits = attn_pick_splits(c, p, n, max_len);
     const size_t qbytes = (size_t)n * qdim * sizeof(float);
     const size_t scratch = attn_scratch_floats(n, n_heads, hd, n_splits) * sizeof(float);
     const size_t meta_bytes = meta.size() * sizeof(int32_t);
@@ -1398,7 +1401,7 @@ int juno_attn_decode_static(juno_ctx *c, juno_kvpool *p, int32_t layer, int32_t 
                   "entry point has %zu", n, n_heads, hd, per_split, room);
         return JUNO_ERR_INVALID_ARG;
     }
-    int n_splits = attn_pick_splits(c, n, p->n_kv_heads, p->head_dim, max_len);
+    int n_splits = attn_pick_splits(c, p, n, max_len);
     n_splits = (int)std::min<size_t>((size_t)n_splits, room / per_split);
     int32_t *d_meta = static_cast<int32_t *>(base);
     float *sc = reinterpret_cast<float *>(static_cast<unsigned char *>(base) + meta_bytes);

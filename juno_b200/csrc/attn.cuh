@@ -66,7 +66,7 @@ struct AttnArgs {
     int ldkv = 0;
 };
 size_t attn_scratch_floats(int n, int n_heads, int hd, int n_splits);
-int attn_pick_splits(const juno_ctx *ctx, int n, int n_kv_heads, int hd, int max_len);
+int attn_pick_splits(const juno_ctx *ctx, const juno_kvpool *pool, int n, int max_len);
 int launch_attn(juno_ctx *ctx, const AttnArgs &a, cudaStream_t st);
 
 #if defined(__CUDACC__)

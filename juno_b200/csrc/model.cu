@@ -1123,7 +1123,7 @@ static int enqueue_layers_prompt(juno_model *m, int n, int pos0, bool fused, boo
                 at.out = P.att + (size_t)r * Hl;
                 at.slots = d_slot + r;
                 at.seq_lens = d_len + r;
-                at.n_splits = attn_pick_splits(c, at.n, m->kv_loc, hd, pos0 + r + at.n);
+                at.n_splits = attn_pick_splits(c, m->pool, at.n, pos0 + r + at.n);
                 at.part_o = m->attn_scratch;
                 at.part_ml = m->attn_scratch + (size_t)at.n * m->heads_loc * at.n_splits * hd;
                 at.algo_bytes = (double)at.n * (pos0 + r) * KVl * 2 * m->pool->elem_bytes;
@@ -1609,7 +1609,7 @@ static int prepare_step(juno_model *m, int n, juno_seq *const *seqs, const int32
     m->step_kv_bytes = 0;
     for (int i = 0; i < n; i++)
         m->step_kv_bytes += (double)(positions[i] + 1) * m->kv_loc * m->hd * 2 * m->pool->elem_bytes;
-    *n_splits = m->stack ? stack_pick_splits(c, m->stack, n, bucket_len(max_len)) : attn_pick_splits(c, n, m->kv_loc, m->hd, bucket_len(max_len));
+    *n_splits = m->stack ? stack_pick_splits(c, m->stack, n, bucket_len(max_len)) : attn_pick_splits(c, m->pool, n, bucket_len(max_len));
     JUNO_CUDA_TRY(cudaMemcpyAsync(m->d_step, m->h_step, (size_t)4 * B * 4, cudaMemcpyHostToDevice, c->stream));
     c->h2d_bytes += 4 * n * 4;
     return JUNO_OK;
@@ -1676,7 +1676,7 @@ static int prefill_run(juno_model *m, juno_seq *seq, const int32_t *token_ids, i
         } else {
             m->step_kv_bytes = 0;
             for (int i = 0; i < n; i++) m->step_kv_bytes += (double)(pos0 + i + 1) * m->kv_loc * m->hd * 2 * m->pool->elem_bytes;
-            const int n_splits = attn_pick_splits(c, n, m->kv_loc, m->hd, bucket_len(pos0 + n));
+            const int n_splits = attn_pick_splits(c, m->pool, n, bucket_len(pos0 + n));
             JUNO_TRY(launch_embed(m, n, d_tok, d_pos, many ? m->prompt.x[0] : m->x[0], many ? m->prompt.cs : m->rope_cs, st));
             int cur = 0;
             if (many)

@@ -85,6 +85,8 @@ __global__ void __launch_bounds__(kFewThreads, 2) gemm_few_kernel(const __grid_c
     const int k_lo = (int)((long long)p.k_steps * rank / p.splits), steps = (int)((long long)p.k_steps * (rank + 1) / p.splits) - k_lo;
     const int tmem_cols = p.cols <= 32 ? 32 : p.cols <= 64 ? 64 : 128;
     if (threadIdx.x == 0) {
+        prefetch_map(&p.tw);
+        prefetch_map(&p.ta);
         for (int s = 0; s < S; s++) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(full0 + 8 * s) : "memory");
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(empty0 + 8 * s) : "memory");

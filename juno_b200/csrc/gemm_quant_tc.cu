@@ -161,7 +161,7 @@ struct QtUnpack {
 };
 // The tiles of one row tile, nb of them, unpacked into the stages in turn.  TYPE 0: a warp without a row tile, which only keeps step.
 // One body per format: the store takes 32 registers in a row, and where the formats' paths met before it every one was moved.
-template <int TYPE, bool PRECISE>
+template <int TYPE, bool WIDE>
 __device__ __forceinline__ void qt_unpack(QtUnpack &u, const RowPow &P, int nb, volatile unsigned *fail) {
     const int lane = threadIdx.x & 31;
 #pragma unroll 1
@@ -171,12 +171,12 @@ __device__ __forceinline__ void qt_unpack(QtUnpack &u, const RowPow &P, int nb, 
         if constexpr (TYPE != 0) {
             bar_wait(u.tile_bar + u.slot * 8, u.tpar, fail);
             __syncwarp();
-            tile_factors_f16<TYPE>(F, P, tile, lane);
+            tile_factors_f16<TYPE, WIDE>(F, P, tile, lane);
         }
 #pragma unroll
         for (int h = 0; h < 2; h++) {
             uint32_t r[32];
-            if constexpr (TYPE != 0) tile_half_f16<TYPE, PRECISE>(F, tile, h, lane, r);
+            if constexpr (TYPE != 0) tile_half_f16<TYPE, WIDE>(F, tile, h, lane, r);
             bar_wait(u.free + u.sa * 8, u.apar ^ 1u, fail);
             __syncwarp();
             if constexpr (TYPE != 0) {
@@ -264,7 +264,7 @@ __global__ void __launch_bounds__((kQtWarps + 4) * 32, 2) gemm_quant_kernel(cons
             const bool active = warp < w.r;
             const int rt = w.lo + warp, seg = active ? qt_seg(p, rt) : 0, type = p.type[seg];
             RowPow P;
-            if (active) P = row_pow_load(p.pow[seg], (rt - p.rt_begin[seg]) * 16 + g);
+            if (active) P = row_pow_load(p.pow[seg], (rt - p.rt_begin[seg]) * 16 + g, type, PRECISE);
             if (!active)
                 qt_unpack<0, false>(u, P, nb, fail);
             else if (type == 12)
@@ -284,7 +284,7 @@ __global__ void __launch_bounds__((kQtWarps + 4) * 32, 2) gemm_quant_kernel(cons
             if (active) {
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const int col0 = w.block * p.N, cols = min(p.N, p.n - col0);
-                const float undo0 = row_pow_undo(P, 0), undo1 = row_pow_undo(P, 1);
+                const float undo0 = P.undo[0], undo1 = P.undo[1];
 #pragma unroll 1
                 for (int c = 0; c < cols; c += 16) {
                     uint32_t r[8];

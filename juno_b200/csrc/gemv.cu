@@ -13,6 +13,7 @@
 #include "layout.cuh"
 #include "dequant.cuh"
 #include "repack.cuh"
+#include "row_pow.cuh"
 
 namespace juno {
 
@@ -125,28 +126,30 @@ int launch_dequant(juno_ctx *ctx, const juno_qmat *m, int64_t row_start, int64_t
 }
 
 // ───────────────────────────── resident matrix ─────────────────────────────────────────────
-// The power of two of every row (tile_f16.cuh): what brings the largest scale of the row, times what it is multiplied with, into
-// [2^14, 2^15), as two FP16 factors.  One warp per row tile: 16 rows x two super-blocks at a time.
+// The powers of two of every row.  One warp per row tile: 16 rows x two super-blocks at a time.
 __global__ void row_pow_kernel(int type, const uint8_t *tiles, int64_t nb, uint32_t *pow) {
     const int lane = threadIdx.x, row = lane & 15;
     const uint8_t *t0 = tiles + (size_t)blockIdx.x * nb * tile_bytes(type);
     auto half_at = [](const uint8_t *p) { return fabsf(__half2float(*reinterpret_cast<const __half *>(p))); };
-    float top = 0.f;
+    RowScales r;
     for (int64_t sb = lane >> 4; sb < nb; sb += 2) {
         const uint8_t *t = t0 + sb * tile_bytes(type);
-        if (type == 12)
-            top = fmaxf(top, fmaxf(63.f * half_at(t + row * 4), half_at(t + row * 4 + 2)));
-        else if (type == 14)
-            top = fmaxf(top, 128.f * half_at(t + 3328 + row * 2));
-        else
-            for (int j = 0; j < 8; j++) top = fmaxf(top, half_at(t + 4096 + row * 16 + j * 2));
+        if (type == 12) {
+            uint8_t sc[8], mn[8];
+            for (int j = 0; j < 8; j++) {  // (scale, scale, min, min) bytes of the sub-block pairs
+                sc[j] = t[64 + row * 16 + (j >> 1) * 4 + (j & 1)];
+                mn[j] = t[64 + row * 16 + (j >> 1) * 4 + 2 + (j & 1)];
+            }
+            row_scales_q4(r, half_at(t + row * 4), half_at(t + row * 4 + 2), sc, mn);
+        } else if (type == 14) {
+            row_scales_q6(r, half_at(t + 3328 + row * 2), reinterpret_cast<const int8_t *>(t + 3072 + row * 16));
+        } else {
+            for (int j = 0; j < 8; j++) row_scales_q8(r, half_at(t + 4096 + row * 16 + j * 2));
+        }
     }
-    top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 16));
-    int e = 15;
-    if (top > 0.f && top < 3.0e38f) frexpf(top, &e);
-    const int p = min(15 - e, 30), a = min(p, 15);
-    if (lane < 16)
-        pow[blockIdx.x * 16 + row] = (uint32_t)__half_as_ushort(__float2half_rn(ldexpf(1.f, a))) | (uint32_t)__half_as_ushort(__float2half_rn(ldexpf(1.f, p - a))) << 16;
+    r.top = fmaxf(r.top, __shfl_xor_sync(0xffffffffu, r.top, 16));
+    r.most = fmaxf(r.most, __shfl_xor_sync(0xffffffffu, r.most, 16));
+    if (lane < 16) pow[blockIdx.x * 16 + row] = row_pow_word(r);
 }
 
 int qmat_create(juno_ctx *ctx, const void *blocks, int type, int64_t rows_total, int64_t cols_total, int64_t row0,

@@ -267,10 +267,16 @@ __global__ void __launch_bounds__((kQtWarps + 4) * 32, 2) gemm_quant_kernel(cons
             if (active) P = row_pow_load(p.pow[seg], (rt - p.rt_begin[seg]) * 16 + g, type, PRECISE);
             if (!active)
                 qt_unpack<0, false>(u, P, nb, fail);
+            else if (type == 12 && (PRECISE || P.wide))
+                qt_unpack<12, true>(u, P, nb, fail);
             else if (type == 12)
                 qt_unpack<12, PRECISE>(u, P, nb, fail);
+            else if (type == 14 && (PRECISE || P.wide))
+                qt_unpack<14, true>(u, P, nb, fail);
             else if (type == 14)
                 qt_unpack<14, PRECISE>(u, P, nb, fail);
+            else if (P.wide)
+                qt_unpack<8, true>(u, P, nb, fail);
             else
                 qt_unpack<8, false>(u, P, nb, fail);
             if (!waited) {  // what earlier kernels wrote and read is done with

@@ -126,7 +126,8 @@ int launch_dequant(juno_ctx *ctx, const juno_qmat *m, int64_t row_start, int64_t
 }
 
 // ───────────────────────────── resident matrix ─────────────────────────────────────────────
-// The powers of two of every row.  One warp per row tile: 16 rows x two super-blocks at a time.
+// The powers of two of every row and whether its row tile is unpacked the wide way (row_pow_word).  One warp per row tile: 16 rows x two
+// super-blocks at a time.
 __global__ void row_pow_kernel(int type, const uint8_t *tiles, int64_t nb, uint32_t *pow) {
     const int lane = threadIdx.x, row = lane & 15;
     const uint8_t *t0 = tiles + (size_t)blockIdx.x * nb * tile_bytes(type);
@@ -149,7 +150,11 @@ __global__ void row_pow_kernel(int type, const uint8_t *tiles, int64_t nb, uint3
     }
     r.top = fmaxf(r.top, __shfl_xor_sync(0xffffffffu, r.top, 16));
     r.most = fmaxf(r.most, __shfl_xor_sync(0xffffffffu, r.most, 16));
-    if (lane < 16) pow[blockIdx.x * 16 + row] = row_pow_word(r);
+    r.low = fminf(r.low, __shfl_xor_sync(0xffffffffu, r.low, 16));
+    r.low_sub = fminf(r.low_sub, __shfl_xor_sync(0xffffffffu, r.low_sub, 16));
+    const uint32_t w = row_pow_word(type, r);
+    const bool wide = __any_sync(0xffffffffu, w & kRowWide);
+    if (lane < 16) pow[blockIdx.x * 16 + row] = wide ? w | kRowWide : w;
 }
 
 int qmat_create(juno_ctx *ctx, const void *blocks, int type, int64_t rows_total, int64_t cols_total, int64_t row0,

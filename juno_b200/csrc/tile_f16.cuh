@@ -8,10 +8,12 @@
 // warps); see gemm_quant_tc.cu for what it takes now.  S and m round once from exact products, the result rounds once: the same error as s and m in
 // FP16 have (products of random rows with Q4_K 5.8e-4, Q6_K 3.5e-4, Q8_0 2.9e-4 relative), as long as the blocks of a row are alike.
 //
-// Wide: Q4_K and Q6_K in prompts (PRECISE).  The power of two puts the largest weight of the row below 2^15, so that
-// weights down to 2^-29 of it are FP16 numbers of full precision.  s and m are kept in FP32, exact, w = s*q - m by an FP32 multiply-add, rounded
-// to FP16: once, but for the 2^-24 of the multiply-add, whatever the minima.  Errors of products of random rows 2.9e-4 for all
-// formats.  It costs half as many instructions again.
+// Wide: for row tiles whose blocks lie far apart (row_pow_word), and in prompts (PRECISE).  The power of two puts the largest weight of the row below 2^15, so that
+// weights down to 2^-29 of it are FP16 numbers of full precision.  Q4_K and Q6_K: s and m in FP32, exact, w = s*q - m by an FP32 multiply-add, rounded
+// to FP16: once, but for the 2^-24 of the multiply-add, whatever the minima.  Q8_0: q, exact, times d * 2^e.  Errors of products of random rows 2.9e-4 for all
+// formats, a third less for Q4_K and Q6_K.  It costs half as many instructions again; prompts do not notice, steps of few rows do: with all tiles wide
+// Llama-3-8B with 4 layers, 9 / 32 / 64 requests 448 / 542 / 713 -> 534 / 628 / 798 us a step, TinyLlama 1273 / 1431 / 1680 -> 1383 / 1531 / 1719, in Q8_0 1236 /
+// 1392 / 1679 -> 1253 / 1417 / 1684.
 //
 // A half of a tile is 128 of its 256 columns.  Lane (g, t) of the warp gets, for each of the half's eight 16-column groups, four
 // registers of two values: row g columns (4t, 4t+2), row g columns (4t+1, 4t+3), and the same of row g + 8.  That is the order in
@@ -69,7 +71,7 @@ __device__ __forceinline__ RowPow row_pow_load(const uint32_t *pow, int row, int
 #pragma unroll
     for (int k = 0; k < 2; k++) {
         const uint32_t w = __ldg(pow + row + 8 * k);
-        P.wide = precise && type != 8;
+        P.wide = (w & kRowWide) != 0 || (precise && type != 8);
         const int e = (int)(P.wide ? w >> 8 & 0xFFu : w & 0xFFu) - kRowPowBias, first = min(e, 15);
         P.undo[k] = __uint_as_float((uint32_t)(127 + (P.wide ? 0 : 24) - e) << 23);
         P.a[k] = P.wide && type != 8 ? (uint32_t)(127 + e) << 23 : (uint32_t)(15 + first) * 0x04000400u;
@@ -238,6 +240,7 @@ __device__ __forceinline__ void q8_factors(TileFactors &F, const RowPow &P, uint
 #pragma unroll
     for (int k = 0; k < 8; k++) F.f[k] = h2_mul(h2_mul(d[k], P.a[k >> 2]), P.b[k >> 2]);
 }
+template <bool WIDE>
 __device__ __forceinline__ void q8_half_f16(const TileFactors &F, uint32_t tile, int half, int lane, uint32_t (&o)[32]) {
     uint4 w[4];
 #pragma unroll
@@ -251,8 +254,14 @@ __device__ __forceinline__ void q8_half_f16(const TileFactors &F, uint32_t tile,
 #pragma unroll
             for (int i = 0; i < 2; i++) {
                 uint32_t *p = o + 8 * j + 4 * i + 2 * row;
-                p[0] = h2_fma(__byte_perm(w4[2 * row + i], 0u, 0x4240), s, c);
-                p[1] = h2_fma(__byte_perm(w4[2 * row + i], 0u, 0x4341), s, c);
+                const uint32_t v = w4[2 * row + i];
+                if constexpr (WIDE) {  // q as it is, exact, times the scale
+                    p[0] = h2_mul(h2_sub(__byte_perm(v, 0x64646464u, 0x4240), kH1152), s);
+                    p[1] = h2_mul(h2_sub(__byte_perm(v, 0x64646464u, 0x4341), kH1152), s);
+                } else {
+                    p[0] = h2_fma(__byte_perm(v, 0u, 0x4240), s, c);
+                    p[1] = h2_fma(__byte_perm(v, 0u, 0x4341), s, c);
+                }
             }
         }
     }
@@ -274,7 +283,7 @@ __device__ __forceinline__ void tile_factors_f16(TileFactors &F, const RowPow &P
 template <int TYPE, bool WIDE>
 __device__ __forceinline__ void tile_half_f16(const TileFactors &F, uint32_t tile, int half, int lane, uint32_t (&o)[32]) {
     if constexpr (TYPE == 8)
-        q8_half_f16(F, tile, half, lane, o);
+        q8_half_f16<WIDE>(F, tile, half, lane, o);
     else if constexpr (TYPE == 12 && WIDE)
         q4_half_wide(F, tile, half, lane, o);
     else if constexpr (TYPE == 12)

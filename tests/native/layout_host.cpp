@@ -137,3 +137,20 @@ extern "C" int ring_check(int n, int slots, int fail) {
     }
     return open != issued - used;
 }
+
+// ── powers of two of a row and the way its row tile is unpacked (row_pow.cuh) ─────────────
+#include "../../juno_b200/csrc/row_pow.cuh"
+
+// factors: the |d| of every super-block (Q8_0: block), then |dmin| (Q4_K).  scales: per super-block 8 scales and 8 minima (Q4_K) or 16 scales (Q6_K).
+extern "C" uint32_t row_pow_of(int type, int blocks, const float *factors, const uint8_t *scales) {
+    RowScales r;
+    for (int b = 0; b < blocks; b++) {
+        if (type == 12)
+            row_scales_q4(r, factors[b], factors[blocks + b], scales + b * 16, scales + b * 16 + 8);
+        else if (type == 14)
+            row_scales_q6(r, factors[b], reinterpret_cast<const int8_t *>(scales + b * 16));
+        else
+            row_scales_q8(r, factors[b]);
+    }
+    return row_pow_word(type, r);
+}

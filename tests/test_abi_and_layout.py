@@ -115,3 +115,62 @@ def test_rings_know_the_copies_that_are_in_flight(layout_host, slots):
     for n in range(1, 30):
         for fail in range(n + 1):
             assert layout_host.ring_check(n, slots, fail) == 0, (n, fail)
+
+
+@pytest.mark.parametrize("t", [12, 14, 8])
+def test_row_tiles_that_quick_unpacking_would_cost_digits_are_wide(layout_host, t):
+    """The powers of two of a row and the choice between quick and wide unpacking (csrc/row_pow.cuh, as the device finds them).  Wherever a row stays quick, the
+    weights of every super-block, however far below the largest, are off by at most a quarter more than scales, minima and weights rounded to 11 bits
+    each, at their own size, would be; and rows whose super-blocks are alike do stay quick.  Wide, the largest weight lies in [2^12, 2^15) (the bound of it in the
+    upper half) unless that would take digits from a row that FP16 holds as it is."""
+    import ctypes as C
+    L = layout_host
+    L.row_pow_of.restype, L.row_pow_of.argtypes = C.c_uint32, [C.c_int, C.c_int, C.c_void_p, C.c_void_p]
+
+    def r11(v):
+        m, e = np.frexp(v)
+        return np.ldexp(np.round(m * 2048.0) / 2048.0, e)
+
+    def h(v):
+        return np.asarray(v, np.float64).astype(np.float16).astype(np.float64)
+
+    rng = np.random.default_rng(t)
+    quick = 0
+    for trial in range(300):
+        n, spread = 16, float(rng.choice([1.0, 3.0])) if trial % 2 else 2.0 ** rng.uniform(0, 13)
+        d = (2.0 ** rng.uniform(-17, -6) * spread ** rng.uniform(-1, 0, n)).astype(np.float16).astype(np.float64)
+        if t == 12:
+            sc, mn = rng.integers(16, 64, (n, 8)), rng.integers(0, 64, (n, 8))
+            dm = h(d * rng.choice([0.0, 1.0, 7.5, 15.0]))
+            q = rng.integers(0, 16, (n, 8, 32)).astype(np.float64)
+            s, m = d[:, None] * sc, dm[:, None] * mn
+            scales, factors = np.concatenate([sc, mn], 1).astype(np.uint8), np.concatenate([d, dm]).astype(np.float32)
+        elif t == 14:
+            sc = rng.integers(16, 128, (n, 16)) * rng.choice([-1, 1], (n, 16))
+            q = rng.integers(-32, 32, (n, 16, 16)).astype(np.float64)
+            s, m = d[:, None] * sc, np.zeros((n, 16))
+            scales, factors = sc.astype(np.int8).view(np.uint8), d.astype(np.float32)
+        else:
+            q = rng.integers(-127, 128, (n, 1, 32)).astype(np.float64)
+            s, m = d[:, None], np.zeros((n, 1))
+            scales, factors = np.zeros(1, np.uint8), d.astype(np.float32)
+        scales, factors = np.ascontiguousarray(scales), np.ascontiguousarray(factors)
+        word = L.row_pow_of(t, n, factors.ctypes.data, scales.ctypes.data)
+        p, wp, wide = (word & 255) - 64, (word >> 8 & 255) - 64, word >> 16
+        w = s[..., None] * q - m[..., None]
+        own = r11(r11(s)[..., None] * q - r11(m)[..., None])
+        got = h(q * 2.0 ** -24 * h(s * 2.0 ** p)[..., None] - h(m * 2.0 ** (p - 24))[..., None]) * 2.0 ** (24 - p)
+        axes = (1, 2)
+        if not wide:
+            quick += 1
+            assert (np.sqrt(((got - w) ** 2).mean(axes)) <= 1.25 * np.sqrt(((own - w) ** 2).mean(axes)) + 1e-30).all(), (trial, spread)
+        elif trial % 2:
+            raise AssertionError("alike super-blocks, yet wide")
+        most = np.abs(w).max() * 2.0 ** wp
+        assert most < 2.0 ** 15 and (most >= 2.0 ** 12 or wp == 30)
+    assert quick >= 150
+    zero = np.zeros(32, np.float32)
+    assert L.row_pow_of(t, 16, zero.ctypes.data, np.zeros(256, np.uint8).ctypes.data) == 64 | 64 << 8
+    inf = np.full(32, np.inf, np.float32)
+    inf[1:] = 1.0
+    assert L.row_pow_of(t, 16, inf.ctypes.data, np.full(256, 9, np.uint8).ctypes.data) & 0xFFFF == 64 | 64 << 8

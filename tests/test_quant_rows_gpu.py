@@ -110,13 +110,39 @@ def far_apart(t, rows, cols, ratio, place, minimum=7.5, seed=33):
     return raw.reshape(-1)
 
 
+@pytest.mark.parametrize("t", TYPES)
+@pytest.mark.parametrize("ratio", [1, 16, 64, 512, 4096])
+@pytest.mark.parametrize("place", [0, 2, 5])
+def test_blocks_of_one_row_far_apart(mv, oracle, t, ratio, place):
+    """A large super-block takes no digits from the others of its row: the path's 1e-3 holds where the activation is zero on it, and each single weight
+    is off by its own rounding.  Weights come out through activations of a single one: the sum has one term, and is exact.  A weight of a wide row is
+    rounded once (2^-11 of it at most); of a quick one, scale, minimum and weight are (of Q4_K a weight is the difference of two parts)."""
+    rows, cols, batch = 70, 6 * 256, 16
+    raw = far_apart(t, rows, cols, ratio, place)
+    rng = np.random.default_rng(ratio)
+    x = rng.standard_normal((batch, cols)).astype(np.float32)
+    x[::2, place * 256:(place + 1) * 256] = 0
+    A = mv.upload_quantized(raw, t, rows, cols)
+    y, ref = mv.sgemv(A, x), oracle.matvec(t, raw, x, rows, cols)
+    for part in (slice(0, None, 2), slice(1, None, 2)):
+        assert np.linalg.norm(y[part] - ref[part]) < 1e-3 * np.linalg.norm(ref[part])
+    w = oracle.dequantize(t, raw, rows, cols).reshape(rows, cols).astype(np.float64)
+    cols_of = rng.choice(cols, batch, replace=False)
+    one = np.zeros((batch, cols), np.float32)
+    one[np.arange(batch), cols_of] = 1
+    got = mv.sgemv(A, one).astype(np.float64).T
+    if ratio >= 512 and t != synth.Q8_0 or ratio > 512:
+        assert (np.abs(got - w[:, cols_of]) <= 2.0 ** -11 * 1.001 * np.abs(w[:, cols_of]) + 2.0 ** -38 * np.abs(w).max()).all()
+    A.close()
+
+
 def round11(v):
     m, e = np.frexp(v)
     return np.ldexp(np.round(m * 2048.0) / 2048.0, e)
 
 
 @pytest.mark.parametrize("t,minimum,ratio", [(synth.Q4_K, 7.5, 1), (synth.Q4_K, 0, 1), (synth.Q4_K, 4, 1), (synth.Q4_K, 15, 1), (synth.Q4_K, 4, 512),
-                                             (synth.Q6_K, 0, 1), (synth.Q6_K, 0, 512), (synth.Q8_0, 0, 1)])
+                                             (synth.Q6_K, 0, 1), (synth.Q6_K, 0, 512), (synth.Q8_0, 0, 1), (synth.Q8_0, 0, 4096)])
 def test_prompts_round_weights_once(ctx, oracle, t, minimum, ratio):
     """A prompt through one layer against the same in 64 bits with the gate and up weights rounded to 11 bits once.  The rest is made so that nothing else
     rounds, but for the FP16 rows of the down projection (stated too): activations of the feed-forward are plus or minus one, its down weights

@@ -982,25 +982,35 @@ static int prompt_alloc_rows(juno_model *m, int rows) {
     return JUNO_OK;
 }
 
+// Room for the FP16 rows of the weights: two buffers of the largest group of matrices that one product takes.
+static int prompt_alloc_weights(juno_model *m) {
+    JunoPrompt &P = m->prompt;
+    size_t w16 = 0;  // elements
+    for (const JunoLayer &L : m->layers) {
+        auto elems = [&](int k) { return (size_t)L.w[k]->row_tiles * 16 * (size_t)L.w[k]->cols; };
+        w16 = std::max({w16, elems(JUNO_T_ATTN_Q) + elems(JUNO_T_ATTN_K) + elems(JUNO_T_ATTN_V), elems(JUNO_T_ATTN_OUT), elems(JUNO_T_FFN_GATE), elems(JUNO_T_FFN_DOWN)});
+    }
+    JUNO_TRY(dev_alloc((void **)&P.weights, 2 * w16 * 2));
+    P.w16[0] = P.weights;
+    P.w16[1] = P.weights + w16 * 2;
+    return JUNO_OK;
+}
+
 // Room for passes of n positions.  Rows come in powers of two, so that prompts that grow longer ask seldom; when memory is short
-// there is room for fewer (m->prompt.rows), at least for those of before.  JUNO_ERR_OOM: for none.
-static int prompt_reserve(juno_model *m, int n) {
+// there is room for fewer (m->prompt.rows), at least for those of before.  JUNO_ERR_OOM: for none.  A portion whose products unpack the
+// tiles themselves (fused) needs no FP16 rows of the weights: they are asked for after its own rows, for a longer prompt that may come when
+// memory is short, and it goes without them if there is no memory.
+static int prompt_reserve(juno_model *m, int n, bool fused) {
     JunoPrompt &P = m->prompt;
     int rows = kPromptMinRows;
     while (rows < std::min(n, kPromptRows)) rows *= 2;
-    if (rows <= P.rows) return JUNO_OK;
+    if (rows <= P.rows && (fused || P.weights)) return JUNO_OK;
     JUNO_TRY(step_sync(m));
-    if (!P.weights) {
-        size_t w16 = 0;  // elements of the largest group of matrices that one product takes
-        for (const JunoLayer &L : m->layers) {
-            auto elems = [&](int k) { return (size_t)L.w[k]->row_tiles * 16 * (size_t)L.w[k]->cols; };
-            w16 = std::max({w16, elems(JUNO_T_ATTN_Q) + elems(JUNO_T_ATTN_K) + elems(JUNO_T_ATTN_V), elems(JUNO_T_ATTN_OUT), elems(JUNO_T_FFN_GATE), elems(JUNO_T_FFN_DOWN)});
-        }
-        JUNO_TRY(dev_alloc((void **)&P.weights, 2 * w16 * 2));
-        P.w16[0] = P.weights;
-        P.w16[1] = P.weights + w16 * 2;
+    while (!fused && !P.weights && prompt_alloc_weights(m) != JUNO_OK) {
+        if (!P.dev) return JUNO_ERR_OOM;
+        prompt_release_rows(P);
     }
-    while (prompt_alloc_rows(m, rows) != JUNO_OK) {
+    while (rows > P.rows && prompt_alloc_rows(m, rows) != JUNO_OK) {
         if (P.dev) {  // the old rows make room
             prompt_release_rows(P);
         } else if (rows == kPromptMinRows) {
@@ -1010,6 +1020,7 @@ static int prompt_reserve(juno_model *m, int n) {
             rows /= 2;
         }
     }
+    if (!P.weights) prompt_alloc_weights(m);
     return JUNO_OK;
 }
 
@@ -1637,8 +1648,8 @@ static int prefill_run(juno_model *m, juno_seq *seq, const int32_t *token_ids, i
     bool odd = false;
     const int32_t *marked = nullptr;
     // without memory for the workspace of the many-row path the portion goes through the smaller passes
-    const int prompt_rows = prompt_takes(m, n_tokens) && prompt_reserve(m, n_tokens) == JUNO_OK ? m->prompt.rows : 0;
     const bool fused = prompt_fused(m, n_tokens);
+    const int prompt_rows = prompt_takes(m, n_tokens) && prompt_reserve(m, n_tokens, fused) == JUNO_OK ? m->prompt.rows : 0;
     for (int done = 0; done < n_tokens;) {
         const bool many = prompt_rows > 0 && prompt_takes(m, n_tokens - done);
         const int n = std::min(many ? prompt_rows : chunk_max, n_tokens - done), pos0 = start_pos + done;

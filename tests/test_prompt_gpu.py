@@ -174,6 +174,36 @@ def test_prompts_with_little_memory_left(ctx, before, left_mb, passes):
         assert count == passes * per_pass + 3 * logits + hidden, (count, whole)
 
 
+def test_short_prompts_need_no_room_for_fp16_weights(ctx):
+    """300 positions with room for their rows (36 MB), but not for FP16 rows of the weights (67 MB): one pass all the same; and where memory is back, a long prompt
+    finds room for both, in place of the rows that are there."""
+    import torch
+    from juno_b200.handler import B200TransformerHandler
+    arch = synth.Arch(1024, 2, 16, 4, 8192, 512, 1e-5, 10000.0)
+    toks = np.random.default_rng(5).integers(0, arch.vocab, 900)
+
+    def run(h, n, name):
+        count = ctx.counters()["kernel_launches"]
+        return h.prefill_logits(name, toks[:n], 0, [0, n - 1]), ctx.counters()["kernel_launches"] - count
+
+    got = []
+    for left_mb in (None, 45):
+        h = B200TransformerHandler(arch, ctx, max_batch=64, max_seqs=2, max_ctx=1024)
+        h.load(tame(synth.random_model(arch, 54, MAPS["q8_0"], norm="random")))
+        h.prefill("a", toks[:60], 0)
+        held = None
+        if left_mb:
+            torch.cuda.empty_cache()
+            held = torch.empty(torch.cuda.mem_get_info()[0] - (left_mb << 20), dtype=torch.uint8, device="cuda")
+        got.append(run(h, 300, "a"))
+        del held
+        torch.cuda.empty_cache()
+        got.append(run(h, 900, "b"))
+        h.release_gpu_resources()
+    for (rows, count), (want, whole) in zip(got[2:], got[:2]):
+        assert np.array_equal(rows, want) and count == whole
+
+
 def test_profiled_bytes_of_the_products(ctx):
     """What the profile counts for the products of a prompt: 16-bit operands, FP32 results, one column per gate and up row."""
     from juno_b200.handler import B200TransformerHandler

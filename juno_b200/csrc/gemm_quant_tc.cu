@@ -25,13 +25,14 @@
 #include <mutex>
 
 #include "gemm_quant.cuh"
+#include "quant_split.cuh"
 #include "ring.cuh"
 #include "tc5.cuh"
 #include "tile_f16.cuh"
 
 namespace juno {
 
-constexpr int kQtWarps = 8, kQtThreads = (kQtWarps + 3) * 32, kQtMaxRing = 4, kQtMaxStages = 4, kQtMaxSplit = 8, kQtMaxN = 224;
+constexpr int kQtThreads = (kQtWarps + 3) * 32, kQtMaxRing = 4, kQtMaxStages = 4;
 constexpr int kQtLd = kQtWarps * 16 + 4;       // floats of a row's partial sums: the pad spreads a fragment over the banks
 constexpr int kQtPairSmem = 112 * 1024;        // two CTAs per SM
 constexpr int kQtOneSmem = 224 * 1024;
@@ -468,31 +469,36 @@ int gemm_min_batch() {
     return v;
 }
 
-// Clusters of `splits` CTAs that the device holds at a time, one CTA per SM (the driver counts no more for a kernel that allocates tensor
-// memory; two do run on an SM when they have half of it each).
-static int qt_clusters(juno_ctx *c, int splits, int *out) {
+// Clusters of every size that the device holds at a time, one CTA per SM (the driver counts no more for a kernel that allocates tensor memory; two
+// do run on an SM when they have half of it each); 0 for a size that it does not take.
+static int qt_clusters(juno_ctx *c, int (&fit)[kQtMaxSplit + 1]) {
     static std::mutex mu;
-    static int fit[16][kQtMaxSplit + 1] = {{0}};
+    static int known[16][kQtMaxSplit + 1] = {{0}};
     std::lock_guard<std::mutex> lk(mu);
-    int &f = fit[c->device & 15][splits];
-    if (f == 0) {
+    int *f = known[c->device & 15];
+    if (f[1] == 0) {
         JUNO_CUDA_TRY(cudaFuncSetAttribute(gemm_quant_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kQtOneSmem));
         JUNO_CUDA_TRY(cudaFuncSetAttribute(gemm_quant_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kQtOneSmem));
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)splits);
-        cfg.blockDim = dim3(kQtThreads);
-        cfg.dynamicSmemBytes = kQtOneSmem;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = (unsigned)splits;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        JUNO_CUDA_TRY(cudaOccupancyMaxActiveClusters(&f, gemm_quant_kernel<true>, &cfg));
-        JUNO_REQUIRE(f > 0, "quantised product: no cluster of %d CTAs fits", splits);
+        for (int s = kQtMaxSplit; s >= 1; s--) {
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3((unsigned)s);
+            cfg.blockDim = dim3(kQtThreads);
+            cfg.dynamicSmemBytes = kQtOneSmem;
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = (unsigned)s;
+            attr[0].val.clusterDim.y = 1;
+            attr[0].val.clusterDim.z = 1;
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+            f[s] = 0;
+            if (cudaOccupancyMaxActiveClusters(&f[s], gemm_quant_kernel<true>, &cfg) != cudaSuccess) {
+                cudaGetLastError();
+                f[s] = 0;
+            }
+        }
     }
-    *out = f;
+    std::copy(f, f + kQtMaxSplit + 1, fit);
     return JUNO_OK;
 }
 
@@ -525,38 +531,18 @@ int launch_gemm_quant(juno_ctx *c, const GemmQuantArgs &a, cudaStream_t st) {
     p.epi = a.epi;
     p.scale = a.scale;
     p.err = c->gemv_scratch.qerr;
-    // Rows of x per pass over the weights: one pass up to 224 rows, then two, four, ...  With more than 224 only two stages of x fit.  Prompts
-    // of 256 positions in one and in two passes: Llama-3-8B 6.80 and 6.45 ms, TinyLlama Q4_K_M 2.57 and 2.19 ms; of 200: 5.44 and 6.06, 2.23 and
-    // 2.27; three passes or five were slower than two or four everywhere.
-    p.col_blocks = 1;
-    while ((a.n + p.col_blocks - 1) / p.col_blocks > kQtMaxN) p.col_blocks *= 2;
-    p.N = ((a.n + p.col_blocks - 1) / p.col_blocks + 15) / 16 * 16;
-    p.col_blocks = (a.n + p.N - 1) / p.N;
+    QuantSplit q = quant_passes(a.n);
+    p.N = q.N;
+    p.col_blocks = q.col_blocks;
     // half an SM per CTA (the next kernel's copies start while this one ends, and one CTA's exchange hides behind the other's products),
     // as long as the sums and two stages fit half of the tensor memory
     const bool pair = p.N <= 128 && (size_t)p.slot_bytes * 2 * kQtWarps + 2 * (size_t)p.N * 256 + 1024 <= kQtPairSmem;
-    // CTAs that share K: estimated in SM cycles, unpacking or multiplying 128 columns of a piece, whatever takes longer, with both CTAs of
-    // an SM at it, plus what a piece and an exchange cost beside that.  2048 x 5632 Q4_K, 9 rows with 1 / 2 / 3 / 6: 20.2 / 17.2 / 15.7 / 12.6 us;
-    // 28672 x 4096 does not gain from any.
-    double best = 1e30;
-    for (int s = 1; s <= kQtMaxSplit && s <= p.nb; s++) {
-        int n = 0, per = 1;  // clusters; pieces of a cluster
-        JUNO_TRY(qt_clusters(c, s, &n));
-        if (pair) n *= 2;
-        if (s > 1) {  // every cluster one piece
-            n = n / p.col_blocks * p.col_blocks;
-            if (n < p.col_blocks || (rt + n / p.col_blocks - 1) / (n / p.col_blocks) > kQtWarps) continue;
-        }
-        const int share = (int)(((long long)rt * p.col_blocks + n - 1) / n);
-        if (s == 1) per = (share + kQtWarps - 1) / kQtWarps;
-        const double half = std::max(35.0 * std::max((share + per - 1) / per, 4), 4.0 * p.N) * (pair ? 2 : 1);
-        const double cost = per * ((double)((p.nb + s - 1) / s) * 2 * half + 1500) + (s > 1 ? 2000 + 2.0 * p.N * share : 0);
-        if (cost < best) {
-            best = cost;
-            p.splits = s;
-            p.clusters = std::min(n, rt * p.col_blocks);
-        }
-    }
+    int fit[kQtMaxSplit + 1];
+    JUNO_TRY(qt_clusters(c, fit));
+    quant_split(q, rt, p.nb, pair, fit);
+    JUNO_REQUIRE(q.splits > 0, "quantised product: no cluster fits device %d", c->device);
+    p.splits = q.splits;
+    p.clusters = q.clusters;
     const size_t budget = pair ? kQtPairSmem : kQtOneSmem, x_bytes = (size_t)p.N * 256;
     // stages before tiles in flight: as many as the tensor memory holds beside the sums
     p.tmem_cols = pair ? 256 : 512;

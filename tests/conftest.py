@@ -51,7 +51,7 @@ def layout_host():
     import subprocess
     src = os.path.join(ROOT, "tests", "native", "layout_host.cpp")
     so = os.path.join(ROOT, "tests", "native", "liblayout_host.so")
-    deps = [src] + [os.path.join(ROOT, "juno_b200", "csrc", f) for f in ("layout.cuh", "dequant.cuh", "repack.cuh", "qsplit.cuh", "ring.cuh", "row_pow.cuh")]
+    deps = [src] + [os.path.join(ROOT, "juno_b200", "csrc", f) for f in ("layout.cuh", "dequant.cuh", "repack.cuh", "qsplit.cuh", "ring.cuh", "row_pow.cuh", "quant_split.cuh")]
     if not os.path.exists(so) or os.path.getmtime(so) < max(os.path.getmtime(d) for d in deps):
         subprocess.check_call(["g++", "-O2", "-std=c++17", "-ffp-contract=off", "-shared", "-fPIC", "-o", so, src])
     L = C.CDLL(so)

@@ -154,3 +154,13 @@ extern "C" uint32_t row_pow_of(int type, int blocks, const float *factors, const
     }
     return row_pow_word(type, r);
 }
+
+// ── spread of a quantised product over the GPU (quant_split.cuh) ──────────────────────────
+#include "../../juno_b200/csrc/quant_split.cuh"
+
+// out: N, col_blocks, splits, clusters
+extern "C" void quant_split_of(int n, int rt, int nb, int pair, const int *fit, int *out) {
+    QuantSplit q = quant_passes(n);
+    quant_split(q, rt, nb, pair != 0, fit);
+    out[0] = q.N, out[1] = q.col_blocks, out[2] = q.splits, out[3] = q.clusters;
+}

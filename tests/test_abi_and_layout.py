@@ -174,3 +174,25 @@ def test_row_tiles_that_quick_unpacking_would_cost_digits_are_wide(layout_host, 
     inf = np.full(32, np.inf, np.float32)
     inf[1:] = 1.0
     assert L.row_pow_of(t, 16, inf.ctypes.data, np.full(256, 9, np.uint8).ctypes.data) & 0xFFFF == 64 | 64 << 8
+
+
+@pytest.mark.parametrize("missing", [(), (8,), (5, 7, 8), (2, 3, 4, 5, 6, 7, 8), (1, 2, 3, 4, 5, 6, 7, 8)])
+def test_quantised_products_skip_cluster_sizes_that_do_not_fit(layout_host, missing):
+    """The choice of CTAs that share K (csrc/quant_split.cuh) where the device takes some cluster sizes only: another size that fits is taken, for any product;
+    a cluster that shares K has one piece of at most eight row tiles of one column block."""
+    import ctypes as C
+    fit = (C.c_int * 9)(0, *[0 if s in missing else 148 // s for s in range(1, 9)])
+    out = (C.c_int * 4)()
+    for n in (1, 9, 64, 129, 224, 225, 500, 1000):
+        for rt in (1, 2, 7, 64, 128, 160, 384, 1792, 8016):
+            for nb in (1, 2, 8, 16, 56):
+                for pair in (0, 1):
+                    layout_host.quant_split_of(n, rt, nb, pair, fit, out)
+                    N, blocks, splits, clusters = out
+                    assert N % 16 == 0 and 16 <= N <= 224 and (blocks - 1) * N < n <= blocks * N
+                    if len(missing) == 8:
+                        assert splits == 0
+                        continue
+                    assert 1 <= splits <= nb and splits not in missing and 1 <= clusters <= fit[splits] * (1 + pair)
+                    if splits > 1:
+                        assert clusters % blocks == 0 and -(-rt * blocks // clusters) <= 8

@@ -21,6 +21,7 @@
 #include "gemm_rows.cuh"
 #include "model.cuh"
 #include "prompt.cuh"
+#include "quant_split.cuh"
 #include "qgemv.cuh"
 #include "stack.cuh"
 
@@ -920,13 +921,13 @@ static bool prompt_takes(const juno_model *m, int n) {
 // 70 / 200 / 333 / 500 positions 10.3 / 9.8 / 13.5 / 13.8 and 4.2 / 5.5 / 8.6 / 12.9 ms; TinyLlama Q4_K_M 70 / 200 / 333 / 500 positions 2.70 / 3.31 / 3.17 / 3.64 and
 // 1.77 / 2.23 / 2.74 / 3.33 ms, 600 positions 3.39 and 3.59.  Layers with fewer tiles than there are warps to unpack them are all launches: two layers of width 512, 250
 // positions 145 and 165 us (four of width 1024, 2752 tiles each: 381 and 342).
-constexpr int kFusedRows = 512, kFusedTiles = 2368;
+constexpr int kFusedRows = 512;
 static bool prompt_fused(const juno_model *m, int n) {
     if (m->stack || n > kFusedRows) return false;
     int64_t tiles = 0;
     for (const juno_qmat *w : m->layers[0].w)
         if (w) tiles += w->row_tiles * w->nb;
-    return tiles >= kFusedTiles;
+    return tiles >= (int64_t)m->ctx->sm_count * 2 * kQtWarps;  // two CTAs per SM
 }
 
 static void prompt_release_rows(JunoPrompt &P) {

@@ -191,10 +191,12 @@ __device__ __forceinline__ void put_staged(const StageRowsArgs &a, __half *out, 
 }
 
 // One CTA per row.  The row stays in registers between the pass that finds its norm and its largest magnitude and the pass that writes
-// it: read once, written once, bound by memory for many rows and by one round trip for a few.  V: groups of four columns per thread.
+// it: read once, written once, bound by memory for many rows and by one round trip for a few.  V: groups of four columns per thread; 16 of them
+// need 120 registers, one CTA per SM (with the 64 of two, K 28672 spilled 1.5 KB a thread; 9 rows of K 16640 17.0 -> 9.5 to 14.2 us, a layer's row kernels in
+// a prompt of 2000 positions 188 -> 182; the kernel below 12.9 to 18.8 and 226).
 constexpr int kStageThreads = 512, kStageCols = kStageThreads * 4;
 template <int V>
-__global__ void __launch_bounds__(kStageThreads, V <= 4 ? 3 : 2) stage_rows_kernel(const StageRowsArgs a) {
+__global__ void __launch_bounds__(kStageThreads, V <= 4 ? 3 : V <= 8 ? 2 : 1) stage_rows_kernel(const StageRowsArgs a) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, K = a.K;
     const size_t row = blockIdx.x;
     constexpr int kWarps = kStageThreads / 32;

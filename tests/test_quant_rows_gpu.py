@@ -186,3 +186,48 @@ def test_prompts_round_weights_once(ctx, oracle, t, minimum, ratio):
     ref = res / np.sqrt((res * res).mean(1, keepdims=True)) * on @ (head / 64.0).T
     err = np.linalg.norm(got - ref) / np.linalg.norm(ref)
     assert err < 6e-5, err
+
+
+@pytest.mark.parametrize("cols", [16384, 16640, 28672, 32768, 33024])
+def test_long_rows(mv, oracle, cols):
+    """Rows of x on both sides of the widths that staging keeps in registers, one CTA per SM or two, and of those that it reads twice."""
+    rng = np.random.default_rng(cols)
+    raw = synth.random_blocks(rng, synth.Q4_K, 40, cols)
+    x = rng.standard_normal((9, cols)).astype(np.float32) * (2.0 ** np.arange(-12, 15, 3, dtype=np.float32))[:, None]
+    A = mv.upload_quantized(raw, synth.Q4_K, 40, cols)
+    y, ref = mv.sgemv(A, x), oracle.matvec(synth.Q4_K, raw, x, 40, cols)
+    assert max(rel_err(a, b) for a, b in zip(y, ref)) < 1e-3
+    A.close()
+
+
+@pytest.mark.parametrize("hidden", [16640, 33024])
+def test_long_rows_with_norms_and_addends(ctx, oracle, hidden):
+    """The same inside a model, whose rows are summed, stored and normed on their way to FP16: nine requests at their first position, the attention adds zero."""
+    from juno_b200.handler import B200TransformerHandler
+    arch = synth.Arch(hidden, 1, hidden // 128, hidden // 256, 256, 64, 1e-5, 10000.0)
+    rng = np.random.default_rng(hidden)
+    shapes = {k: synth.tensor_shape(arch, k) for k in (synth.T_TOKEN_EMBD, synth.T_OUTPUT, synth.T_ATTN_Q, synth.T_ATTN_K, synth.T_ATTN_V, synth.T_ATTN_OUT,
+                                                       synth.T_FFN_GATE, synth.T_FFN_UP, synth.T_FFN_DOWN)}
+
+    def tensors():
+        for k, (rows, cols) in shapes.items():
+            if k in (synth.T_ATTN_Q, synth.T_ATTN_K, synth.T_ATTN_V, synth.T_ATTN_OUT):
+                yield k, 0, synth.Q4_K, rows, cols, np.zeros(rows * cols // 256 * 144, np.uint8)
+            else:
+                yield from tame([(k, 0, synth.Q8_0, rows, cols, synth.random_blocks(rng, synth.Q8_0, rows, cols))])
+        for k in (synth.T_OUTPUT_NORM, synth.T_ATTN_NORM, synth.T_FFN_NORM):
+            yield k, 0, synth.F32, 1, hidden, (1 + 0.3 * rng.standard_normal(hidden)).astype(np.float32).view(np.uint8)
+
+    w = {(k, t): raw for k, _, t, _, _, raw in tensors()}
+    h = B200TransformerHandler(arch, ctx, max_batch=16, max_seqs=16, max_ctx=16)
+    h.load((k, 0, t, *(shapes[k] if t != synth.F32 else (1, hidden)), raw) for (k, t), raw in w.items())
+    got = h.forward_batch(["r%d" % i for i in range(9)], [[5 * i] for i in range(9)], [0] * 9)
+    h.release_gpu_resources()
+    emb, head, gate, up, down = (oracle.dequantize(synth.Q8_0, w[k, synth.Q8_0], *shapes[k]).reshape(shapes[k]).astype(np.float64)
+                                 for k in (synth.T_TOKEN_EMBD, synth.T_OUTPUT, synth.T_FFN_GATE, synth.T_FFN_UP, synth.T_FFN_DOWN))
+    normed = lambda v, k: v / np.sqrt((v * v).mean(1, keepdims=True) + arch.rms_eps) * w[k, synth.F32].view(np.float32)
+    x = emb[5 * np.arange(9)]
+    g = normed(x, synth.T_FFN_NORM) @ gate.T
+    x = x + g / (1 + np.exp(-g)) * (normed(x, synth.T_FFN_NORM) @ up.T) @ down.T
+    ref = normed(x, synth.T_OUTPUT_NORM) @ head.T
+    assert max(rel_err(a, b) for a, b in zip(got, ref)) < TOL

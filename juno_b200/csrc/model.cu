@@ -786,27 +786,30 @@ extern "C" int juno_model_finalize(juno_model *m) {
 namespace juno {
 
 // ───────────────────────────── one decode step, enqueued on the context stream ────────────
-// Product of matrices that share the staged rows x [n][K].
+// Product of matrices that share the staged rows x [n][K]: one launch, or with JUNO_NO_MIXED one per block format.
 static int quant_group(juno_model *m, juno_qmat *const *mats, float *const *outs, int count, int epi, int n, const void *x, const float *scale, int ld_out,
                        cudaStream_t st, bool precise = false) {
-    GemmQuantArgs a;
-    a.nseg = count;
-    for (int s = 0; s < count; s++) {
-        a.seg[s].w = mats[s]->dev;
-        a.seg[s].out = outs[s];
-        a.seg[s].rows = epi == EPI_SILU_PAIR ? (int)mats[s]->rows / 2 : (int)mats[s]->rows;
-        a.seg[s].row_tiles = (int)mats[s]->row_tiles;
-        a.seg[s].type = mats[s]->type;
-        a.seg[s].row_pow = mats[s]->row_pow;
+    for (int i = 0; i < count;) {
+        GemmQuantArgs a;
+        for (a.nseg = 0; i < count && (a.nseg == 0 || m->mix_formats || mats[i]->type == a.seg[0].type); i++) {
+            GemvSeg &g = a.seg[a.nseg++];
+            g.w = mats[i]->dev;
+            g.out = outs[i];
+            g.rows = epi == EPI_SILU_PAIR ? (int)mats[i]->rows / 2 : (int)mats[i]->rows;
+            g.row_tiles = (int)mats[i]->row_tiles;
+            g.type = mats[i]->type;
+            g.row_pow = mats[i]->row_pow;
+        }
+        a.K = (int)mats[0]->cols;
+        a.n = n;
+        a.x = x;
+        a.scale = scale;
+        a.ld_out = ld_out;
+        a.epi = epi;
+        a.precise = precise;
+        JUNO_TRY(launch_gemm_quant(m->ctx, a, st));
     }
-    a.K = (int)mats[0]->cols;
-    a.n = n;
-    a.x = x;
-    a.scale = scale;
-    a.ld_out = ld_out;
-    a.epi = epi;
-    a.precise = precise;
-    return launch_gemm_quant(m->ctx, a, st);
+    return JUNO_OK;
 }
 
 // Layers and output projection of one step on the batched path (n >= gemm_min_batch()): every product is ONE pass

@@ -4,8 +4,9 @@ import pytest
 
 from conftest import rel_err
 from juno_b200 import synth
-from juno_b200.handler import B200InferencePipeline, ForwardRequest, generate_greedy
+from juno_b200.handler import B200InferencePipeline, B200TransformerHandler, ForwardRequest, generate_greedy
 from modelutil import SMALL128, TINY, build_pair
+from test_prompt_gpu import tame
 
 pytestmark = pytest.mark.gpu
 TOL = 1e-3
@@ -270,6 +271,28 @@ def test_batched_tcgen05_route_in_a_forward_pass(ctx, oracle):
     # FP16 operands on this path: about 1e-3 on most sequences, a few amplified by the random-init model
     assert float(np.median(errs)) < 2e-3 and errs[int(0.9 * n)] < 2e-2, (float(np.median(errs)), errs[-4:])
     h.release_gpu_resources()
+
+
+@pytest.mark.parametrize("n", [4, 12, 40])
+def test_one_launch_per_block_format_on_request(ctx, monkeypatch, n):
+    """JUNO_NO_MIXED=1: V (Q6_K) apart from Q and K (Q4_K), in the exact and in the batched products, with the same results."""
+    def step():
+        h = B200TransformerHandler(SMALL128, ctx, max_batch=64, max_seqs=n, max_ctx=16)
+        h.load(tame(synth.random_model(SMALL128, 43)))
+        ctx.profile(True)
+        ctx.profile_read()
+        logits = h.forward_batch([f"s{i}" for i in range(n)], [[7 * i] for i in range(n)], [0] * n)
+        prof = ctx.profile_read()
+        ctx.profile(False)
+        h.release_gpu_resources()
+        return logits, prof["gemv_q4k"]["launches"], prof["gemv_q6k"]["launches"]
+
+    monkeypatch.delenv("JUNO_NO_MIXED", raising=False)
+    mixed, q4, q6 = step()
+    monkeypatch.setenv("JUNO_NO_MIXED", "1")
+    apart, q4_apart, q6_apart = step()
+    assert rel_err(apart, mixed) < 1e-3  # K may be split otherwise: sums in another order, and a few values that round to another FP16 number after them
+    assert (q4_apart, q6_apart) == (q4, q6 + SMALL128.n_layers)
 
 
 @pytest.mark.parametrize("n_seq", [16, 64])

@@ -43,36 +43,15 @@ struct GemmQuantParams {
     const uint32_t *pow[3];  // powers of two of the rows
     float *out[3];
     int rows[3], type[3], rt_begin[4];
-    int total_rt, nb, n, N, col_blocks;  // N: rows of x per pass, a multiple of 16
-    int ld_out, epi, splits, clusters;
+    QuantShares shares;
+    EvenShares blocks;       // 256-column blocks over the CTAs of a cluster
+    int nb, n, N;  // N: rows of x per pass, a multiple of 16
+    int ld_out, epi, splits;
     int ring, slot_bytes, stages, tmem_cols;
     const float *scale;
     unsigned *err;
 };
 
-// A cluster's share of the (column block, row tile) pairs, in pieces of up to eight row tiles of one column block.
-struct QtWalk {
-    int f, end;        // flat index of the piece's first row tile; end of the share
-    int block, lo, r;  // column block, first row tile, row tiles of the piece
-};
-__device__ __forceinline__ void qt_piece(QtWalk &w, int total_rt) {
-    w.block = w.f / total_rt;
-    w.lo = w.f - w.block * total_rt;
-    const int rem = min(w.end, (w.block + 1) * total_rt) - w.f, k = (rem + kQtWarps - 1) / kQtWarps;
-    w.r = k > 0 ? (rem + k - 1) / k : 0;
-}
-__device__ __forceinline__ QtWalk qt_begin(const GemmQuantParams &p, int cluster) {
-    const long long total = (long long)p.col_blocks * p.total_rt;
-    QtWalk w;
-    w.f = (int)(total * cluster / p.clusters);
-    w.end = (int)(total * (cluster + 1) / p.clusters);
-    qt_piece(w, p.total_rt);
-    return w;
-}
-__device__ __forceinline__ void qt_next(QtWalk &w, int total_rt) {
-    w.f += w.r;
-    qt_piece(w, total_rt);
-}
 __device__ __forceinline__ int qt_seg(const GemmQuantParams &p, int rt) { return rt >= p.rt_begin[2] ? 2 : rt >= p.rt_begin[1] ? 1 : 0; }
 
 __device__ __forceinline__ void mma_f16_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
@@ -127,15 +106,15 @@ struct QtTiles {
     unsigned bytes;
     int sb, owner, s0, nb, issued;
     __device__ __forceinline__ void seek(const GemmQuantParams &p) {  // first piece from here on in which the warp has a row tile
-        while (w.r > 0 && owner >= w.r) qt_next(w, p.total_rt);
+        while (w.r > 0 && owner >= w.r) qt_next(w, p.shares.total_rt);
         if (w.r <= 0) return;
         const int rt = w.lo + owner, s = qt_seg(p, rt);
         bytes = (unsigned)tile_bytes(p.type[s]);
         src = p.w[s] + ((size_t)(rt - p.rt_begin[s]) * p.nb + s0) * bytes;
         sb = 0;
     }
-    __device__ __forceinline__ void init(const GemmQuantParams &p, int warp, int cluster, int first, int count) {
-        w = qt_begin(p, cluster);
+    __device__ __forceinline__ void init(const GemmQuantParams &p, int warp, const QtWalk &begin, int first, int count) {
+        w = begin;
         owner = warp;
         s0 = first;
         nb = count;
@@ -148,7 +127,7 @@ struct QtTiles {
         issued++;
         src += bytes;
         if (++sb == nb) {
-            qt_next(w, p.total_rt);
+            qt_next(w, p.shares.total_rt);
             seek(p);
         }
     }
@@ -201,6 +180,18 @@ __device__ __forceinline__ void qt_unpack(QtUnpack &u, const RowPow &P, int nb, 
     }
 }
 
+// Read again where they are used: kept, they would cost the unpacking warps registers.
+__device__ __forceinline__ int cluster_rank() {
+    int r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ int cluster_id() {
+    int r;
+    asm volatile("mov.u32 %0, %%clusterid.x;" : "=r"(r));
+    return r;
+}
+
 template <bool PRECISE>
 __global__ void __launch_bounds__((kQtWarps + 4) * 32, 2) gemm_quant_kernel(const __grid_constant__ GemmQuantParams p) {
     extern __shared__ uint8_t smem_raw[];
@@ -209,18 +200,30 @@ __global__ void __launch_bounds__((kQtWarps + 4) * 32, 2) gemm_quant_kernel(cons
     __shared__ uint32_t tmem_slot;
     __shared__ unsigned fail_s;
     __shared__ int issued_s[kQtWarps + 1];  // copies into each ring, and into the stages of x
-    __shared__ QtTiles tiles_s[kQtWarps];  // not in registers: only the copying warp needs them
+    // not in registers while tiles are unpacked: where the copying warp is, and the piece of every unpacking warp
+    __shared__ QtTiles tiles_s[kQtWarps];
+    __shared__ QtWalk walk_s[kQtWarps];
     volatile unsigned *fail = &fail_s;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int rank = (int)(blockIdx.x % (unsigned)p.splits), cluster = (int)(blockIdx.x / (unsigned)p.splits);
-    const int s0 = p.nb * rank / p.splits, nb = p.nb * (rank + 1) / p.splits - s0;  // this CTA's 256-column blocks
+    const int s0 = p.blocks.begin(cluster_rank()), nb = p.blocks.begin(cluster_rank() + 1) - s0;  // this CTA's 256-column blocks
     const uint32_t x0 = (s_u32(smem_raw) + 1023u) & ~1023u, x_bytes = (uint32_t)p.N * 256u;  // 128 columns of x: two boxes of 64
     // whose tiles: an unpacking warp's own; lane w of the copying warp sees to those of warp w
     const int owner = warp < kQtWarps ? warp : lane & (kQtWarps - 1);
     const uint32_t ring = x0 + (uint32_t)p.stages * x_bytes + (uint32_t)(owner * p.ring * p.slot_bytes);
     const uint32_t tile_bar = s_u32(bars) + (uint32_t)(owner * kQtMaxRing) * 8u, tile_free = tile_bar + kQtWarps * kQtMaxRing * 8, full = s_u32(bars) + 2 * kQtWarps * kQtMaxRing * 8, free = full + kQtMaxStages * 8,
                    acc_full = free + kQtMaxStages * 8, acc_free = acc_full + 8;
+    // Before the CTA meets, every warp finds its first piece, an unpacking warp also the powers of two of its rows there: divisions and a load from
+    // memory that would follow one another behind the dependency wait otherwise.
+    QtWalk w;
+    RowPow P{{0u, 0u}};
+    auto load_pow = [&]() {
+        const int rt = w.lo + warp, seg = qt_seg(p, rt);
+        const uint32_t *pow = p.pow[seg] + (rt - p.rt_begin[seg]) * 16 + (lane >> 2);
+        P.w[0] = __ldg(pow);
+        P.w[1] = __ldg(pow + 8);
+    };
     if (warp == kQtWarps + 2) {
+        if (lane == 0) fail_s = 0;
         if (lane < kQtWarps) {
             for (int i = 0; i < p.ring; i++) {
                 mbar_init(tile_bar + i * 8, 1);
@@ -229,7 +232,7 @@ __global__ void __launch_bounds__((kQtWarps + 4) * 32, 2) gemm_quant_kernel(cons
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
             asm volatile("fence.proxy.async;" ::: "memory");
             QtTiles t;
-            t.init(p, owner, cluster, s0, nb);
+            t.init(p, owner, qt_begin(p.shares, cluster_id()), s0, nb);
             for (int i = 0; i < p.ring && t.w.r > 0; i++) t.fetch(p, tile_bar + i * 8, ring + i * p.slot_bytes);
             tiles_s[owner] = t;
         }
@@ -243,13 +246,17 @@ __global__ void __launch_bounds__((kQtWarps + 4) * 32, 2) gemm_quant_kernel(cons
             }
             mbar_init(acc_full, 1);
             mbar_init(acc_free, kQtWarps);
-            fail_s = 0;
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
+        w = qt_begin(p.shares, cluster_id());
         __syncwarp();
     } else if (warp == kQtWarps + 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s_u32(&tmem_slot)), "r"(p.tmem_cols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        w = qt_begin(p.shares, cluster_id());
+    } else {
+        w = qt_begin(p.shares, cluster_id());
+        if (warp < w.r) load_pow();
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -261,22 +268,22 @@ __global__ void __launch_bounds__((kQtWarps + 4) * 32, 2) gemm_quant_kernel(cons
         QtUnpack u{ring, tile_bar, tile_free, full, free, tmem_a + lanes, p.ring, p.slot_bytes, p.stages, 0, 0, 0u, 0u};
         unsigned accpar = 0;
         bool waited = false;
-        for (QtWalk w = qt_begin(p, cluster); w.r > 0; qt_next(w, p.total_rt)) {
-            const bool active = warp < w.r;
-            const int rt = w.lo + warp, seg = active ? qt_seg(p, rt) : 0, type = p.type[seg];
-            RowPow P;
-            if (active) P = row_pow_load(p.pow[seg], (rt - p.rt_begin[seg]) * 16 + g, type, PRECISE);
-            if (!active)
+        while (w.r > 0) {
+            const int type = warp < w.r ? p.type[qt_seg(p, w.lo + warp)] : 0;
+            const bool wide = P.wide(type, PRECISE);
+            if (lane == 0) walk_s[warp] = w;
+            __syncwarp();
+            if (type == 0)
                 qt_unpack<0, false>(u, P, nb, fail);
-            else if (type == 12 && (PRECISE || P.wide))
+            else if (type == 12 && (PRECISE || wide))
                 qt_unpack<12, true>(u, P, nb, fail);
             else if (type == 12)
                 qt_unpack<12, PRECISE>(u, P, nb, fail);
-            else if (type == 14 && (PRECISE || P.wide))
+            else if (type == 14 && (PRECISE || wide))
                 qt_unpack<14, true>(u, P, nb, fail);
             else if (type == 14)
                 qt_unpack<14, PRECISE>(u, P, nb, fail);
-            else if (P.wide)
+            else if (wide)
                 qt_unpack<8, true>(u, P, nb, fail);
             else
                 qt_unpack<8, false>(u, P, nb, fail);
@@ -284,14 +291,19 @@ __global__ void __launch_bounds__((kQtWarps + 4) * 32, 2) gemm_quant_kernel(cons
                 pdl_wait();
                 waited = true;
             }
+            {
+                const volatile QtWalk &v = walk_s[warp];
+                w = QtWalk{v.f, v.end, v.block, v.lo, v.r};
+            }
             asm volatile("prefetch.global.L1 [%0];" ::"l"(p.scale + min(w.block * p.N + lane * 8, p.n - 1)));
             bar_wait(acc_full, accpar, fail);
             accpar ^= 1u;
             __syncwarp();
-            if (active) {
+            if (warp < w.r) {
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const int col0 = w.block * p.N, cols = min(p.N, p.n - col0);
-                const float undo0 = P.undo[0], undo1 = P.undo[1];
+                const int col0 = w.block * p.N, cols = min(p.N, p.n - col0), rt = w.lo + warp, seg = qt_seg(p, rt);
+                const bool wide = P.wide(p.type[seg], PRECISE);
+                const float undo0 = P.undo(0, wide), undo1 = P.undo(1, wide);
 #pragma unroll 1
                 for (int c = 0; c < cols; c += 16) {
                     uint32_t r[8];
@@ -325,6 +337,8 @@ __global__ void __launch_bounds__((kQtWarps + 4) * 32, 2) gemm_quant_kernel(cons
             }
             __syncwarp();
             if (lane == 0) qt_arrive(acc_free);
+            qt_next(w, p.shares.total_rt);
+            if (warp < w.r) load_pow();
         }
     } else if (warp == kQtWarps) {
         pdl_wait();
@@ -333,7 +347,7 @@ __global__ void __launch_bounds__((kQtWarps + 4) * 32, 2) gemm_quant_kernel(cons
             int s = 0, issued = 0;
             unsigned par = 0;
             bool ok = true;
-            for (QtWalk w = qt_begin(p, cluster); ok && w.r > 0; qt_next(w, p.total_rt))
+            for (; ok && w.r > 0; qt_next(w, p.shares.total_rt))
                 for (int k = 0; k < 2 * nb; k++) {
                     if (!(ok = bar_wait(free + s * 8, par ^ 1u, fail))) break;
                     mbar_expect_tx(full + s * 8, x_bytes);
@@ -356,7 +370,7 @@ __global__ void __launch_bounds__((kQtWarps + 4) * 32, 2) gemm_quant_kernel(cons
         int s = 0;
         unsigned par = 0, accpar = 0;
         bool ok = true;
-        for (QtWalk w = qt_begin(p, cluster); w.r > 0; qt_next(w, p.total_rt)) {
+        for (; w.r > 0; qt_next(w, p.shares.total_rt)) {
             ok = bar_wait(acc_free, accpar ^ 1u, fail) && ok;
             accpar ^= 1u;
             for (int k = 0; k < 2 * nb; k++) {
@@ -426,32 +440,32 @@ __global__ void __launch_bounds__((kQtWarps + 4) * 32, 2) gemm_quant_kernel(cons
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(p.tmem_cols) : "memory");
     }
     if (p.splits == 1) return;
+    // a cluster that shares K has one piece; four outputs at a time, a contiguous range of them per CTA
+    w = qt_begin(p.shares, cluster_id());
+    const int sh = p.epi == EPI_SILU_PAIR ? 1 : 2, col0 = w.block * p.N, per = w.r << sh, total = per * min(p.N, p.n - col0), chunk = (total + p.splits - 1) / p.splits;
+    const int first = cluster_rank() * chunk, last = min(total, first + chunk);
     __syncwarp();
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-    {
-        const QtWalk w = qt_begin(p, cluster);  // a cluster that shares K has one piece
-        const int quads = p.epi == EPI_SILU_PAIR ? 2 : 4, col0 = w.block * p.N, cols = min(p.N, p.n - col0), per = w.r * quads, total = per * cols;
-        for (int idx = (int)((long long)total * rank / p.splits) + tid; idx < (int)((long long)total * (rank + 1) / p.splits); idx += kQtThreads) {
-            const int c = idx / per, q = idx - c * per, l = q / quads, row = (q - l * quads) * 4, rt = w.lo + l, seg = qt_seg(p, rt);
-            const int orow = (rt - p.rt_begin[seg]) * quads * 4 + row, b = col0 + c;
-            const uint32_t at = x0 + (uint32_t)(c * kQtLd + l * 16 + row) * 4;
-            const float sc = p.scale[b];
-            float4 v = qt_peer_sum(at, p.splits);
-            v = make_float4(v.x * sc, v.y * sc, v.z * sc, v.w * sc);
-            if (p.epi == EPI_SILU_PAIR) {  // rows 0-7 of a tile are gate rows, rows 8-15 the matching up rows
-                const float4 u = qt_peer_sum(at + 32, p.splits);
-                v = make_float4(__fmul_rn(silu_ref(v.x), u.x * sc), __fmul_rn(silu_ref(v.y), u.y * sc), __fmul_rn(silu_ref(v.z), u.z * sc), __fmul_rn(silu_ref(v.w), u.w * sc));
-            }
-            float *o = p.out[seg] + (size_t)b * p.ld_out + orow;
-            if (orow + 3 < p.rows[seg] && (reinterpret_cast<uintptr_t>(o) & 15) == 0) {
-                *reinterpret_cast<float4 *>(o) = v;
-            } else {
-                const float e[4] = {v.x, v.y, v.z, v.w};
+    for (int idx = first + tid; idx < last; idx += kQtThreads) {
+        const int c = idx / per, q = idx - c * per, l = q >> sh, row = (q - (l << sh)) * 4, rt = w.lo + l, seg = qt_seg(p, rt);
+        const int orow = ((rt - p.rt_begin[seg]) << (sh + 2)) + row, b = col0 + c;
+        const uint32_t at = x0 + (uint32_t)(c * kQtLd + l * 16 + row) * 4;
+        const float sc = p.scale[b];
+        float4 v = qt_peer_sum(at, p.splits);
+        v = make_float4(v.x * sc, v.y * sc, v.z * sc, v.w * sc);
+        if (p.epi == EPI_SILU_PAIR) {  // rows 0-7 of a tile are gate rows, rows 8-15 the matching up rows
+            const float4 u = qt_peer_sum(at + 32, p.splits);
+            v = make_float4(__fmul_rn(silu_ref(v.x), u.x * sc), __fmul_rn(silu_ref(v.y), u.y * sc), __fmul_rn(silu_ref(v.z), u.z * sc), __fmul_rn(silu_ref(v.w), u.w * sc));
+        }
+        float *o = p.out[seg] + (size_t)b * p.ld_out + orow;
+        if (orow + 3 < p.rows[seg] && (reinterpret_cast<uintptr_t>(o) & 15) == 0) {
+            *reinterpret_cast<float4 *>(o) = v;
+        } else {
+            const float e[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-                for (int k = 0; k < 4; k++)
-                    if (orow + k < p.rows[seg]) o[k] = e[k];
-            }
+            for (int k = 0; k < 4; k++)
+                if (orow + k < p.rows[seg]) o[k] = e[k];
         }
     }
     __syncwarp();
@@ -524,7 +538,6 @@ int launch_gemm_quant(juno_ctx *c, const GemmQuantArgs &a, cudaStream_t st) {
         algo += (double)g.rows * a.K * bpw * (a.epi == EPI_SILU_PAIR ? 2 : 1) + (double)a.n * g.rows * 4;
     }
     for (int s = a.nseg; s < 4; s++) p.rt_begin[s] = s < 3 ? 0x7fffffff : rt;
-    p.total_rt = rt;
     p.nb = a.K / 256;
     p.n = a.n;
     p.ld_out = a.ld_out;
@@ -533,7 +546,6 @@ int launch_gemm_quant(juno_ctx *c, const GemmQuantArgs &a, cudaStream_t st) {
     p.err = c->gemv_scratch.qerr;
     QuantSplit q = quant_passes(a.n);
     p.N = q.N;
-    p.col_blocks = q.col_blocks;
     // half an SM per CTA (the next kernel's copies start while this one ends, and one CTA's exchange hides behind the other's products),
     // as long as the sums and two stages fit half of the tensor memory
     const bool pair = p.N <= 128 && (size_t)p.slot_bytes * 2 * kQtWarps + 2 * (size_t)p.N * 256 + 1024 <= kQtPairSmem;
@@ -542,7 +554,8 @@ int launch_gemm_quant(juno_ctx *c, const GemmQuantArgs &a, cudaStream_t st) {
     quant_split(q, rt, p.nb, pair, fit);
     JUNO_REQUIRE(q.splits > 0, "quantised product: no cluster fits device %d", c->device);
     p.splits = q.splits;
-    p.clusters = q.clusters;
+    p.shares = quant_shares(q, rt);
+    p.blocks = even_shares(p.nb, q.splits);
     const size_t budget = pair ? kQtPairSmem : kQtOneSmem, x_bytes = (size_t)p.N * 256;
     // stages before tiles in flight: as many as the tensor memory holds beside the sums
     p.tmem_cols = pair ? 256 : 512;
@@ -557,7 +570,7 @@ int launch_gemm_quant(juno_ctx *c, const GemmQuantArgs &a, cudaStream_t st) {
     JUNO_TRY(tensor_map_bf16(&p.tx, a.x, a.n, a.K, a.K, p.N));
     ProfScope prof(c, st, first_type == 12 ? PROF_GEMV_Q4K : first_type == 14 ? PROF_GEMV_Q6K : PROF_GEMV_Q80, algo), prof_tc(c, st, PROF_GEMM_TC, algo);
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(p.clusters * p.splits));
+    cfg.gridDim = dim3((unsigned)(q.clusters * q.splits));
     cfg.blockDim = dim3(kQtThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;

@@ -59,26 +59,33 @@ __device__ __forceinline__ uint32_t fma_f16(uint32_t v, float s, float c) {
 struct TileFactors {
     uint32_t f[12];
 };
-// What a lane knows of rows g and g + 8: the row's power of two, for FP16 arithmetic as two factors (their product may exceed FP16, second one 1
-// for a wide tile of Q4_K or Q6_K, whose first one is FP32), and what the product has to be multiplied with.
+// The words of rows g and g + 8 (row_pow.cuh): all that a lane keeps of their powers of two while it goes through a row tile.
 struct RowPow {
-    uint32_t a[2], b[2];
-    float undo[2];
-    bool wide;
-};
-__device__ __forceinline__ RowPow row_pow_load(const uint32_t *pow, int row, int type, bool precise) {
-    RowPow P;
-#pragma unroll
-    for (int k = 0; k < 2; k++) {
-        const uint32_t w = __ldg(pow + row + 8 * k);
-        P.wide = (w & kRowWide) != 0 || (precise && type != 8);
-        const int e = (int)(P.wide ? w >> 8 & 0xFFu : w & 0xFFu) - kRowPowBias, first = min(e, 15);
-        P.undo[k] = __uint_as_float((uint32_t)(127 + (P.wide ? 0 : 24) - e) << 23);
-        P.a[k] = P.wide && type != 8 ? (uint32_t)(127 + e) << 23 : (uint32_t)(15 + first) * 0x04000400u;
-        P.b[k] = (uint32_t)(15 + e - first) * 0x04000400u;
+    uint32_t w[2];
+    __device__ __forceinline__ bool wide(int type, bool precise) const { return (w[0] & kRowWide) != 0 || (precise && type != 8); }
+    // What the product has to be multiplied with.
+    __device__ __forceinline__ float undo(int k, bool wide) const {
+        return __uint_as_float((uint32_t)(127 + kRowPowBias + (wide ? 0 : 24) - (int)(wide ? w[k] >> 8 & 0xFFu : w[k] & 0xFFu)) << 23);
     }
-    return P;
-}
+    // The exponent, from the word anew for every tile: kept, what follows from it would cost registers.
+    template <bool WIDE>
+    __device__ __forceinline__ int exponent(int k) const {
+        uint32_t v = w[k];
+        asm volatile("" : "+r"(v));
+        return (int)(WIDE ? v >> 8 & 0xFFu : v & 0xFFu) - kRowPowBias;
+    }
+    template <bool WIDE>
+    __device__ __forceinline__ float f32(int k) const {
+        return __uint_as_float((uint32_t)(127 + exponent<WIDE>(k)) << 23);
+    }
+    // As two FP16 factors: their product may exceed FP16.
+    template <bool WIDE>
+    __device__ __forceinline__ void f16(int k, uint32_t &a, uint32_t &b) const {
+        const int e = exponent<WIDE>(k), first = min(e, 15);
+        a = (uint32_t)(15 + first) * 0x04000400u;
+        b = (uint32_t)(15 + e - first) * 0x04000400u;
+    }
+};
 // Byte K of w in both halves, under the high byte of hi.
 template <int K>
 __device__ __forceinline__ uint32_t byte_h2(uint32_t w, uint32_t hi) {
@@ -92,7 +99,9 @@ __device__ __forceinline__ void q4_factors(TileFactors &F, const RowPow &P, uint
     F.f[0] = a.x, F.f[1] = a.y, F.f[2] = a.z, F.f[3] = a.w, F.f[4] = b.x, F.f[5] = b.y, F.f[6] = b.z, F.f[7] = b.w;
 #pragma unroll
     for (int k = 0; k < 2; k++) {
-        const uint32_t d = h2_mul(h2_mul(lds32(tile + 32 * k + (lane >> 2) * 4), P.a[k]), P.b[k]);  // d | dmin
+        uint32_t pa, pb;
+        P.f16<false>(k, pa, pb);
+        const uint32_t d = h2_mul(h2_mul(lds32(tile + 32 * k + (lane >> 2) * 4), pa), pb);  // d | dmin
         F.f[8 + k] = __byte_perm(d, 0, 0x1010);
         F.f[10 + k] = __byte_perm(d, 0, 0x3232) ^ 0x80008000u;
     }
@@ -129,7 +138,7 @@ __device__ __forceinline__ void q4_wide_factors(TileFactors &F, const RowPow &P,
 #pragma unroll
     for (int k = 0; k < 2; k++) {
         const uint32_t d = lds32(tile + 32 * k + (lane >> 2) * 4);  // d | dmin
-        const float p = __uint_as_float(P.a[k]);
+        const float p = P.f32<true>(k);
         F.f[8 + k] = __float_as_uint(low_f32(d) * p * kTo24 * kTo24);  // for a scale byte and a field in units of 2^-24 each
         F.f[10 + k] = __float_as_uint(high_f32(d) * p * -kTo24);
     }
@@ -165,7 +174,11 @@ __device__ __forceinline__ void q6_factors(TileFactors &F, const RowPow &P, uint
     const uint4 a = lds128(row), b = lds128(row + 128);  // the 16 signed scales
     F.f[0] = a.x, F.f[1] = a.y, F.f[2] = a.z, F.f[3] = a.w, F.f[4] = b.x, F.f[5] = b.y, F.f[6] = b.z, F.f[7] = b.w;
 #pragma unroll
-    for (int k = 0; k < 2; k++) F.f[8 + k] = h2_mul(h2_mul(lds16(tile + 3328 + 16 * k + (lane >> 2) * 2) * 0x10001u, P.a[k]), P.b[k]);
+    for (int k = 0; k < 2; k++) {
+        uint32_t pa, pb;
+        P.f16<false>(k, pa, pb);
+        F.f[8 + k] = h2_mul(h2_mul(lds16(tile + 3328 + 16 * k + (lane >> 2) * 2) * 0x10001u, pa), pb);
+    }
 }
 // Four 6-bit values (q + 32) per word, for sub-blocks 4m + 0..3 of quarter m; their bytes hold columns 4t + 0, 2, 1, 3.
 __device__ __forceinline__ void q6_words(const uint4 &ql, const uint4 &qh, int q, int row, uint32_t NIB, uint32_t HI, uint32_t (&V)[4]) {
@@ -205,7 +218,7 @@ __device__ __forceinline__ void q6_wide_factors(TileFactors &F, const RowPow &P,
     const uint4 a = lds128(row), b = lds128(row + 128);
     F.f[0] = a.x, F.f[1] = a.y, F.f[2] = a.z, F.f[3] = a.w, F.f[4] = b.x, F.f[5] = b.y, F.f[6] = b.z, F.f[7] = b.w;
 #pragma unroll
-    for (int k = 0; k < 2; k++) F.f[8 + k] = __float_as_uint(low_f32(lds16(tile + 3328 + 16 * k + (lane >> 2) * 2)) * __uint_as_float(P.a[k]) * kTo24);
+    for (int k = 0; k < 2; k++) F.f[8 + k] = __float_as_uint(low_f32(lds16(tile + 3328 + 16 * k + (lane >> 2) * 2)) * P.f32<true>(k) * kTo24);
 }
 __device__ __forceinline__ void q6_half_wide(const TileFactors &F, uint32_t tile, int half, int lane, uint32_t (&o)[32]) {
     uint32_t NIB = 0x0F0F0F0Fu, HI = 0x30303030u;
@@ -234,11 +247,17 @@ __device__ __forceinline__ void q6_half_wide(const TileFactors &F, uint32_t tile
 }
 
 // ── Q8_0 ────────────────────────────────────────────────────────────────────────────────────
+template <bool WIDE>
 __device__ __forceinline__ void q8_factors(TileFactors &F, const RowPow &P, uint32_t tile, int lane) {
     const uint4 r = lds128(tile + 4096 + (lane >> 2) * 16), q = lds128(tile + 4224 + (lane >> 2) * 16);
     const uint32_t d[8] = {r.x, r.y, r.z, r.w, q.x, q.y, q.z, q.w};  // two blocks' d each
 #pragma unroll
-    for (int k = 0; k < 8; k++) F.f[k] = h2_mul(h2_mul(d[k], P.a[k >> 2]), P.b[k >> 2]);
+    for (int row = 0; row < 2; row++) {
+        uint32_t pa, pb;
+        P.f16<WIDE>(row, pa, pb);
+#pragma unroll
+        for (int k = 4 * row; k < 4 * row + 4; k++) F.f[k] = h2_mul(h2_mul(d[k], pa), pb);
+    }
 }
 template <bool WIDE>
 __device__ __forceinline__ void q8_half_f16(const TileFactors &F, uint32_t tile, int half, int lane, uint32_t (&o)[32]) {
@@ -270,7 +289,7 @@ __device__ __forceinline__ void q8_half_f16(const TileFactors &F, uint32_t tile,
 template <int TYPE, bool WIDE>
 __device__ __forceinline__ void tile_factors_f16(TileFactors &F, const RowPow &P, uint32_t tile, int lane) {
     if constexpr (TYPE == 8)
-        q8_factors(F, P, tile, lane);
+        q8_factors<WIDE>(F, P, tile, lane);
     else if constexpr (TYPE == 12 && WIDE)
         q4_wide_factors(F, P, tile, lane);
     else if constexpr (TYPE == 12)

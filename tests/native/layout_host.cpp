@@ -164,3 +164,27 @@ extern "C" void quant_split_of(int n, int rt, int nb, int pair, const int *fit, 
     quant_split(q, rt, nb, pair != 0, fit);
     out[0] = q.N, out[1] = q.col_blocks, out[2] = q.splits, out[3] = q.clusters;
 }
+
+// Walks the shares of all clusters as the kernel does.  0: every (column block, row tile) is taken once, pieces stay within a column block and hold at most
+// eight row tiles, and a cluster that shares K has one piece; otherwise the violated property.  *most, *least: row tiles of the largest and the smallest share.
+extern "C" int quant_walk_check(int n, int rt, int nb, int pair, const int *fit, int *most, int *least) {
+    QuantSplit q = quant_passes(n);
+    quant_split(q, rt, nb, pair != 0, fit);
+    const QuantShares s = quant_shares(q, rt);
+    std::vector<uint8_t> seen((size_t)rt * q.col_blocks, 0);
+    *most = 0, *least = 1 << 30;
+    for (int c = 0; c < q.clusters; c++) {
+        int pieces = 0, taken = 0;
+        for (QtWalk w = qt_begin(s, c); w.r > 0; qt_next(w, rt), pieces++) {
+            if (w.r > kQtWarps || w.lo < 0 || w.lo + w.r > rt || w.block < 0 || w.block >= q.col_blocks) return 1;
+            for (int i = 0; i < w.r; i++)
+                if (seen[(size_t)w.block * rt + w.lo + i]++) return 2;
+            taken += w.r;
+        }
+        if (q.splits > 1 && pieces != 1) return 3;
+        *most = std::max(*most, taken), *least = std::min(*least, taken);
+    }
+    for (uint8_t v : seen)
+        if (v != 1) return 4;
+    return 0;
+}

@@ -179,7 +179,7 @@ def test_row_tiles_that_quick_unpacking_would_cost_digits_are_wide(layout_host, 
 @pytest.mark.parametrize("missing", [(), (8,), (5, 7, 8), (2, 3, 4, 5, 6, 7, 8), (1, 2, 3, 4, 5, 6, 7, 8)])
 def test_quantised_products_skip_cluster_sizes_that_do_not_fit(layout_host, missing):
     """The choice of CTAs that share K (csrc/quant_split.cuh) where the device takes some cluster sizes only: another size that fits is taken, for any product;
-    a cluster that shares K has one piece of at most eight row tiles of one column block."""
+    a cluster that shares K has one piece of at most eight row tiles of one column block, and the clusters' shares cover every row tile of every column block once."""
     import ctypes as C
     fit = (C.c_int * 9)(0, *[0 if s in missing else 148 // s for s in range(1, 9)])
     out = (C.c_int * 4)()
@@ -196,3 +196,6 @@ def test_quantised_products_skip_cluster_sizes_that_do_not_fit(layout_host, miss
                     assert 1 <= splits <= nb and splits not in missing and 1 <= clusters <= fit[splits] * (1 + pair)
                     if splits > 1:
                         assert clusters % blocks == 0 and -(-rt * blocks // clusters) <= 8
+                    most, least = C.c_int(), C.c_int()
+                    assert layout_host.quant_walk_check(n, rt, nb, pair, fit, C.byref(most), C.byref(least)) == 0, (n, rt, nb, pair)
+                    assert most.value - least.value <= 1

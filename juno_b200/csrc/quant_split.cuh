@@ -54,30 +54,21 @@ inline void quant_split(QuantSplit &q, int rt, int nb, bool pair, const int *fit
     }
 }
 
-// `total` things over `n` takers: `least` each, and one more for the first `more` of them.
+// `total` things over `n` takers, divided beforehand: taker i begins at total * i / n, rounded down.  One more than the least is taken at even distances: with the larger
+// shares first Llama-3-8B prompts of 333 / 500 positions took 9.55 / 14.2 ms, with them spread 8.55 / 12.95.
 struct EvenShares {
-    int least, more;
-    JHD int begin(int i) const { return i * least + (i < more ? i : more); }
+    int least, more;     // total / n and what is left
+    uint32_t per_n;      // 2^32 / n, rounded up: the quotients below are exact for n up to 2^10
+    JHD int begin(int i) const { return i * least + (int)((uint64_t)(uint32_t)(i * more) * per_n >> 32); }
 };
-inline EvenShares even_shares(int total, int n) { return EvenShares{total / n, total % n}; }
+inline EvenShares even_shares(int total, int n) { return EvenShares{total / n, total % n, (uint32_t)(((1ull << 32) + n - 1) / n)}; }
 
-// What a launch knows of its clusters' shares, divided beforehand: `per` clusters take `span` row tiles one after the other: those of a column block where the clusters
-// divide evenly among the blocks (always where they share K), else of all of them.  A cluster in two column blocks has a piece more: Llama-3-8B, 500 positions in four
-// blocks 13.3 ms, 14.5 with shares that run on from block to block.
+// What a launch knows of its clusters' shares of the (column block, row tile) pairs.
 struct QuantShares {
-    int total_rt, col_blocks, per, span;
+    int total_rt, col_blocks;
     EvenShares of;
 };
-inline QuantShares quant_shares(const QuantSplit &q, int rt) {
-    QuantShares s;
-    const bool apart = q.clusters % q.col_blocks == 0;
-    s.total_rt = rt;
-    s.col_blocks = q.col_blocks;
-    s.per = apart ? q.clusters / q.col_blocks : q.clusters;
-    s.span = apart ? rt : rt * q.col_blocks;
-    s.of = even_shares(s.span, s.per);
-    return s;
-}
+inline QuantShares quant_shares(const QuantSplit &q, int rt) { return QuantShares{rt, q.col_blocks, even_shares(rt * q.col_blocks, q.clusters)}; }
 // A cluster's share of the (column block, row tile) pairs, in pieces of up to eight row tiles of one column block.
 struct QtWalk {
     int f, end;        // flat index of the piece's first row tile; end of the share
@@ -89,10 +80,9 @@ JHD void qt_piece(QtWalk &w, int total_rt) {
     w.r = k > 1 ? (rem + k - 1) / k : rem > 0 ? rem : 0;
 }
 JHD QtWalk qt_begin(const QuantShares &s, int cluster) {
-    const int group = s.col_blocks == 1 ? 0 : cluster / s.per, i = cluster - group * s.per;
     QtWalk w;
-    w.f = group * s.span + s.of.begin(i);
-    w.end = group * s.span + s.of.begin(i + 1);
+    w.f = s.of.begin(cluster);
+    w.end = s.of.begin(cluster + 1);
     w.block = s.col_blocks == 1 ? 0 : w.f / s.total_rt;
     qt_piece(w, s.total_rt);
     return w;

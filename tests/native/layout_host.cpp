@@ -188,3 +188,11 @@ extern "C" int quant_walk_check(int n, int rt, int nb, int pair, const int *fit,
         if (v != 1) return 4;
     return 0;
 }
+
+// The shares of all takers begin at total * i / n.
+extern "C" int even_shares_check(int total, int n) {
+    const EvenShares s = even_shares(total, n);
+    for (int i = 0; i <= n; i++)
+        if (s.begin(i) != (int)((long long)total * i / n)) return 0;
+    return 1;
+}

@@ -199,3 +199,9 @@ def test_quantised_products_skip_cluster_sizes_that_do_not_fit(layout_host, miss
                     most, least = C.c_int(), C.c_int()
                     assert layout_host.quant_walk_check(n, rt, nb, pair, fit, C.byref(most), C.byref(least)) == 0, (n, rt, nb, pair)
                     assert most.value - least.value <= 1
+
+
+def test_even_shares_begin_where_a_division_would_put_them(layout_host):
+    for n in list(range(1, 300)) + [512, 1000, 1024]:
+        for total in (n, n + 1, 2 * n - 1, 384, 1792, 7168, 8016, 32064, 1000003):
+            assert layout_host.even_shares_check(total, n), (total, n)

@@ -38,8 +38,8 @@ def test_ragged_products(mv, oracle, t, rows, cols, batch):
 
 @pytest.mark.parametrize("t", TYPES)
 def test_rows_of_very_different_scale(mv, oracle, t):
-    """Every row has a power of two of its own: factors from the smallest to the largest that FP16 blocks hold, a row of zeros, and one whose
-    minima dwarf its scales.  Scale, minimum, weight and activation are rounded to FP16 once each, so a product is off by less than
+    """Every row, alike in itself, has a power of two of its own: factors from the smallest to the largest that FP16 blocks hold, a row of zeros, and one whose
+    minima dwarf its scales (blocks of one row that differ: test_blocks_of_one_row_far_apart).  Scale, minimum, weight and activation are rounded to FP16 once each, so a product is off by less than
     4 * 2^-11 of the row's largest part of a weight (scale * q or minimum) times the sum of |x|."""
     rng = np.random.default_rng(32)
     rows, cols, batch = 40, 1024, 12

@@ -40,7 +40,7 @@ def _newest_header() -> float:
 
 
 def _compile(src: str, verbose: bool) -> str:
-    # Without --split-compile: it built the same source into one of several libraries (two or three cubins in five runs of nvcc), and steps of one to eight
+    # Without --split-compile: it built the same source into one of several libraries (two cubins each of qgemv.cu and attn.cu in three to five runs of nvcc), and steps of one to eight
     # sequences were 4 to 6 % apart between them (TinyLlama, one request 717 or 750 us; Llama-3-8B, eight 3.65 to 3.89 ms, now 3.76).
     # The files are compiled side by side, so the build takes no longer.
     obj = os.path.join(OBJ, src.replace(".cu", ".o"))

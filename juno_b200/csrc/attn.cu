@@ -342,7 +342,7 @@ __global__ void __launch_bounds__(W * 32, W == kMmaWarps ? kMmaCtas<HD> : kWideC
         sm_q[8 * LDT + g * LDT + 2 * i + 1] = __float2half_rn(y1 - __half2float(h1h));
     }
     __syncthreads();
-    // A fragments of q (rows 0..7 only): a0 = (row r8, k 2c..2c+1), a2 = (row r8, k 2c+8..2c+9) of every 16-column step
+    // A fragments of q: a0 = (row r8, k 2c..2c+1), a2 = (row r8, k 2c+8..2c+9) of every 16-column step, high limbs; a1 and a3, of rows r8 + 8, low limbs
     uint32_t qh[KS][2], ql[KS][2];
 #pragma unroll
     for (int ks = 0; ks < KS; ks++) {
@@ -463,7 +463,7 @@ __global__ void __launch_bounds__(W * 32, W == kMmaWarps ? kMmaCtas<HD> : kWideC
     // this lane's share of the row sum -> row sum
     l_run += __shfl_xor_sync(0xffffffffu, l_run, 1);
     l_run += __shfl_xor_sync(0xffffffffu, l_run, 2);
-    // merge the four warps through shared memory (the K/V tiles are dead)
+    // merge the warps through shared memory (the K/V tiles are dead)
     __syncthreads();
     float *mg_o = reinterpret_cast<float *>(sm_kv);       // [warp][G][HD]
     float *mg_m = mg_o + W * G * HD;               // [warp][G]

@@ -5,7 +5,8 @@
 
 namespace juno {
 
-// out[r][row] = scale[r] * sum_c w(row, c) x[r][c] for r < n, in one pass over the quantised blocks per 256 rows of x.
+// out[r][row] = scale[r] * sum_c w(row, c) x[r][c] for r < n, in one pass over the quantised blocks for up to 224 rows of x, in two, four, ... of
+// equal parts above (quant_passes).
 struct GemmQuantArgs {
     GemvSeg seg[3];  // matrices that share the input; any mix of block formats
     int nseg = 1;

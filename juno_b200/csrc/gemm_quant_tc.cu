@@ -5,7 +5,7 @@
 // copy of the weights goes through memory.  Unpacked values that went through shared memory would cost 64 cycles of its bandwidth to
 // write and as many for the MMA to read them; the tensor memory takes them in 32, in the register layout that a tile's lanes have anyway
 // (tcgen05.st 16x256b is an mma fragment), and the multiplication costs the unpacking warps nothing.  Bound by the unpacking up to about
-// 128 rows, by the MMAs above: 186 cycles of a scheduler per 128 columns of a Q4_K tile (Q6_K 250, Q8_0 166) where the multiply-adds
+// 128 rows, by the MMAs above: quick 186 cycles of a scheduler per 128 columns of a Q4_K tile (Q6_K 250, Q8_0 166) where the multiply-adds
 // would take 112; the byte permutes and shifts run at a quarter of the rate.
 //
 // A CTA takes up to eight row tiles (128 weight rows, the M of the MMA) at a time and walks along its part of K.  Eight warps own a row
@@ -15,9 +15,10 @@
 // rank order.
 //
 // Measured in chains of 20 launches with their staging against the kernels before (mma.sync with the batch as N, tcgen05 through shared memory),
-// Q4_K, 9 / 32 / 64 rows: 28672 x 4096 41.6 / 52.2 / 60.9 -> 26.9 / 28.3 / 30.6 us; 4096 x 14336 23.5 / 43.9 / 57.5 -> 21.6 / 22.3 / 25.2;
-// 4096 x 4096 10.0 / 19.8 / 19.0 -> 13.0 / 13.3 / 17.7; 2560 x 2048 7.7 / 9.6 / 15.2 -> 10.3 / 11.0 / 12.3 (a launch costs 2 us more: tensor memory,
-// TMA, exchange).  Whole calls: Llama-3-8B with 4 layers, 48 requests 1.19 -> 0.84 ms; 200 positions of the 8B model 9.8 -> 5.5 ms.
+// Q4_K with quick tiles, 9 / 32 / 64 rows: 28672 x 4096 45.8 / 56.5 / 60.8 -> 25.7 / 27.0 / 29.2 us; 4096 x 14336 25.4 / 36 to 47 / 45 to 60 -> 18.9 / 20.0 /
+// 23.6; 4096 x 4096 10.5 / 20.3 / 18.8 -> 11.1 / 11.6 / 16.0; 2048 x 2048 8.0 / 9.8 / 12.3 -> 8.3 / 9.0 / 11.1.  The smallest with 9 to 16 rows stay up to
+// 0.6 us behind: tensor memory, tensor copies and the give-back before the exchange.  Whole calls: TinyLlama, 9 / 64 requests 1334 / 2363 -> 1102 / 1530 us;
+// Llama-3-8B with 4 layers, 48 requests 1.04 -> 0.58 ms; 200 positions of the 8B model 9.9 -> 5.4 ms.
 #include <cuda.h>
 
 #include <algorithm>

@@ -910,9 +910,9 @@ constexpr int kPromptMinRows = 128, kPromptRows = 2048;  // least and most posit
 
 static int step_sync(juno_model *m);
 
-// Does a portion of n positions take the many-row path?  Its cost hardly depends on n below a few hundred (every weight is read,
-// turned into FP16 and read again), so it pays as soon as the batched kernels would need a second pass: Llama-3-8B, 65 positions
-// through them 14 ms.  A model opened for few sequences has small passes that cost less each, hence the third pass there.
+// Does a portion of n positions take the many-row path?  As soon as the batched kernels would need a second pass over the weights: 65
+// positions of Llama-3-8B / TinyLlama as 64 and 1 6.7 / 2.9 ms, as one pass of many rows 4.3 / 1.7.  A model opened for few sequences has small passes
+// that cost less each, hence the third pass there.
 static bool prompt_takes(const juno_model *m, int n) {
     if (m->stack || m->world > 1) return false;
     const int chunk = std::min(m->cfg.max_batch, kGemmMaxBatch);
@@ -921,8 +921,8 @@ static bool prompt_takes(const juno_model *m, int n) {
 
 // Do the products of a portion of n positions unpack the quantised tiles themselves (gemm_quant_tc.cu)?  That costs an unpacking per 224 rows,
 // where FP16 rows of the weights cost one for all of them, a write and a read, and the product itself runs on pairs of SMs.  FP16 rows / unpacking: Llama-3-8B
-// 70 / 200 / 333 / 500 positions 10.3 / 9.8 / 13.5 / 13.8 and 4.2 / 5.5 / 8.6 / 12.9 ms; TinyLlama Q4_K_M 70 / 200 / 333 / 500 positions 2.70 / 3.31 / 3.17 / 3.64 and
-// 1.77 / 2.23 / 2.74 / 3.33 ms, 600 positions 3.39 and 3.59.  Layers with fewer tiles than there are warps to unpack them are all launches: two layers of width 512, 250
+// 70 / 200 / 333 / 500 positions 10.3 / 9.8 / 13.5 / 13.8 and 4.0 / 5.4 / 8.5 / 12.9 ms; TinyLlama Q4_K_M 70 / 200 / 333 / 500 positions 2.74 / 3.25 / 3.19 / 3.67 and
+// 1.55 / 2.04 / 2.59 / 3.19 ms, 600 positions 3.39 and 3.59.  Layers with fewer tiles than there are warps to unpack them are all launches: two layers of width 512, 250
 // positions 145 and 165 us (four of width 1024, 2752 tiles each: 381 and 342).
 constexpr int kFusedRows = 512;
 static bool prompt_fused(const juno_model *m, int n) {

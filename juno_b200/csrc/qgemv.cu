@@ -645,36 +645,19 @@ __global__ void __launch_bounds__(kQThreads, OCC) qgemv_kernel(const __grid_cons
 #pragma unroll
         for (int b = 0; b < NSEQ; b++) ss[b] = 0.f;
         const int pairs = p.bc * NB;
-        // With one CTA per SM there are registers to ask for the rows of several pairs before the first is converted: a pair's way from
-        // the L2 is as long as its conversion.  TinyLlama, steps of 4 / 8 requests, one pair at a time 0.975 / 1.367 ms, as below 0.940 / 1.293;
-        // Llama-3-8B, 8 requests 3.87 and 3.60.
-        constexpr int AHEAD = OCC == 2 || TAGGED ? 1 : NT >= 3 ? 3 : 2;
-        for (int pr0 = warp; pr0 < pairs; pr0 += kQWarps * AHEAD) {
-            QIn t[AHEAD];
-            float nw[AHEAD][8];
+        // One pair after the other: asking for the rows of two or three before the first is converted took registers from the tile loop and, built twice alike, time
+        // (TinyLlama, 1 / 4 / 6 requests 704 / 891 / 1055 us, so 714 / 902 / 1068; Llama-3-8B, 1 / 3 / 5 requests 1.797 / 2.276 / 2.819 ms, so 1.811 / 2.297 / 2.880, 7 and 8 within
+        // 0.4 % of one another).
+        for (int pr = warp; pr < pairs; pr += kQWarps) {
+            const int b = pr / NB, sb = sb_first + pr - b * NB;
+            QIn t;
+            quantize_fetch<TAGGED>(q, b, sb, lane, t);
+            if (q.normw && pr != warp) ld8(q.normw + sb * 256 + lane * 8, w8);
+            float part = 0.f;
+            quantize_slice<TYPE>(q, SPLIT ? blockIdx.x < (unsigned)p.splits : blockIdx.x == 0, b, sb, lane, t, w8, xop + (size_t)pr * B::bytes, part);
 #pragma unroll
-            for (int a = 0; a < AHEAD; a++) {
-                const int pr = pr0 + a * kQWarps, b = pr / NB, sb = sb_first + pr - b * NB;
-                if (pr >= pairs) break;
-                quantize_fetch<TAGGED>(q, b, sb, lane, t[a]);
-                if (q.normw) {
-                    if (pr != warp)
-                        ld8(q.normw + sb * 256 + lane * 8, nw[a]);
-                    else
-#pragma unroll
-                        for (int i = 0; i < 8; i++) nw[a][i] = w8[i];
-                }
-            }
-#pragma unroll
-            for (int a = 0; a < AHEAD; a++) {
-                const int pr = pr0 + a * kQWarps, b = pr / NB, sb = sb_first + pr - b * NB;
-                if (pr >= pairs) break;
-                float part = 0.f;
-                quantize_slice<TYPE>(q, SPLIT ? blockIdx.x < (unsigned)p.splits : blockIdx.x == 0, b, sb, lane, t[a], nw[a], xop + (size_t)pr * B::bytes, part);
-#pragma unroll
-                for (int bb = 0; bb < NSEQ; bb++)
-                    if (bb == b) ss[bb] += part;
-            }
+            for (int bb = 0; bb < NSEQ; bb++)
+                if (bb == b) ss[bb] += part;
         }
         if (p.normw) {
             for (int b = 0; b < p.bc; b++) {

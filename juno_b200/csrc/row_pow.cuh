@@ -55,8 +55,8 @@ JHD void row_scales_q8(RowScales &r, float d) {
 // that would show beside the rounding of the other operand and of the scale, the row tile is wide.  Relative error of a product in which only the
 // blocks below the largest count, against rounding every scale and weight at its own size (Q4_K, centred blocks): super-blocks 16 / 32 / 64 / 128
 // times below 5.7e-4 and 5.7e-4, 5.9e-4 and 6.1e-4, 4.7e-4 and 5.2e-4, 5.3e-4 and 8.2e-4; Q6_K 64 / 128 / 512 times 3.4e-4 and 3.4e-4, 3.3e-4 and 3.4e-4,
-// 2.4e-4 and 6.3e-4; Q8_0 512 / 4096 times 2.1e-4 and 2.2e-4, 2.0e-4 and 1.1e-3.  Sub-blocks lie up to 63 (128) times below their neighbours in any
-// row; alone they may reach 7.5e-4 (Q4_K), 3.8e-4 (Q6_K).
+// 2.4e-4 and 6.3e-4; Q8_0 512 / 4096 times 2.1e-4 and 2.2e-4, 2.0e-4 and 1.1e-3.  A sub-block alone, 64 (128)
+// times and more below the largest scale: at the limit 1.9e-4 and 2.1e-4 (Q4_K, scale 1), 2.01e-4 and 2.04e-4 (Q6_K); half of that scale 3.3e-4, 2.2e-4.
 JHD uint32_t row_pow_word(int type, const RowScales &r) {
     int e = 15, p = 0, w = 0;
     if (r.top > 0.f && r.top < 3.0e38f) {
@@ -68,7 +68,7 @@ JHD uint32_t row_pow_word(int type, const RowScales &r) {
         w = 15 - e < 30 ? 15 - e : 30;
         if (w < 0 && r.most <= 65504.f) w = 0;
     }
-    const float low = type == 12 ? 512.f : type == 14 ? 256.f : 64.f, low_sub = type == 12 ? 128.f : type == 14 ? 64.f : 0.f;
+    const float low = type == 12 ? 512.f : type == 14 ? 256.f : 64.f, low_sub = type == 12 ? 256.f : type == 14 ? 128.f : 0.f;
     const bool wide = ldexpf(r.low, p) < low || ldexpf(r.low_sub, p) < low_sub;
     return (uint32_t)(p + kRowPowBias) | (uint32_t)(w + kRowPowBias) << 8 | (wide ? kRowWide : 0u);
 }

@@ -169,6 +169,13 @@ def test_row_tiles_that_quick_unpacking_would_cost_digits_are_wide(layout_host, 
         most = np.abs(w).max() * 2.0 ** wp
         assert most < 2.0 ** 15 and (most >= 2.0 ** 12 or wp == 30)
     assert quick >= 150
+    if t != 8:  # a lone sub-block 64 (Q4_K) or 128 (Q6_K) times and more below the bound of the row's scales
+        small = np.full(256, 60, np.uint8)
+        small[3] = 1
+        one = np.full(32, 2.0 ** -10, np.float32)
+        assert (L.row_pow_of(t, 16, (one * 1.01).ctypes.data, small.ctypes.data) >> 16) == 0
+        one[:1] /= 4
+        assert (L.row_pow_of(t, 16, one.ctypes.data, small.ctypes.data) >> 16) == 1
     zero = np.zeros(32, np.float32)
     assert L.row_pow_of(t, 16, zero.ctypes.data, np.zeros(256, np.uint8).ctypes.data) == 64 | 64 << 8
     inf = np.full(32, np.inf, np.float32)
